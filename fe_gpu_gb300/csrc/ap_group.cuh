@@ -1,0 +1,140 @@
+// Alternating projections on group tables.
+//
+// A projection of the AP scheme needs only the group means of the current
+// residual r = r0 - sum_e D_e alpha_e, and those follow from group tables alone:
+//
+//   mean_d = mu_d - (1 / n_d) sum_{e != d} N_de alpha_e - alpha_d,
+//
+// with mu_d the group means of r0, n_d the group sizes, N_de = D_d'D_e the row
+// counts of every (group of d, group of e) pair and alpha_e the accumulated
+// updates. The rows are read once for mu and written once at the end, whatever
+// the number of iterations; an iteration moves the group tables, the id tuples
+// and the count matrices.
+// FP64 form, whole fits, rows -> tables: 13M rows over 4142/13/12 groups, 4
+// columns 64.7 -> 12.3 ms; 2M rows over 100k/12k/20 groups, 12 columns 281 -> 63
+// ms; 5M rows over 940k/13/12, 4 columns 40.0 -> 20.6 ms; 800 rows 6.6 -> 1.8 ms.
+//
+// A visit of a dimension evaluates the coupling sum once and runs one
+// projection; the symmetric order projects its end dimensions twice in a row,
+// and the second projection of such a pair only repeats the table update
+// (the coupling sum has not changed).
+//
+// Kernels by dimension:
+//  * launch_ap_visit: one thread per (group, column): swept sources over the
+//    group's positions or from complete sums, small sources through their count
+//    matrices, and the update, in one launch.
+//  * launch_ap_small: a dimension of at most DENSE_SMALL_MAX_G groups: its count
+//    matrices with every other dimension are reduced over those groups; the
+//    last block to finish folds the blocks' sums and runs the projections.
+//  * launch_ap_repeat: one more projection on the stored coupling sums.
+#pragma once
+
+#include "sweep.cuh"
+
+namespace fegb {
+
+// Relaxation state of a dimension: a ring of eight slots, one per projection, the
+// four of an iteration in one half. A projection reads the two before it,
+// applies the reference's rule (fe_gpu_demean.f90:213-218) and records the
+// relaxation it used and its largest update.
+struct ApSlot {
+    double relax;
+    unsigned long long change;  // bits of max |update|
+};
+constexpr int AP_PER_ITERATION = 4;
+constexpr int AP_SLOTS = 2 * AP_PER_ITERATION;
+
+struct ApCtl {
+    double tol;
+    double max_update;  // largest update of the last iteration
+    int iterations;
+    int stop;           // set when an iteration stayed below tol: later launches return at once
+};
+
+// Count matrix of a small dimension s against a dimension e, G_e x Gs.
+template <typename T>
+struct ApDense {
+    const void* N;     // uint8, or uint32 when wide
+    int wide;
+    int Gs;
+    int max_count;
+    const T* tab;      // visit: the small dimension's table; small: the table of e
+    const unsigned long long* amax;  // per column: bits of max |tab| so far
+    int Ge;            // small: groups of e
+};
+
+template <typename T>
+struct ApTables {
+    int G, C, ld;                // ld: row stride of the tables of T
+    const double* mu;            // G x C group means of r0
+    const double* inv;           // 1 / group size (0: empty)
+    T* tab;                      // accumulated updates (gathered by the other dimensions)
+    double* alpha64;             // FP32 form: the updates in FP64 (G x C); null: tab is FP64
+    double* prev;                // G x C relaxation memory
+    double* base;                // G x C: mu - coupling sum / n of the last visit
+    unsigned long long* amax;    // C: bits of the running max |tab| per column
+    ApSlot* slots;
+};
+
+template <typename T>
+struct ApVisit {
+    ApTables<T> t;
+    int slot;
+    const ApCtl* ctl;
+    // swept sources: complete sums of -(weighted source rows) (G x C), or the
+    // group's positions (off set), or neither
+    const T* sums;
+    const int32_t* off;
+    int n_src;
+    const int32_t* src_gid[SWEEP_MAXP];
+    const T* src_tab[SWEEP_MAXP];
+    const float* weight;
+    int n_dense;
+    ApDense<T> dense[SWEEP_MAXP];
+};
+
+template <typename T>
+struct ApSmall {
+    ApTables<T> t;
+    int slot;
+    int projections;  // 1 or 2 in a row
+    const ApCtl* ctl;
+    int n_src;
+    ApDense<T> src[SWEEP_MAXP];
+    double* partials;            // ap_small_scratch() doubles
+    unsigned long long* limbs;   // 2 x Gs x C, zero between launches
+    unsigned* counter;           // zero between launches
+};
+
+template <typename T>
+int launch_ap_visit(const ApVisit<T>& p, cudaStream_t s);
+template <typename T>
+int launch_ap_repeat(const ApTables<T>& t, int slot, const ApCtl* ctl, cudaStream_t s);
+template <typename T>
+int launch_ap_small(const ApSmall<T>& p, cudaStream_t s);
+// doubles of ApSmall::partials for a dimension of Gs groups with n_src sources
+size_t ap_small_scratch(int Gs, int C, int n_src);
+
+// Slots of all dimensions for a start from relaxation `relax` and last change
+// `prev_change` per dimension (device arrays of n_fe).
+int launch_ap_reset(ApSlot* slots, const double* relax, const double* prev_change, int n_fe, ApCtl* ctl, double tol,
+                    cudaStream_t s);
+// End of an iteration whose projections used the slots of half 0 or 1: their
+// largest update against the tolerance.
+int launch_ap_check(const ApSlot* slots, int n_fe, int half, ApCtl* ctl, cudaStream_t s);
+
+// Row counts of the (group of e, group of s) pairs, N[g * Gs + t], s with at
+// most DENSE_SMALL_MAX_G groups; *mx (device) = the largest count.
+// Sorted form: off (G_e + 1) are e's groups in the row order of gid_s, no group
+// longer than AP_COUNT_LONGEST rows. N8 receives the counts, clamped to 255
+// (exact when *mx < 256); N32, when set, the counts as they are.
+constexpr int AP_COUNT_LONGEST = 1 << 16;
+int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int Gs, uint8_t* N8, uint32_t* N32,
+                       unsigned* mx, cudaStream_t s);
+// Form for matrices of at most AP_COUNT_SMALL entries, any row order; N is
+// zeroed by the call.
+constexpr int AP_COUNT_SMALL = 12 * 1024;
+int count_pairs_small(const int32_t* gid_e, int Ge, const int32_t* gid_s, long long n, int Gs, uint32_t* N,
+                      cudaStream_t s);
+
+}  // namespace fegb

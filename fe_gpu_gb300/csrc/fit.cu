@@ -10,6 +10,7 @@
 #include "linalg.cuh"
 #include "prep.cuh"
 #include "sweep.cuh"
+#include "ap_group.cuh"
 #include "batch_est.cuh"
 
 #include <algorithm>
@@ -883,30 +884,6 @@ int ap_iteration(Problem& P, T* data, PendingList& pl, const ProjectionOpts& o, 
     return 0;
 }
 
-int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update) {
-    *iterations = 0;
-    *converged = 1;
-    *max_update = 0.0;
-    if (P.n_fe == 0 || P.n == 0) return 0;
-    FEGB_TRY(reset_ap_state(P, false));
-    PendingList pl;
-    ProjectionOpts o;
-    int hit = 0;
-    double mu = 0.0;
-    for (int iter = 1; iter <= max_iter; ++iter) {
-        FEGB_TRY(ap_iteration<double>(P, P.X, pl, o, &mu));
-        *iterations = iter;
-        if (mu < tol) {
-            hit = 1;
-            break;
-        }
-    }
-    FEGB_TRY(apply_all_pending<double>(P, P.X, pl));
-    *converged = hit;
-    *max_update = mu;
-    return 0;
-}
-
 // inc[t][c] = sum over the swept dimensions j of alpha_j[ids_j[t]][c], in
 // dimension order (FP64)
 struct TupleInc {
@@ -940,6 +917,39 @@ int cluster_score_sums(Problem& P, const double* S, int ns, const int32_t* perm,
 
 int tuple_row_sums(Problem& P, const double* X, int C, double* out, Scratch& scr, int timed_kind);
 
+// Subtracts the FE coefficients alpha_all from the FP64 rows. With compressed
+// streams the swept dimensions' coefficients are first combined per id tuple:
+// two FP64 subtractions per element at 20M (tuple, period) instead of three.
+int apply_alpha_rows(Problem& P) {
+    if (P.n <= 0) return 0;
+    PendingSet<double> ps{};
+    std::vector<char> in_tuple(P.n_fe, 0);
+    if (P.row_tuple && P.tuple_n == P.n && P.tuple_sw.size() > 1) {
+        TupleInc ti{};
+        ti.nd = (int)P.tuple_sw.size();
+        for (int j = 0; j < ti.nd; ++j) {
+            ti.ids[j] = P.tuple_ids[j];
+            ti.alpha[j] = P.dims[P.tuple_sw[j]].alpha;
+            in_tuple[P.tuple_sw[j]] = 1;
+        }
+        tuple_increments_kernel<<<grid_stride_blocks((long long)P.tuple_m * P.C, 256), 256, 0, P.s>>>(
+            ti, P.tuple_m, P.C, P.inc_tab);
+        FEGB_LAUNCH_CHECK("tuple increments");
+        ps.gid[ps.n] = P.row_tuple;
+        ps.tab[ps.n] = P.inc_tab;
+        ++ps.n;
+    }
+    for (int e = 0; e < P.n_fe; ++e) {
+        if (in_tuple[e]) continue;
+        ps.gid[ps.n] = P.dims[e].gid;
+        ps.tab[ps.n] = P.dims[e].alpha;
+        ++ps.n;
+    }
+    FEGB_TRY(launch_apply_pending<double>(P.X, P.C, P.n, ps, P.s));
+    P.demean_bytes += (double)P.n * (4.0 * ps.n + 16.0 * P.C);
+    return 0;
+}
+
 // FP64 group means of the current FP64 residual for every dimension, after
 // subtracting the FE increments of the previous refinement round from the rows
 // (apply_alpha; one element pass, then read-only sweeps). With compressed CG
@@ -947,35 +957,7 @@ int tuple_row_sums(Problem& P, const double* X, int C, double* out, Scratch& scr
 // sums and short sweeps of those (n C + sum_d m C additions instead of
 // n C per dimension). Returns max |mean|.
 int fp64_mean_pass(Problem& P, bool apply_alpha, double* mu_max) {
-    if (apply_alpha && P.n > 0) {
-        PendingSet<double> ps{};
-        std::vector<char> in_tuple(P.n_fe, 0);
-        if (P.row_tuple && P.tuple_n == P.n && P.tuple_sw.size() > 1) {
-            // one combined increment per tuple of the swept dimensions: two FP64
-            // subtractions per element at 20M (tuple, period) instead of three
-            TupleInc ti{};
-            ti.nd = (int)P.tuple_sw.size();
-            for (int j = 0; j < ti.nd; ++j) {
-                ti.ids[j] = P.tuple_ids[j];
-                ti.alpha[j] = P.dims[P.tuple_sw[j]].alpha;
-                in_tuple[P.tuple_sw[j]] = 1;
-            }
-            tuple_increments_kernel<<<grid_stride_blocks((long long)P.tuple_m * P.C, 256), 256, 0, P.s>>>(
-                ti, P.tuple_m, P.C, P.inc_tab);
-            FEGB_LAUNCH_CHECK("tuple increments");
-            ps.gid[ps.n] = P.row_tuple;
-            ps.tab[ps.n] = P.inc_tab;
-            ++ps.n;
-        }
-        for (int e = 0; e < P.n_fe; ++e) {
-            if (in_tuple[e]) continue;
-            ps.gid[ps.n] = P.dims[e].gid;
-            ps.tab[ps.n] = P.dims[e].alpha;
-            ++ps.n;
-        }
-        FEGB_TRY(launch_apply_pending<double>(P.X, P.C, P.n, ps, P.s));
-        P.demean_bytes += (double)P.n * (4.0 * ps.n + 16.0 * P.C);
-    }
+    if (apply_alpha) FEGB_TRY(apply_alpha_rows(P));
     FEGB_CUDA(cudaMemsetAsync(P.max_bits + 1, 0, sizeof(unsigned long long), P.s), "reset mu max");
     std::vector<char> via_tuples(P.n_fe, 0);
     Scratch ts(P.s);
@@ -1019,67 +1001,6 @@ int fp64_mean_pass(Problem& P, bool apply_alpha, double* mu_max) {
     *mu_max = bits_to_double(b);
     return 0;
 }
-
-// Mixed form: FP64 residual r (P.X) and FP64 FE increments alpha; the inner
-// alternating projections run on an FP32 correction block c with the FP64 group
-// means of r as a per-group bias (group means of r + c = mu + means of c).
-int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update,
-                 int* outer) {
-    *iterations = 0;
-    *converged = 1;
-    *max_update = 0.0;
-    *outer = 0;
-    if (P.n_fe == 0 || P.n == 0) return 0;
-    const int max_outer = 12;
-    double mu = 0.0, mu_prev = DBL_MAX;
-    int total_iter = 0;
-    bool apply_alpha = false;
-    int hit = 0;
-    for (int round = 0; round < max_outer; ++round) {
-        FEGB_TRY(fp64_mean_pass(P, apply_alpha, &mu));
-        *outer = round + 1;
-        if (mu < tol) {
-            hit = 1;
-            break;
-        }
-        if (total_iter >= max_iter) break;
-        if (round > 2 && mu > 0.5 * mu_prev) break;  // refinement stalled
-        mu_prev = mu;
-        // inner FP32 correction sweeps
-        FEGB_CUDA(cudaMemsetAsync(P.Xc, 0, sizeof(float) * (size_t)P.n * P.C, P.s), "zero correction");
-        FEGB_TRY(reset_ap_state(P, true));
-        PendingList pl;
-        double inner_tol = std::max(0.25 * tol, 1e-5 * mu);
-        double upd = 0.0;
-        for (int it = 0; it < max_iter - total_iter; ++it) {
-            // per-dimension bias = FP64 means of r
-            ProjectionOpts o;
-            o.alpha = true;
-            // the bias differs per dimension: run the iteration projection by projection
-            FEGB_CUDA(cudaMemsetAsync(P.max_bits, 0, sizeof(unsigned long long), P.s), "reset max");
-            for (int sweep = 0; sweep < 2; ++sweep) {
-                for (int pass = 0; pass < 2; ++pass) {
-                    for (int sidx = 0; sidx < P.n_fe; ++sidx) {
-                        int d = pass == 0 ? P.order[sidx] : P.order[P.n_fe - 1 - sidx];
-                        o.bias = P.dims[d].mu;
-                        FEGB_TRY(project<float>(P, d, P.Xc, pl, o));
-                    }
-                }
-            }
-            unsigned long long b = 0;
-            FEGB_TRY(d2h_sync(&b, P.max_bits, sizeof(b), P.s, "inner max copy"));
-            upd = bits_to_double(b);
-            ++total_iter;
-            if (upd < inner_tol) break;
-        }
-        apply_alpha = true;
-    }
-    *iterations = total_iter;
-    *converged = hit;
-    *max_update = mu;
-    return 0;
-}
-
 
 // ----------------------- conjugate gradients (alpha space) -----------------------
 
@@ -1403,6 +1324,86 @@ int cg_schur_precond(Problem& P, CGBuffers<T>& B) {
     return 0;
 }
 
+// Count matrix of a small dimension d and a dimension e (G_e x G_d), uint8 when
+// every count is below 256. mx: a device word.
+template <typename T>
+int count_matrix(Problem& P, CGBuffers<T>& B, int d, int e, unsigned* mx) {
+    Scratch& scr = *P.scr;
+    const Dim &De = P.dims[e], &Dd = P.dims[d];
+    const size_t cnt = (size_t)De.G * Dd.G;
+    unsigned hmx = 0;
+    // the primary's rows are in storage order: counted block by block without
+    // the 4-byte matrix in between, unless one group holds very many rows
+    int longest = AP_COUNT_LONGEST + 1;
+    if (e == P.primary && De.off && cnt > (size_t)AP_COUNT_SMALL)
+        FEGB_TRY(max_group_length(De.off, De.G, &longest, P.s));
+    if (longest <= AP_COUNT_LONGEST) {
+        FEGB_TRY(dalloc(scr, &B.N8[d][e], cnt, "count matrix (uint8)"));
+        FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, Dd.G, B.N8[d][e], nullptr, mx, P.s));
+        FEGB_TRY(d2h_sync(&hmx, mx, sizeof(hmx), P.s, "count max copy"));
+        if (hmx >= 256) {
+            B.N8[d][e] = nullptr;
+            FEGB_TRY(dalloc(scr, &B.N32[d][e], cnt, "count matrix (uint32)"));
+            FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, Dd.G, nullptr, B.N32[d][e], mx, P.s));
+        }
+    } else {
+        Scratch tmp(P.s);  // the uint32 counts, released once narrowed or copied
+        uint32_t* N = nullptr;
+        FEGB_TRY(tmp.alloc(&N, cnt, "count matrix"));
+        if (cnt <= (size_t)AP_COUNT_SMALL) {
+            FEGB_TRY(count_pairs_small(De.gid, De.G, Dd.gid, P.n, Dd.G, N, P.s));
+        } else {
+            FEGB_CUDA(cudaMemsetAsync(N, 0, sizeof(uint32_t) * cnt, P.s), "count matrix zero");
+            FEGB_TRY(launch_count_pairs(De.gid, Dd.gid, P.n, Dd.G, N, P.s));
+        }
+        FEGB_TRY(launch_count_max(N, (long long)cnt, mx, P.s));
+        FEGB_TRY(d2h_sync(&hmx, mx, sizeof(hmx), P.s, "count max copy"));
+        if (hmx < 256) {
+            FEGB_TRY(dalloc(scr, &B.N8[d][e], cnt, "count matrix (uint8)"));
+            FEGB_TRY(launch_narrow_counts(N, (long long)cnt, B.N8[d][e], P.s));
+        } else {
+            FEGB_TRY(dalloc(scr, &B.N32[d][e], cnt, "count matrix (uint32)"));
+            FEGB_CUDA(cudaMemcpyAsync(B.N32[d][e], N, sizeof(uint32_t) * cnt, cudaMemcpyDeviceToDevice, P.s),
+                      "count matrix copy");
+        }
+    }
+    if (P.pair_max.size() != (size_t)P.n_fe) P.pair_max.assign(P.n_fe, std::vector<int>(P.n_fe, -1));
+    P.pair_max[d][e] = P.pair_max[e][d] = (int)std::min<unsigned>(hmx, 0x7fffffffu);
+    return 0;
+}
+
+// The position streams of the swept dimensions and which of them are short.
+template <typename T>
+int operator_streams(Problem& P, CGBuffers<T>& B) {
+    FEGB_TRY(cg_streams(P, B));
+    // streams whose groups are all short (a worker's few firms) take the
+    // one-thread-per-group sweep
+    for (int d = 0; d < P.n_fe; ++d) {
+        auto& st = B.stream[d];
+        st.short_groups = false;
+        if (st.n_src < 1 || st.n_src > 3 || !st.off || P.dims[d].G <= 0) continue;
+        if ((long long)P.dims[d].G * CG_SHORT_MEAN < st.m) continue;
+        int longest = 0;
+        FEGB_TRY(max_group_length(st.off, P.dims[d].G, &longest, P.s));
+        st.short_groups = longest <= CG_SHORT_MAX;
+    }
+    return 0;
+}
+
+// The operator sweep's sums / head / tail, compact rows of C.
+template <typename T>
+int operator_sums(Problem& P, CGBuffers<T>& B) {
+    Scratch& scr = *P.scr;
+    const int C = P.C;
+    const long long nchunks = std::max(1LL, seg_nchunks(P.n, CG_CHUNK));
+    int gmax = 1;
+    for (int d = 0; d < P.n_fe; ++d) gmax = std::max(gmax, P.dims[d].G);
+    FEGB_TRY(dalloc(scr, &B.sums, (size_t)gmax * C, "cg sums"));
+    FEGB_TRY(dalloc(scr, &B.head, (size_t)nchunks * C, "cg heads"));
+    FEGB_TRY(dalloc(scr, &B.tail, (size_t)nchunks * C, "cg tails"));
+    return 0;
+}
+
 template <typename T>
 int cg_alloc(Problem& P, CGBuffers<T>& B) {
     Scratch& scr = *P.scr;
@@ -1497,26 +1498,7 @@ int cg_alloc(Problem& P, CGBuffers<T>& B) {
                 sums += (long long)P.dims[d].G * C;
                 for (int e = 0; e < P.n_fe; ++e) {
                     if (e == d || P.dims[e].G <= 0) continue;
-                    const size_t cnt = (size_t)P.dims[e].G * P.dims[d].G;
-                    Scratch tmp(P.s);  // the uint32 counts, released once narrowed or copied
-                    uint32_t* N = nullptr;
-                    FEGB_TRY(tmp.alloc(&N, cnt, "count matrix"));
-                    FEGB_CUDA(cudaMemsetAsync(N, 0, sizeof(uint32_t) * cnt, P.s), "count matrix zero");
-                    FEGB_TRY(launch_count_pairs(P.dims[e].gid, P.dims[d].gid, P.n, P.dims[d].G, N, P.s));
-                    FEGB_TRY(launch_count_max(N, (long long)cnt, mx, P.s));
-                    unsigned hmx = 0;
-                    FEGB_TRY(d2h_sync(&hmx, mx, sizeof(hmx), P.s, "count max copy"));
-                    if (P.pair_max.size() != (size_t)P.n_fe) P.pair_max.assign(P.n_fe, std::vector<int>(P.n_fe, -1));
-                    P.pair_max[d][e] = P.pair_max[e][d] = (int)std::min<unsigned>(hmx, 0x7fffffffu);
-                    if (hmx < 256) {
-                        FEGB_TRY(dalloc(scr, &B.N8[d][e], cnt, "count matrix (uint8)"));
-                        FEGB_TRY(launch_narrow_counts(N, (long long)cnt, B.N8[d][e], P.s));
-                    } else {
-                        FEGB_TRY(dalloc(scr, &B.N32[d][e], cnt, "count matrix (uint32)"));
-                        FEGB_CUDA(cudaMemcpyAsync(B.N32[d][e], N, sizeof(uint32_t) * cnt, cudaMemcpyDeviceToDevice,
-                                                  P.s),
-                                  "count matrix copy");
-                    }
+                    FEGB_TRY(count_matrix(P, B, d, e, mx));
                     parts += (long long)dense_chunks(P.dims[e].G) * P.dims[d].G * C;
                 }
             }
@@ -1527,28 +1509,9 @@ int cg_alloc(Problem& P, CGBuffers<T>& B) {
             }
         }
     }
-    FEGB_TRY(cg_streams(P, B));
-    // streams whose groups are all short (a worker's few firms) take the
-    // one-thread-per-group sweep
-    for (int d = 0; d < P.n_fe; ++d) {
-        auto& st = B.stream[d];
-        st.short_groups = false;
-        if (st.n_src < 1 || st.n_src > 3 || !st.off || P.dims[d].G <= 0) continue;
-        if ((long long)P.dims[d].G * CG_SHORT_MEAN < st.m) continue;
-        int longest = 0;
-        FEGB_TRY(max_group_length(st.off, P.dims[d].G, &longest, P.s));
-        st.short_groups = longest <= CG_SHORT_MAX;
-    }
+    FEGB_TRY(operator_streams(P, B));
     if (B.schur) FEGB_TRY(cg_schur_precond(P, B));
-    // the operator sweep's sums / head / tail, compact rows of C
-    {
-        const long long nchunks = std::max(1LL, seg_nchunks(P.n, CG_CHUNK));
-        int gmax = 1;
-        for (int d = 0; d < P.n_fe; ++d) gmax = std::max(gmax, P.dims[d].G);
-        FEGB_TRY(dalloc(scr, &B.sums, (size_t)gmax * C, "cg sums"));
-        FEGB_TRY(dalloc(scr, &B.head, (size_t)nchunks * C, "cg heads"));
-        FEGB_TRY(dalloc(scr, &B.tail, (size_t)nchunks * C, "cg tails"));
-    }
+    FEGB_TRY(operator_sums(P, B));
     return 0;
 }
 
@@ -1581,7 +1544,7 @@ struct CGTimer {
 // of -(sum of the sources' rows, weighted) into B.sums (storage type, stride C).
 // Returns the number of swept sources (0: no sweep, B.sums untouched).
 template <typename T>
-int cg_sweep(Problem& P, CGBuffers<T>& B, int d, int* n_src) {
+int cg_sweep(Problem& P, CGBuffers<T>& B, int d, int* n_src, const int* stop = nullptr) {
     const int C = P.C;
     const int L = B.ld;
     const auto& st = B.stream[d];
@@ -1598,6 +1561,7 @@ int cg_sweep(Problem& P, CGBuffers<T>& B, int d, int* n_src) {
         rp.src_tab[i] = B.p + B.off[st.src_dim[i]] * L;
     }
     rp.weight = st.weight;
+    rp.stop = stop;
     rp.sums = B.sums;
     rp.head = B.head;
     rp.tail = B.tail;
@@ -1611,7 +1575,7 @@ int cg_sweep(Problem& P, CGBuffers<T>& B, int d, int* n_src) {
     } else {
         FEGB_TRY(launch_cg_rows<T>(rp, P.s));
         FEGB_TRY(launch_group_sums<T>(st.off, B.head, B.tail, CG_CHUNK, C, st.long_list, st.n_long, st.multi_list,
-                                      st.n_multi, B.sums, P.s));
+                                      st.n_multi, B.sums, P.s, stop));
     }
     FEGB_TRY(tm.end());
     P.demean_bytes += bytes;
@@ -2083,6 +2047,388 @@ int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* conver
         if (umma_err) return set_error("CG operator: a tensor-core count-matrix pass timed out waiting on its copies");
     }
     *iterations = total;
+    *converged = hit;
+    *max_update = mu;
+    return 0;
+}
+
+// ------------------- alternating projections on group tables -------------------
+
+// Host poll of a loop that runs ahead of it: AP_AHEAD iterations may be queued
+// beyond the last one whose state the host has read. The launches of an
+// iteration queued after the stop return at once.
+constexpr int AP_AHEAD = 2;
+
+struct ApPoll {
+    ApCtl* host = nullptr;  // pinned, AP_AHEAD + 1 states
+    cudaEvent_t ev[AP_AHEAD + 1] = {};
+    ~ApPoll() {
+        for (auto& e : ev)
+            if (e) cudaEventDestroy(e);
+    }
+    int open() {
+        // one small pinned block per host thread, released when the thread ends;
+        // a thread runs one fit at a time
+        thread_local struct Pinned {
+            ApCtl* p = nullptr;
+            ~Pinned() {
+                if (p) cudaFreeHost(p);
+            }
+        } pinned;
+        if (!pinned.p)
+            FEGB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pinned.p), sizeof(ApCtl) * (AP_AHEAD + 1),
+                                    cudaHostAllocPortable),
+                      "projection poll");
+        host = pinned.p;
+        for (auto& e : ev) FEGB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "projection poll");
+        return 0;
+    }
+};
+
+// Whether the AP form runs on group tables (ap_group.cuh): the count matrices
+// of the small dimensions need C <= 32, and wider rows would make every
+// position's gather as long as the row itself.
+bool ap_on_groups(int C, int n_fe, long long n) { return C <= 32 && n_fe > 0 && n > 0; }
+
+// The group tables of an AP run in storage type T, with what they gather from.
+template <typename T>
+struct ApGroups {
+    CGBuffers<T> B;
+    double* base = nullptr;      // Gt x C
+    unsigned long long* amax = nullptr;  // n_fe x C
+    ApSlot* slots = nullptr;     // n_fe x AP_SLOTS
+    ApCtl* ctl = nullptr;
+    double* partials = nullptr;
+    unsigned long long* limbs = nullptr;
+    unsigned* counter = nullptr;
+    std::vector<std::vector<int>> max_count;  // [small][e]
+    ApPoll poll;
+
+    int build(Problem& P) {
+        Scratch& scr = *P.scr;
+        const int C = P.C;
+        B.ld = cg_row_stride(C, (int)sizeof(T));
+        B.off.assign(P.goff.begin(), P.goff.end() - 1);
+        B.dense.assign(P.n_fe, 0);
+        B.N8.assign(P.n_fe, std::vector<uint8_t*>(P.n_fe, nullptr));
+        B.N32.assign(P.n_fe, std::vector<uint32_t*>(P.n_fe, nullptr));
+        max_count.assign(P.n_fe, std::vector<int>(P.n_fe, 0));
+        std::vector<int> Gd(P.n_fe);
+        for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
+        const std::vector<char> plan = cg_dense_plan(Gd, C, P.n);
+        unsigned* mx = nullptr;
+        FEGB_TRY(dalloc(scr, &mx, 1, "count max"));
+        size_t part = 1, limb = 2;
+        for (int d = 0; d < P.n_fe; ++d) {
+            if (!plan[d]) continue;
+            B.dense[d] = 1;
+            B.any_dense = true;
+            for (int e = 0; e < P.n_fe; ++e) {
+                if (e == d || P.dims[e].G <= 0) continue;
+                FEGB_TRY(count_matrix(P, B, d, e, mx));
+                max_count[d][e] = P.pair_max[d][e];
+            }
+            part = std::max(part, ap_small_scratch(Gd[d], C, P.n_fe - 1));
+            limb = std::max(limb, (size_t)2 * Gd[d] * C * std::max(1, P.n_fe - 1));
+        }
+        FEGB_TRY(operator_streams(P, B));
+        FEGB_TRY(operator_sums(P, B));
+        const size_t np = (size_t)std::max(1LL, P.Gt) * B.ld;
+        FEGB_TRY(dalloc(scr, &B.p, np, "group tables"));
+        FEGB_TRY(dalloc(scr, &base, (size_t)std::max(1LL, P.Gt) * C, "coupling sums"));
+        FEGB_TRY(dalloc(scr, &amax, (size_t)P.n_fe * C, "table maxima"));
+        FEGB_TRY(dalloc(scr, &slots, (size_t)P.n_fe * AP_SLOTS, "projection slots"));
+        FEGB_TRY(dalloc(scr, &ctl, 1, "projection state"));
+        FEGB_TRY(dalloc(scr, &partials, part, "small-dimension partials"));
+        FEGB_TRY(dalloc(scr, &limbs, limb, "small-dimension sums"));
+        FEGB_TRY(dalloc(scr, &counter, 1, "small-dimension counter"));
+        FEGB_CUDA(cudaMemsetAsync(limbs, 0, sizeof(unsigned long long) * limb, P.s), "small-dimension sums zero");
+        FEGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), P.s), "small-dimension counter zero");
+        return poll.open();
+    }
+
+    ApTables<T> tables(const Problem& P, int d) const {
+        ApTables<T> t{};
+        const Dim& D = P.dims[d];
+        t.G = D.G;
+        t.C = P.C;
+        t.ld = B.ld;
+        t.mu = D.mu;
+        t.inv = P.inv_counts_all + P.goff[d];
+        t.tab = B.p + P.goff[d] * B.ld;
+        t.alpha64 = sizeof(T) == 4 ? D.alpha : nullptr;
+        t.prev = D.prev;
+        t.base = base + P.goff[d] * P.C;
+        t.amax = amax + (size_t)d * P.C;
+        t.slots = slots + (size_t)d * AP_SLOTS;
+        return t;
+    }
+
+    // count matrix of small dimension s against e, with the table of `of`
+    ApDense<T> matrix(const Problem& P, int s, int e, int of) const {
+        ApDense<T> m{};
+        m.wide = B.N8[s][e] ? 0 : 1;
+        m.N = B.N8[s][e] ? static_cast<const void*>(B.N8[s][e]) : static_cast<const void*>(B.N32[s][e]);
+        m.Gs = P.dims[s].G;
+        m.Ge = P.dims[e].G;
+        m.max_count = max_count[s][e];
+        m.tab = B.p + P.goff[of] * B.ld;
+        m.amax = amax + (size_t)of * P.C;
+        return m;
+    }
+
+    // `projections` projections in a row of dimension d, the first in `slot`
+    int visit(Problem& P, int d, int slot, int projections) {
+        if (P.dims[d].G <= 0) return 0;
+        P.projections += projections;
+        if (B.dense[d]) {
+            ApSmall<T> q{};
+            q.t = tables(P, d);
+            q.slot = slot;
+            q.projections = projections;
+            q.ctl = ctl;
+            q.partials = partials;
+            q.limbs = limbs;
+            q.counter = counter;
+            double bytes = 0.0;
+            for (int e = 0; e < P.n_fe; ++e)
+                if (e != d && P.dims[e].G > 0) {
+                    q.src[q.n_src++] = matrix(P, d, e, e);
+                    bytes += (double)P.dims[e].G * ((B.N8[d][e] ? 1.0 : 4.0) * P.dims[d].G + (double)P.C * sizeof(T));
+                }
+            if (q.n_src > 0) {
+                CGTimer tm(P);
+                FEGB_TRY(tm.begin(6 + (sizeof(T) == 4 ? 1 : 0), bytes));
+                FEGB_TRY(launch_ap_small<T>(q, P.s));
+                FEGB_TRY(tm.end());
+                P.demean_bytes += bytes;
+                return 0;
+            }
+        }
+        ApVisit<T> v{};
+        v.t = tables(P, d);
+        v.slot = slot;
+        v.ctl = ctl;
+        const auto& st = B.stream[d];
+        double bytes = (double)P.dims[d].G * P.C * (8.0 * 5 + 2.0 * sizeof(T));
+        if (st.n_src > 0) {
+            if (st.short_groups) {
+                v.off = st.off;
+                v.n_src = st.n_src;
+                for (int i = 0; i < st.n_src; ++i) {
+                    v.src_gid[i] = st.src_gid[i];
+                    v.src_tab[i] = B.p + P.goff[st.src_dim[i]] * B.ld;
+                }
+                v.weight = st.weight;
+                bytes += (double)st.m * (4.0 * st.n_src + (st.weight ? 4.0 : 0.0) + (double)st.n_src * P.C * sizeof(T));
+            } else {
+                int n_src = 0;
+                FEGB_TRY(cg_sweep<T>(P, B, d, &n_src, &ctl->stop));
+                v.sums = B.sums;
+            }
+        }
+        for (int s = 0; s < P.n_fe; ++s)
+            if (s != d && B.dense[s] && P.dims[s].G > 0) {
+                v.dense[v.n_dense++] = matrix(P, s, d, s);
+                bytes += (double)P.dims[d].G * (B.N8[s][d] ? 1.0 : 4.0) * P.dims[s].G;
+            }
+        CGTimer tm(P);
+        FEGB_TRY(tm.begin(4 + (sizeof(T) == 4 ? 1 : 0), bytes));
+        FEGB_TRY(launch_ap_visit<T>(v, P.s));
+        for (int j = 1; j < projections; ++j) FEGB_TRY(launch_ap_repeat<T>(v.t, slot + j, ctl, P.s));
+        FEGB_TRY(tm.end());
+        P.demean_bytes += bytes;
+        return 0;
+    }
+
+    // One iteration: two symmetric sweeps (fe_gpu_demean.f90:144-292). The first
+    // projection repeats the dimension that the previous iteration ended with.
+    int iteration(Problem& P, int half) {
+        std::vector<int> seq;
+        for (int sweep = 0; sweep < 2; ++sweep) {
+            for (int i = 0; i < P.n_fe; ++i) seq.push_back(P.order[i]);
+            for (int i = P.n_fe - 1; i >= 0; --i) seq.push_back(P.order[i]);
+        }
+        std::vector<int> next(P.n_fe, half * AP_PER_ITERATION);
+        size_t i = 0;
+        for (; i < seq.size() && seq[i] == P.order[0]; ++i) {
+            const int d = seq[i];
+            FEGB_TRY(launch_ap_repeat<T>(tables(P, d), next[d]++, ctl, P.s));
+            P.projections += P.dims[d].G > 0;
+        }
+        while (i < seq.size()) {
+            const int d = seq[i];
+            size_t j = i;
+            while (j < seq.size() && seq[j] == d) ++j;
+            FEGB_TRY(visit(P, d, next[d], (int)(j - i)));
+            next[d] += (int)(j - i);
+            i = j;
+        }
+        return launch_ap_check(slots, P.n_fe, half, ctl, P.s);
+    }
+
+    // Iterations from the means mu_all (of the current rows) until the largest
+    // update stays below tol; the relaxation state continues from P.relax,
+    // P.prev_change and the prev tables. Leaves the updates in alpha_all.
+    int run(Problem& P, double tol, int max_iter, int* iterations, double* max_update) {
+        const int C = P.C;
+        FEGB_CUDA(cudaMemsetAsync(B.p, 0, sizeof(T) * (size_t)std::max(1LL, P.Gt) * B.ld, P.s), "group tables zero");
+        FEGB_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (size_t)P.n_fe * C, P.s), "table maxima zero");
+        if (sizeof(T) == 4)
+            FEGB_CUDA(cudaMemsetAsync(P.alpha_all, 0, sizeof(double) * (size_t)std::max(1LL, P.Gt) * C, P.s),
+                      "alpha zero");
+        const int d0 = P.order[0];  // no updates yet: its coupling sums are zero
+        FEGB_CUDA(cudaMemcpyAsync(base + P.goff[d0] * C, P.dims[d0].mu, sizeof(double) * (size_t)P.dims[d0].G * C,
+                                  cudaMemcpyDeviceToDevice, P.s),
+                  "coupling sums start");
+        FEGB_TRY(launch_ap_reset(slots, P.relax, P.prev_change, P.n_fe, ctl, tol, P.s));
+        ApCtl last{};
+        int queued = 0;
+        const int proj0 = P.projections;
+        while (queued < max_iter && !last.stop) {
+            FEGB_TRY(iteration(P, queued & 1));
+            const int at = queued % (AP_AHEAD + 1);
+            FEGB_CUDA(cudaMemcpyAsync(poll.host + at, ctl, sizeof(ApCtl), cudaMemcpyDeviceToHost, P.s),
+                      "projection state copy");
+            FEGB_CUDA(cudaEventRecord(poll.ev[at], P.s), "projection state event");
+            ++queued;
+            if (queued > AP_AHEAD) {
+                const int old = (queued - 1 - AP_AHEAD) % (AP_AHEAD + 1);
+                FEGB_CUDA(cudaEventSynchronize(poll.ev[old]), "projection state wait");
+                last = poll.host[old];
+            }
+        }
+        FEGB_TRY(d2h_sync(&last, ctl, sizeof(last), P.s, "projection state copy"));
+        // projections of the iterations that ran
+        if (queued > 0) P.projections = proj0 + (int)((long long)(P.projections - proj0) / queued * last.iterations);
+        *iterations = last.iterations;
+        *max_update = last.max_update;
+        if (sizeof(T) == 8)
+            FEGB_TRY(launch_to_f64<double>(reinterpret_cast<const double*>(B.p), B.ld, P.alpha_all, C, P.Gt, P.s));
+        return 0;
+    }
+};
+
+int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update) {
+    *iterations = 0;
+    *converged = 1;
+    *max_update = 0.0;
+    if (P.n_fe == 0 || P.n == 0) return 0;
+    FEGB_TRY(reset_ap_state(P, false));
+    PendingList pl;
+    ProjectionOpts o;
+    int hit = 0;
+    double mu = 0.0;
+    // The group tables carry the means of the rows as they stand, to FP64
+    // rounding: 2^-53 of the largest mean, some 64 of them over the sums. While
+    // that is not far below the tolerance (columns with a large level) the
+    // projections run on the rows, whose level the first iteration takes out.
+    constexpr double AP_ROUND = 64.0 * 0x1p-53;
+    constexpr int AP_ROW_ITERATIONS = 3;
+    int iter = 0;
+    if (ap_on_groups(P.C, P.n_fe, P.n)) {
+        ApGroups<double> A;
+        FEGB_TRY(A.build(P));
+        while (iter < max_iter && iter <= AP_ROW_ITERATIONS) {
+            double level = 0.0;
+            FEGB_TRY(fp64_mean_pass(P, false, &level));
+            if (AP_ROUND * level <= 1e-3 * tol) {
+                int it = 0;
+                FEGB_TRY(A.run(P, tol, max_iter - iter, &it, &mu));
+                FEGB_TRY(apply_alpha_rows(P));
+                *iterations = iter + it;
+                *converged = mu < tol;
+                *max_update = mu;
+                return 0;
+            }
+            FEGB_TRY(ap_iteration<double>(P, P.X, pl, o, &mu));
+            ++iter;
+            FEGB_TRY(apply_all_pending<double>(P, P.X, pl));
+            if (mu < tol) {
+                hit = 1;
+                break;
+            }
+        }
+    }
+    while (!hit && iter < max_iter) {
+        FEGB_TRY(ap_iteration<double>(P, P.X, pl, o, &mu));
+        ++iter;
+        hit = mu < tol;
+    }
+    FEGB_TRY(apply_all_pending<double>(P, P.X, pl));
+    *iterations = iter;
+    *converged = hit;
+    *max_update = mu;
+    return 0;
+}
+
+// One inner solve of the mixed form on the FP32 correction rows Xc.
+int ap_solve_rows(Problem& P, double inner_tol, int max_iter, int* iterations) {
+    FEGB_CUDA(cudaMemsetAsync(P.Xc, 0, sizeof(float) * (size_t)P.n * P.C, P.s), "zero correction");
+    PendingList pl;
+    *iterations = 0;
+    for (int it = 0; it < max_iter; ++it) {
+        ProjectionOpts o;
+        o.alpha = true;
+        FEGB_CUDA(cudaMemsetAsync(P.max_bits, 0, sizeof(unsigned long long), P.s), "reset max");
+        for (int sweep = 0; sweep < 2; ++sweep) {
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int sidx = 0; sidx < P.n_fe; ++sidx) {
+                    int d = pass == 0 ? P.order[sidx] : P.order[P.n_fe - 1 - sidx];
+                    o.bias = P.dims[d].mu;  // the FP64 means of r, dimension by dimension
+                    FEGB_TRY(project<float>(P, d, P.Xc, pl, o));
+                }
+            }
+        }
+        unsigned long long b = 0;
+        FEGB_TRY(d2h_sync(&b, P.max_bits, sizeof(b), P.s, "inner max copy"));
+        ++*iterations;
+        if (bits_to_double(b) < inner_tol) break;
+    }
+    return 0;
+}
+
+// Mixed form: FP64 residual r (P.X) and FP64 FE increments alpha; the inner
+// alternating projections run in FP32, on group tables from the FP64 group
+// means of r or, for wide rows, on an FP32 correction block c with those means
+// as a per-group bias (group means of r + c = mu + means of c).
+int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update,
+                 int* outer) {
+    *iterations = 0;
+    *converged = 1;
+    *max_update = 0.0;
+    *outer = 0;
+    if (P.n_fe == 0 || P.n == 0) return 0;
+    const int max_outer = 12;
+    double mu = 0.0, mu_prev = DBL_MAX;
+    int total_iter = 0;
+    bool apply_alpha = false;
+    int hit = 0;
+    const bool groups = ap_on_groups(P.C, P.n_fe, P.n);
+    ApGroups<float> A;
+    if (groups) FEGB_TRY(A.build(P));
+    for (int round = 0; round < max_outer; ++round) {
+        FEGB_TRY(fp64_mean_pass(P, apply_alpha, &mu));
+        *outer = round + 1;
+        if (mu < tol) {
+            hit = 1;
+            break;
+        }
+        if (total_iter >= max_iter) break;
+        if (round > 2 && mu > 0.5 * mu_prev) break;  // refinement stalled
+        mu_prev = mu;
+        FEGB_TRY(reset_ap_state(P, true));
+        const double inner_tol = std::max(0.25 * tol, 1e-5 * mu);
+        int it = 0;
+        double upd = 0.0;
+        if (groups)
+            FEGB_TRY(A.run(P, inner_tol, max_iter - total_iter, &it, &upd));
+        else
+            FEGB_TRY(ap_solve_rows(P, inner_tol, max_iter - total_iter, &it));
+        total_iter += it;
+        apply_alpha = true;
+    }
+    *iterations = total_iter;
     *converged = hit;
     *max_update = mu;
     return 0;
@@ -2769,6 +3115,16 @@ int estimate_on_problem(Problem& P, const fegb_config& cfg, const int* G_all, lo
     return 0;
 }
 
+// What build_problem prepares for the within-transform: the FP32 correction
+// block of the mixed AP form on rows, and the group order of every dimension
+// swept by the CG operator or the group-table projections.
+bool ap_needs_rows(const fegb_config& cfg, int C, int n_fe, long long n) {
+    return cfg.precision == FEGB_PREC_MIXED && cfg.demean_method == FEGB_DEMEAN_AP && !ap_on_groups(C, n_fe, n);
+}
+bool needs_group_orders(const fegb_config& cfg, int C, int n_fe, long long n) {
+    return cfg.demean_method == FEGB_DEMEAN_CG || ap_on_groups(C, n_fe, n);
+}
+
 class StreamHolder {
   public:
     explicit StreamHolder(void* user) {
@@ -2819,8 +3175,8 @@ int estimate_device_impl(const fegb_config* cfg_in, long long n, int k, int l, i
     auto t0 = Clock::now();
     long long n_single = 0;
     FEGB_TRY(build_problem(P, n, k, l, n_fe, y, W, Z, ids, group_sizes, cfg.drop_singletons != 0,
-                           !pre && cfg.precision == FEGB_PREC_MIXED && cfg.demean_method == FEGB_DEMEAN_AP, &n_single,
-                           !pre && cfg.demean_method == FEGB_DEMEAN_CG));
+                           !pre && ap_needs_rows(cfg, 1 + k + l, n_fe, n), &n_single,
+                           !pre && needs_group_orders(cfg, 1 + k + l, n_fe, n)));
     std::vector<int> G(n_fe);
     for (int d = 0; d < n_fe; ++d) G[d] = P.dims[d].G;
     // TSS of the raw y over the rows used
@@ -2963,8 +3319,8 @@ int within_impl(const fegb_config& cfg, long long n, int k, int l, int n_fe, dou
     P.profile = cfg.profile != 0;
     long long n_single = 0;
     FEGB_TRY(build_problem(P, n, k, l, n_fe, d_y, d_W, d_Z, ids, group_sizes, false,
-                           cfg.precision == FEGB_PREC_MIXED && cfg.demean_method == FEGB_DEMEAN_AP, &n_single,
-                           cfg.demean_method == FEGB_DEMEAN_CG));
+                           ap_needs_rows(cfg, 1 + k + l, n_fe, n), &n_single,
+                           needs_group_orders(cfg, 1 + k + l, n_fe, n)));
     int it = 0, conv = 1, outer = 0;
     double mu = 0.0;
     if (cfg.demean_method == FEGB_DEMEAN_CG) {

@@ -628,7 +628,9 @@ template <typename S>
 __global__ void __launch_bounds__(FIN_THREADS)
     group_sums_kernel(const int32_t* __restrict__ off, const double* __restrict__ head,
                       const double* __restrict__ tail, int R, int C, const int32_t* __restrict__ long_list,
-                      int n_long, const int32_t* __restrict__ multi_list, int n_multi, S* __restrict__ sums) {
+                      int n_long, const int32_t* __restrict__ multi_list, int n_multi, S* __restrict__ sums,
+                      const int* __restrict__ stop) {
+    if (stop && *stop) return;
     __shared__ double smem[FIN_THREADS];
     if ((int)blockIdx.x < n_long) {
         const int g = long_list[blockIdx.x];
@@ -933,18 +935,18 @@ int find_multi_groups(const int32_t* off, int G, int R, int32_t* list, int* n_mu
 template <typename S>
 int launch_group_sums(const int32_t* off, const double* head, const double* tail, int R, int C,
                       const int32_t* long_list, int n_long, const int32_t* multi_list, int n_multi, S* sums,
-                      cudaStream_t s) {
+                      cudaStream_t s, const int* stop) {
     const long long nb = (long long)n_long + ((long long)n_multi + FIN_THREADS / 32 - 1) / (FIN_THREADS / 32);
     if (nb <= 0) return 0;
     group_sums_kernel<S><<<(unsigned)nb, FIN_THREADS, 0, s>>>(off, head, tail, R, C, long_list, n_long, multi_list,
-                                                              n_multi, sums);
+                                                              n_multi, sums, stop);
     FEGB_LAUNCH_CHECK("group sums across chunks");
     return 0;
 }
 template int launch_group_sums<float>(const int32_t*, const double*, const double*, int, int, const int32_t*, int,
-                                      const int32_t*, int, float*, cudaStream_t);
+                                      const int32_t*, int, float*, cudaStream_t, const int*);
 template int launch_group_sums<double>(const int32_t*, const double*, const double*, int, int, const int32_t*, int,
-                                       const int32_t*, int, double*, cudaStream_t);
+                                       const int32_t*, int, double*, cudaStream_t, const int*);
 
 int find_long_groups(const int32_t* off, int G, int R, int32_t* list, int* n_long, cudaStream_t s) {
     *n_long = 0;
@@ -1897,6 +1899,7 @@ __device__ __forceinline__ void cg_run_push(CGRun<T, TILE>& st, int g, T a, cons
 template <typename T, int CGR_TILE, int NSRC>
 __global__ void __launch_bounds__(256, (sizeof(T) == 4 && CGR_TILE <= 12) ? CG_ROWS_MINB : 2)
     cg_rows_kernel(CGRowsParams<T> p, int ntiles) {
+    if (p.stop && *p.stop) return;
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5;
     const long long nchunks = (p.n + CG_CHUNK - 1) / CG_CHUNK;

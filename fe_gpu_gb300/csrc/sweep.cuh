@@ -127,7 +127,7 @@ int find_multi_groups(const int32_t* off, int G, int R, int32_t* list, int* n_mu
 template <typename S>
 int launch_group_sums(const int32_t* off, const double* head, const double* tail, int R, int C,
                       const int32_t* long_list, int n_long, const int32_t* multi_list, int n_multi, S* sums,
-                      cudaStream_t s);
+                      cudaStream_t s, const int* stop = nullptr);
 // sums[g][c] = tail[qs][c] + sum_{qs<q<=qe} head[q][c] for the listed groups.
 int launch_long_sums(const int32_t* off, const double* head, const double* tail, int R, int C, const int32_t* list,
                      int n_long, double* sums, cudaStream_t s);
@@ -187,6 +187,9 @@ struct CGRowsParams {
     T* sums;
     double* head;
     double* tail;
+    // optional device flag: when set, the launch returns at once (a loop that
+    // has stopped while its next iterations were already queued)
+    const int* stop;
 };
 
 template <typename T>
