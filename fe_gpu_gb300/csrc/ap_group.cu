@@ -10,17 +10,19 @@ namespace {
 constexpr int AP_THREADS = 256;
 
 // Fixed-point sums of FP64 table values. GB300 adds FP64 at 1/64 of the FP32
-// rate, 64-bit integers at about 1/3 of it; so counts x values are summed as
-// integers: a value v of a column with max |v| < 2^(e+1) becomes
-// round(v 2^k), k = 61 - bits - e, where the counts of one sum add up to at most
-// 2^bits. Such sums are exact and their order does not matter; with bits <= 9
-// the one rounding of a value is at most half an ulp of the column's largest
-// value, no more than an FP64 sum of such values loses.
-constexpr int AP_FIX_BITS = 9;
+// rate, and converts to and from it no faster; 64-bit integers run at about 1/3.
+// So counts x values are summed as integers: a value v of a column with
+// max |v| < 2^(e+1) becomes round(v 2^k), k = 51 - e, 53 bits with the sign (one
+// rounding of at most half an ulp of the column's largest value, no more than an
+// FP64 sum of such values loses), in two digits hi 2^26 + lo. Products with
+// counts add up in one 64-bit integer per digit: all counts of a dimension add up
+// to n < 2^31 rows, so neither overflows whatever the counts, and the sums are
+// exact in any order.
+constexpr int FIX_LO = 26;
 
-__device__ __forceinline__ int fix_exponent(unsigned long long amax_bits, int bits) {
+__device__ __forceinline__ int fix_exponent(unsigned long long amax_bits) {
     const int e = (int)((amax_bits >> 52) & 0x7ff);
-    return 61 - bits - (e - 1023);  // k
+    return 51 - (e - 1023);  // k
 }
 
 __device__ __forceinline__ long long to_fixed(double v, int k) {
@@ -28,25 +30,27 @@ __device__ __forceinline__ long long to_fixed(double v, int k) {
     const int e = (int)((b >> 52) & 0x7ff);
     if (e == 0) return 0;
     const unsigned long long m = ((unsigned long long)b & ((1ULL << 52) - 1ULL)) | (1ULL << 52);
-    const int sh = e - 1075 + k;  // at most 61 - bits - 52
-    unsigned long long r;
-    if (sh >= 0)
-        r = m << min(sh, 10);
-    else if (sh > -54)
-        r = (m + (1ULL << (-sh - 1))) >> (-sh);
-    else
-        r = 0;
+    const int sh = max(1, 1075 - k - e);
+    const unsigned long long r = sh < 54 ? (m + (1ULL << (sh - 1))) >> sh : 0ULL;
     return b < 0 ? -(long long)r : (long long)r;
 }
 
-// Factor of the fixed-point sums of a column, 2^-k. A column with an infinity
-// or NaN in its table has no fixed-point form: its factor is NaN, and so are its
-// sums.
-__device__ __forceinline__ double unfix_factor(unsigned long long amax_bits, int bits) {
-    constexpr unsigned long long INF = 0x7ffULL << 52;
-    if (amax_bits >= INF) return __longlong_as_double((long long)(INF | 1ULL << 51));
-    const int e = max(-1022, min(1023, -fix_exponent(amax_bits, bits)));
-    return __longlong_as_double((long long)(e + 1023) << 52);
+struct FixDigits {
+    int hi;
+    unsigned lo;
+};
+__device__ __forceinline__ FixDigits fix_digits(long long f) {
+    FixDigits d;
+    d.hi = (int)(f >> FIX_LO);
+    d.lo = (unsigned)f & ((1u << FIX_LO) - 1u);
+    return d;
+}
+struct FixSum {
+    long long hi, lo;
+};
+__device__ __forceinline__ void fix_add(FixSum& s, unsigned n, const FixDigits& d) {
+    s.hi += (long long)(int)n * d.hi;  // counts are below 2^31
+    s.lo = (long long)((unsigned long long)s.lo + (unsigned long long)n * d.lo);
 }
 
 // Relaxation of the projection in `slot`, from the two before it.
@@ -68,6 +72,37 @@ __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsig
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
     return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL;
 }
+// a 2^-k, rounded to nearest, on the integer pipe (the conversion instruction
+// runs at the FP64 rate)
+__device__ __forceinline__ double from_fixed(long long a, int k) {
+    if (a == 0) return 0.0;
+    const unsigned long long u = a < 0 ? 0ULL - (unsigned long long)a : (unsigned long long)a;
+    const int lz = __clzll((long long)u);
+    const unsigned long long m = u << lz;  // leading bit at 63
+    const int e = 63 - lz - k + 1022;      // the leading 1 of the fraction adds one to the exponent
+    if (e <= 0) return 0.0;
+    const unsigned long long f = (m >> 11) + ((m >> 10) & 1ULL);
+    return __longlong_as_double((long long)(((unsigned long long)e << 52) + f) | (a & (long long)(1ULL << 63)));
+}
+
+// value of a fixed-point sum; a column with an infinity or NaN in its table has
+// no fixed-point form, and its sums are NaN
+__device__ __forceinline__ double fix_value(const FixSum& s, unsigned long long amax_bits) {
+    if (amax_bits >= (0x7ffULL << 52)) return __longlong_as_double(0x7ff8LL << 48);
+    const int k = fix_exponent(amax_bits);
+    const long long hi = s.hi + (s.lo >> FIX_LO), lo = s.lo & ((1LL << FIX_LO) - 1);
+    if (hi < (1LL << (62 - FIX_LO)) && hi > -(1LL << (62 - FIX_LO))) return from_fixed(hi * (1LL << FIX_LO) + lo, k);
+    return from_fixed(hi, k - FIX_LO) + from_fixed(lo, k);
+}
+
+// float -> T; to double on the integer pipe, for the counts that weights are
+// (normal numbers)
+__device__ __forceinline__ void count_to(float w, float& o) { o = w; }
+__device__ __forceinline__ void count_to(float w, double& o) {
+    const unsigned long long b = __float_as_uint(w);
+    o = __longlong_as_double((long long)(((b >> 23) + 896ULL) << 52 | (b & 0x7fffffULL) << 29));
+}
+
 // |v| for the convergence maximum, which passes over NaN as the row sweeps' does
 __device__ __forceinline__ unsigned long long update_bits(double v) {
     const unsigned long long b = abs_bits(v);
@@ -140,122 +175,148 @@ __device__ __forceinline__ T dense_dot(const CT* __restrict__ N, int Gs, const T
     for (; t < Gs; ++t) a = fma((T)N[t], tab[t * C + c], a);
     return a;
 }
-__device__ __forceinline__ long long dense_dot_fixed(const uint8_t* __restrict__ N, int Gs,
-                                                     const long long* __restrict__ tab, int C, int c) {
-    long long a = 0;
-    int t = 0;
-    if ((Gs & 3) == 0) {  // rows start on 4 bytes
-        for (; t < Gs; t += 4) {
-            const unsigned w = *reinterpret_cast<const unsigned*>(N + t);
-            a += (long long)(w & 255u) * tab[t * C + c];
-            a += (long long)((w >> 8) & 255u) * tab[(t + 1) * C + c];
-            a += (long long)((w >> 16) & 255u) * tab[(t + 2) * C + c];
-            a += (long long)(w >> 24) * tab[(t + 3) * C + c];
-        }
-        return a;
+// the same in fixed point; rows of N start on 4 counts and are zero past Gs, as
+// the table is up to a multiple of four rows
+__device__ __forceinline__ void dense_dot_fixed(const uint8_t* __restrict__ N, int pitch,
+                                                const FixDigits* __restrict__ tab, int C, int c, FixSum& a) {
+#pragma unroll 2
+    for (int t = 0; t < pitch; t += 4) {
+        const unsigned w = *reinterpret_cast<const unsigned*>(N + t);
+        fix_add(a, w & 255u, tab[t * C + c]);
+        fix_add(a, (w >> 8) & 255u, tab[(t + 1) * C + c]);
+        fix_add(a, (w >> 16) & 255u, tab[(t + 2) * C + c]);
+        fix_add(a, w >> 24, tab[(t + 3) * C + c]);
     }
-    for (; t < Gs; ++t) a += (long long)(unsigned)N[t] * tab[t * C + c];
-    return a;
+}
+__device__ __forceinline__ void dense_dot_fixed(const uint32_t* __restrict__ N, int pitch,
+                                                const FixDigits* __restrict__ tab, int C, int c, FixSum& a) {
+    for (int t = 0; t < pitch; t += 4) {
+        const uint4 w = *reinterpret_cast<const uint4*>(N + t);
+        fix_add(a, w.x, tab[t * C + c]);
+        fix_add(a, w.y, tab[(t + 1) * C + c]);
+        fix_add(a, w.z, tab[(t + 2) * C + c]);
+        fix_add(a, w.w, tab[(t + 3) * C + c]);
+    }
 }
 
-__device__ __forceinline__ int fix_bits(int groups, int max_count) {
-    return 32 - __clz(groups * max_count);  // groups * max_count < 2^bits
-}
-inline bool fix_ok(int groups, int max_count) {
-    return max_count > 0 && (long long)groups * max_count < (1 << AP_FIX_BITS);
-}
-
-// One visit: thread (r, c) takes column c of groups g0 + r, + rows per step...
-// The small sources' tables sit in shared memory (as fixed-point integers where
-// the counts allow it: FP64 form, uint8 counts).
+// One visit: thread (r, c) takes column c of the block's groups r, r + rps, ...
+// The small sources' tables sit in shared memory, in the FP64 form as
+// fixed-point digits of one scale per column, so that a group's sum over all of
+// them is one pair of integers. What is left on the FP64 pipe, which bounds the
+// kernel, is one FMA per swept position and the update (100k groups, 12 columns,
+// 20 small groups: 37 us with FP64 sums, 19 us).
 template <typename T>
-__global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p, unsigned fixed_mask) {
+__global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
     if (p.ctl->stop) return;
     extern __shared__ __align__(16) unsigned char ap_smem[];
-    unsigned long long* red = reinterpret_cast<unsigned long long*>(ap_smem);
-    unsigned char* tabs = ap_smem + sizeof(unsigned long long) * AP_THREADS;
+    constexpr bool FIX = sizeof(T) == 8;
+    unsigned long long* red = reinterpret_cast<unsigned long long*>(ap_smem);  // AP_THREADS
+    unsigned long long* cmax = red + AP_THREADS;                               // C, to 32
+    unsigned char* tabs = reinterpret_cast<unsigned char*>(cmax + 32);
     const ApTables<T>& t = p.t;
     const int C = t.C;
     const int rps = AP_THREADS / C;
     const int rr = (int)threadIdx.x / C;
     const int c = (int)threadIdx.x - rr * C;
     const bool active = rr < rps;
-    // small tables: entry (t, c) at dst[t * C + c], 8 bytes per entry in the
-    // FP64 form (double or fixed point), 4 in the FP32 form
-    {
+    const bool small = p.n_dense > 0 && !p.small_known;
+    // small tables: entry (t, c) at dst[t * C + c], pitch rows (zero past Gs)
+    if (small) {
+        if (FIX) {
+            for (int i = threadIdx.x; i < C; i += AP_THREADS) {
+                unsigned long long m = 0;
+                for (int e = 0; e < p.n_dense; ++e) m = umax64(m, p.dense[e].amax[i]);
+                cmax[i] = m;
+            }
+            __syncthreads();
+        }
         T* dst = reinterpret_cast<T*>(tabs);
         for (int e = 0; e < p.n_dense; ++e) {
             const ApDense<T>& D = p.dense[e];
-            const bool fx = (fixed_mask >> e) & 1u;
-            const int bits = fx ? fix_bits(D.Gs, D.max_count) : 0;
-            for (int i = threadIdx.x; i < D.Gs * C; i += AP_THREADS) {
+            for (int i = threadIdx.x; i < D.pitch * C; i += AP_THREADS) {
                 const int tt = i / C, cc = i - tt * C;
-                const T v = D.tab[tt * t.ld + cc];
-                if (sizeof(T) == 8 && fx)
-                    reinterpret_cast<long long*>(dst)[i] = to_fixed((double)v, fix_exponent(D.amax[cc], bits));
+                const T v = tt < D.Gs ? D.tab[tt * t.ld + cc] : T(0);
+                if (FIX)
+                    reinterpret_cast<FixDigits*>(dst)[i] = fix_digits(to_fixed((double)v, fix_exponent(cmax[cc])));
                 else
                     dst[i] = v;
             }
-            dst += D.Gs * C;
+            dst += D.pitch * C;
         }
     }
     const double relax = ap_relax(t.slots, p.slot);
     if (blockIdx.x == 0 && threadIdx.x == 0) ap_open_slot(t.slots, p.slot, relax);
     __syncthreads();
     unsigned long long upd = 0, av = 0;
-    if (active) {
-        double unfix[SWEEP_MAXP];
-        for (int e = 0; e < p.n_dense; ++e)
-            unfix[e] = ((fixed_mask >> e) & 1u)
-                           ? unfix_factor(p.dense[e].amax[c], fix_bits(p.dense[e].Gs, p.dense[e].max_count))
-                           : 0.0;
+    if (active)
         for (long long g = (long long)blockIdx.x * rps + rr; g < t.G; g += (long long)gridDim.x * rps) {
             const long long idx = g * C + c;
-            T acc = T(0);  // the coupling sum
+            T acc = T(0);  // the swept sources' coupling sum
             if (p.sums) {
                 acc = t.inv[g] != 0.0 ? -p.sums[idx] : T(0);  // sums of an empty group are not written
             } else if (p.off) {
                 const int j0 = p.off[g], j1 = p.off[g + 1];
-                int j = j0;
-                for (; j + 2 <= j1; j += 2) {
-                    T v0 = T(0), v1 = T(0);
-                    for (int e = 0; e < p.n_src; ++e) {
+                const int32_t* __restrict__ sg0 = p.src_gid[0];
+                const T* __restrict__ st0 = p.src_tab[0];
+                for (int j = j0; j < j1; j += 2) {
+                    const bool two = j + 1 < j1;
+                    T v0 = st0[(long long)sg0[j] * t.ld + c];
+                    T v1 = two ? st0[(long long)sg0[j + 1] * t.ld + c] : T(0);
+                    for (int e = 1; e < p.n_src; ++e) {
                         const int32_t* __restrict__ sg = p.src_gid[e];
                         const T* __restrict__ st = p.src_tab[e];
                         v0 += st[(long long)sg[j] * t.ld + c];
-                        v1 += st[(long long)sg[j + 1] * t.ld + c];
+                        if (two) v1 += st[(long long)sg[j + 1] * t.ld + c];
                     }
-                    acc = p.weight ? fma((T)p.weight[j], v0, acc) : acc + v0;
-                    acc = p.weight ? fma((T)p.weight[j + 1], v1, acc) : acc + v1;
-                }
-                if (j < j1) {
-                    T v0 = T(0);
-                    for (int e = 0; e < p.n_src; ++e) v0 += p.src_tab[e][(long long)p.src_gid[e][j] * t.ld + c];
-                    acc = p.weight ? fma((T)p.weight[j], v0, acc) : acc + v0;
+                    T w0 = T(1), w1 = T(1);
+                    if (p.weight) {
+                        count_to(p.weight[j], w0);
+                        if (two) count_to(p.weight[j + 1], w1);
+                    }
+                    acc = fma(w0, v0, acc);
+                    if (two) acc = fma(w1, v1, acc);
                 }
             }
-            const T* st = reinterpret_cast<const T*>(tabs);
             double cpl = (double)acc;
-            for (int e = 0; e < p.n_dense; ++e) {
-                const ApDense<T>& D = p.dense[e];
-                if (sizeof(T) == 8 && ((fixed_mask >> e) & 1u))
-                    cpl += (double)dense_dot_fixed(static_cast<const uint8_t*>(D.N) + g * D.Gs, D.Gs,
-                                                   reinterpret_cast<const long long*>(st), C, c) *
-                           unfix[e];
-                else if (D.wide)
-                    cpl += (double)dense_dot<T>(static_cast<const uint32_t*>(D.N) + g * D.Gs, D.Gs, st, C, c);
-                else
-                    cpl += (double)dense_dot<T>(static_cast<const uint8_t*>(D.N) + g * D.Gs, D.Gs, st, C, c);
-                st += D.Gs * C;
+            if (p.n_dense > 0) {
+                double sm = 0.0;
+                if (p.small_known) {
+                    sm = p.small_sums[idx];
+                } else if (FIX) {
+                    FixSum f{0, 0};
+                    const FixDigits* st = reinterpret_cast<const FixDigits*>(tabs);
+                    for (int e = 0; e < p.n_dense; ++e) {
+                        const ApDense<T>& D = p.dense[e];
+                        if (D.wide)
+                            dense_dot_fixed(static_cast<const uint32_t*>(D.N) + g * D.pitch, D.pitch, st, C, c, f);
+                        else
+                            dense_dot_fixed(static_cast<const uint8_t*>(D.N) + g * D.pitch, D.pitch, st, C, c, f);
+                        st += D.pitch * C;
+                    }
+                    sm = fix_value(f, cmax[c]);
+                } else {
+                    T f = T(0);
+                    const T* st = reinterpret_cast<const T*>(tabs);
+                    for (int e = 0; e < p.n_dense; ++e) {
+                        const ApDense<T>& D = p.dense[e];
+                        if (D.wide)
+                            f += dense_dot<T>(static_cast<const uint32_t*>(D.N) + g * D.pitch, D.Gs, st, C, c);
+                        else
+                            f += dense_dot<T>(static_cast<const uint8_t*>(D.N) + g * D.pitch, D.Gs, st, C, c);
+                        st += D.pitch * C;
+                    }
+                    sm = (double)f;
+                }
+                if (p.small_sums && !p.small_known) p.small_sums[idx] = sm;
+                cpl = (p.sums || p.off) ? cpl + sm : sm;
             }
-            const double base = t.mu[idx] - cpl * t.inv[g];
+            const double base = fma(-cpl, t.inv[g], t.mu[idx]);
             t.base[idx] = base;
             double u;
             const double an = ap_update(t, g, c, base, relax, &u);
             upd = umax64(upd, update_bits(u));
             av = umax64(av, abs_bits(an));
         }
-    }
     ap_block_max(upd, av, c, active, C, rps, red, t.slots + p.slot, t.amax);
 }
 
@@ -281,162 +342,164 @@ __global__ void __launch_bounds__(AP_THREADS) ap_repeat_kernel(ApTables<T> t, in
     ap_block_max(upd, av, c, active, C, rps, red, t.slots + slot, t.amax);
 }
 
-constexpr int AP_TILE = 64;       // groups of a source staged at a time
-constexpr int AP_FLUSH = 32;      // groups per fixed-point run
-constexpr int AP_PART_BLOCKS = 152;  // blocks per source whose partials are folded in order
-constexpr int AP_FIX_BLOCKS = 608;
-
-__device__ __forceinline__ void ap_cp16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void ap_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void ap_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
-// bytes of gsrc -> smem: whole 16-byte pieces asynchronously, the rest with plain stores
-__device__ __forceinline__ void ap_stage(unsigned char* d, const unsigned char* g, long long bytes) {
-    const long long whole = bytes & ~15LL;
-    for (long long o = (long long)threadIdx.x * 16; o < whole; o += AP_THREADS * 16) ap_cp16(d + o, g + o);
-    for (long long o = whole + threadIdx.x; o < bytes; o += AP_THREADS) d[o] = g[o];
-}
+// Blocks per source of a small dimension's visit: enough that a lane has some
+// AP_DEPTH groups, and no more than fit at once. The FP32 form's partials are
+// folded by one block, hence their lower limit.
+constexpr int AP_DEPTH = 4;
+constexpr int AP_PART_BLOCKS = 152;
+constexpr int AP_FIX_BLOCKS = 304;
+constexpr int AP_HALF = 32;  // groups of the small dimension per block: two blocks share a larger one
 
 struct ApSmallGrid {
-    int first[SWEEP_MAXP + 1];  // first block of each source
-    unsigned fixed_mask;        // sources summed in fixed point
+    int first[2 * SWEEP_MAXP + 1];  // first block of each (source, half)
+    int halves;
 };
 
-// Small dimension (Gs groups): block b of a source reduces a range of the
-// source's groups, sum_g N[g][t] tab[g][c] for all (t, c), tile by tile through
-// shared memory (the next tile loads while this one is used). Thread: pairs
-// (t, c) with c fastest, NP per thread, or a slice of the groups when the
-// pairs are fewer than the threads. Fixed-point sums run over AP_FLUSH groups
-// and are split into two 32-bit limbs added up exactly in 64-bit global
-// atomics; other sums leave one FP64 partial per block, folded in block order.
+// sums over a warp's slots (lane = slot * C + c): valid in the lanes of slot 0
+template <typename V>
+__device__ __forceinline__ V warp_slot_sum(V v, int slot, int slots, int C, int top) {
+    for (int o = top; o > 0; o >>= 1) {
+        const V w = __shfl_down_sync(0xffffffffu, v, o * C);
+        if (slot + o < slots) v += w;
+    }
+    return v;
+}
+
+// the four counts at N[4 w .. 4 w + 3] of a row
+__device__ __forceinline__ uint4 four_counts(const uint8_t* row, int w) {
+    const unsigned x = reinterpret_cast<const unsigned*>(row)[w];
+    return make_uint4(x & 255u, (x >> 8) & 255u, (x >> 16) & 255u, x >> 24);
+}
+__device__ __forceinline__ uint4 four_counts(const uint32_t* row, int w) { return reinterpret_cast<const uint4*>(row)[w]; }
+
+// acc[t] += N[g][t] * tab[g][c] over this lane's groups
+template <typename CT, int GT>
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int t0, int words,
+                                           const double* __restrict__ tab, int ld, int c, int k, long long g,
+                                           long long Ge, long long gstep, FixSum (&acc)[GT]) {
+#pragma unroll 2
+    for (; g < Ge; g += gstep) {
+        const CT* __restrict__ row = N + g * pitch + t0;
+        const FixDigits a = fix_digits(to_fixed(tab[g * ld + c], k));
+#pragma unroll
+        for (int w = 0; w < GT / 4; ++w) {
+            if (w >= words) break;
+            const uint4 x = four_counts(row, w);
+            fix_add(acc[4 * w], x.x, a);
+            fix_add(acc[4 * w + 1], x.y, a);
+            fix_add(acc[4 * w + 2], x.z, a);
+            fix_add(acc[4 * w + 3], x.w, a);
+        }
+    }
+}
+template <typename CT, int GT>
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int t0, int words,
+                                           const float* __restrict__ tab, int ld, int c, int, long long g,
+                                           long long Ge, long long gstep, float (&acc)[GT]) {
+#pragma unroll 2
+    for (; g < Ge; g += gstep) {
+        const CT* __restrict__ row = N + g * pitch + t0;
+        const float a = tab[g * ld + c];
+#pragma unroll
+        for (int w = 0; w < GT / 4; ++w) {
+            if (w >= words) break;
+            const uint4 x = four_counts(row, w);
+            acc[4 * w] = fmaf((float)x.x, a, acc[4 * w]);
+            acc[4 * w + 1] = fmaf((float)x.y, a, acc[4 * w + 1]);
+            acc[4 * w + 2] = fmaf((float)x.z, a, acc[4 * w + 2]);
+            acc[4 * w + 3] = fmaf((float)x.w, a, acc[4 * w + 3]);
+        }
+    }
+}
+
+// Small dimension: sum_g N[g][t] tab[g][c] of one source for up to GT of its
+// groups t and all c. A warp holds 32 / C slots of C lanes; a lane walks over
+// groups g (neighbouring slots on neighbouring groups: table rows and count rows
+// are read as contiguous runs, without shared memory) and keeps the sums of its
+// column for its t in registers: two integer multiply-adds and the byte's
+// extraction per count, or one FMA in the FP32 form. Integer sums are folded
+// over the block and added to 64-bit global accumulators (exact, so the order is
+// free); FP32 sums leave one FP64 partial per block, folded in block order.
 // The last block to finish turns the sums into the projections.
-template <typename T, int NP>
-__global__ void __launch_bounds__(AP_THREADS) ap_small_kernel(ApSmall<T> p, ApSmallGrid gr) {
+// 100k x 20 and 12k x 20 counts, 12 columns: 81 us with FP64 sums of both
+// operands in shared memory, 41 us in this form; 940k x 13, 4 columns: 75 -> 44.
+template <typename T, int GT>
+__global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2) ap_small_kernel(ApSmall<T> p, ApSmallGrid gr) {
     if (p.ctl->stop) return;
     extern __shared__ __align__(16) unsigned char ap_smem[];
     __shared__ bool s_last;
+    constexpr bool FIX = sizeof(T) == 8;
+    constexpr int WARPS = AP_THREADS / 32;
     const ApTables<T>& t = p.t;
-    const int C = t.C, Gs = t.G, ld = t.ld;
+    const int C = t.C, Gs = t.G;
     const int P = Gs * C;
-    int src = 0;
-    while (src + 1 < p.n_src && (int)blockIdx.x >= gr.first[src + 1]) ++src;
+    int part = 0;
+    while (part + 1 < p.n_src * gr.halves && (int)blockIdx.x >= gr.first[part + 1]) ++part;
+    const int src = part / gr.halves;
+    const int t0 = (part - src * gr.halves) * AP_HALF;
+    const int nt = min(Gs - t0, gr.halves > 1 ? AP_HALF : Gs);
     const ApDense<T>& D = p.src[src];
-    const bool fx = sizeof(T) == 8 && ((gr.fixed_mask >> src) & 1u);
-    const int bits = fx ? fix_bits(AP_FLUSH, D.max_count) : 0;
-    const int nb = gr.first[src + 1] - gr.first[src], b = (int)blockIdx.x - gr.first[src];
-    const long long tiles = (D.Ge + AP_TILE - 1) / AP_TILE;
-    const long long t0 = tiles * b / nb, t1 = tiles * (b + 1) / nb;
-    const size_t a_bytes = sizeof(T) * (size_t)AP_TILE * ld;
-    const size_t n_bytes = (size_t)AP_TILE * Gs * (D.wide ? 4 : 1);
-    const size_t buf = a_bytes + n_bytes;
-    // pairs of this thread and its slice of the groups
-    const int Pr = min(AP_THREADS, (P + 31) & ~31);
-    const int S = NP > 1 ? 1 : AP_THREADS / Pr;
-    const int slice = NP > 1 ? 0 : (int)threadIdx.x / Pr;
-    const int pair0 = NP > 1 ? (int)threadIdx.x : (int)threadIdx.x - slice * Pr;
-    int pt[NP], pc[NP];
-    bool ok[NP];
-    double sum[NP];
-    long long lo[NP], hi[NP];
+    const int nb = gr.first[part + 1] - gr.first[part], b = (int)blockIdx.x - gr.first[part];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slots = 32 / C;
+    const int slot = lane / C, c = lane - slot * C;
+    int top = 1;
+    while (top < slots) top <<= 1;
+    top >>= 1;
+    const int words = (nt + 3) / 4;
+    const long long gstep = (long long)nb * WARPS * slots;
+    const long long g0 = slot < slots ? ((long long)b * WARPS + warp) * slots + slot : D.Ge;
+    const int PB = nt * C;  // sums of this block
+    if constexpr (FIX) {
+        FixSum acc[GT];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-        const int pr = pair0 + i * AP_THREADS;
-        ok[i] = pr < P && slice < S;
-        pt[i] = ok[i] ? pr / C : 0;
-        pc[i] = ok[i] ? pr - pt[i] * C : 0;
-        sum[i] = 0.0;
-        lo[i] = hi[i] = 0;
-    }
-    auto stage = [&](long long tile, unsigned char* d) {
-        const long long g0 = tile * AP_TILE;
-        const int nt = (int)min((long long)AP_TILE, D.Ge - g0);
-        ap_stage(d, reinterpret_cast<const unsigned char*>(D.tab + g0 * ld), (long long)nt * ld * sizeof(T));
-        ap_stage(d + a_bytes, static_cast<const unsigned char*>(D.N) + g0 * Gs * (D.wide ? 4 : 1),
-                 (long long)nt * Gs * (D.wide ? 4 : 1));
-    };
-    if (t0 < t1) stage(t0, ap_smem);
-    ap_commit();
-    for (long long tile = t0; tile < t1; ++tile) {
-        unsigned char* cur = ap_smem + ((tile - t0) & 1 ? buf : 0);
-        unsigned char* nxt = ap_smem + ((tile - t0) & 1 ? 0 : buf);
-        if (tile + 1 < t1) stage(tile + 1, nxt);
-        ap_commit();
-        ap_wait_prev();
-        __syncthreads();
-        const int nt = (int)min((long long)AP_TILE, D.Ge - tile * AP_TILE);
-        T* a = reinterpret_cast<T*>(cur);
-        if (fx) {
-            for (int i = threadIdx.x; i < nt * C; i += AP_THREADS) {
-                const int gl = i / C, cc = i - gl * C;
-                T* v = a + gl * ld + cc;
-                *reinterpret_cast<long long*>(v) = to_fixed((double)*v, fix_exponent(D.amax[cc], bits));
-            }
-            __syncthreads();
-            const long long* af = reinterpret_cast<const long long*>(a);
-            const uint8_t* n8 = cur + a_bytes;
-            for (int f = 0; f < nt; f += AP_FLUSH) {
-                const int fe = min(nt, f + AP_FLUSH);
+        for (int i = 0; i < GT; ++i) acc[i] = FixSum{0, 0};
+        const int k = fix_exponent(D.amax[c]);
+        if (D.wide)
+            small_walk<uint32_t, GT>(static_cast<const uint32_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, k, g0, D.Ge,
+                                     gstep, acc);
+        else
+            small_walk<uint8_t, GT>(static_cast<const uint8_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, k, g0, D.Ge,
+                                    gstep, acc);
+        long long* red = reinterpret_cast<long long*>(ap_smem);  // WARPS x PB x 2
 #pragma unroll
-                for (int i = 0; i < NP; ++i) {
-                    if (!ok[i]) continue;
-                    long long acc = 0;
-#pragma unroll 4
-                    for (int gl = f + slice; gl < fe; gl += S)
-                        acc += (long long)(unsigned)n8[gl * Gs + pt[i]] * af[gl * ld + pc[i]];
-                    lo[i] += (long long)(acc & 0xffffffffLL);
-                    hi[i] += acc >> 32;
-                }
-            }
-        } else if (D.wide) {
-            const uint32_t* n32 = reinterpret_cast<const uint32_t*>(cur + a_bytes);
-#pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                if (!ok[i]) continue;
-                T acc = T(0);
-#pragma unroll 4
-                for (int gl = slice; gl < nt; gl += S) acc = fma((T)n32[gl * Gs + pt[i]], a[gl * ld + pc[i]], acc);
-                sum[i] += (double)acc;
-            }
-        } else {
-            const uint8_t* n8 = cur + a_bytes;
-#pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                if (!ok[i]) continue;
-                T acc = T(0);
-#pragma unroll 4
-                for (int gl = slice; gl < nt; gl += S) acc = fma((T)n8[gl * Gs + pt[i]], a[gl * ld + pc[i]], acc);
-                sum[i] += (double)acc;
+        for (int i = 0; i < GT; ++i) {
+            if (i >= nt) break;
+            const long long lo = warp_slot_sum(acc[i].lo, slot, slots, C, top);
+            const long long hi = warp_slot_sum(acc[i].hi, slot, slots, C, top);
+            if (lane < C) {
+                red[2 * (warp * PB + i * C + lane)] = lo;
+                red[2 * (warp * PB + i * C + lane) + 1] = hi;
             }
         }
-        __syncthreads();  // this buffer is refilled by the next step
-    }
-    // this block's sums: limbs into the global accumulators, or its FP64 partial
-    if (fx) {
-#pragma unroll
-        for (int i = 0; i < NP; ++i) {
-            if (!ok[i]) continue;
-            unsigned long long* l = p.limbs + 2 * ((size_t)src * P + pair0 + i * AP_THREADS);
-            if (lo[i]) atomicAdd(l, (unsigned long long)lo[i]);
-            if (hi[i]) atomicAdd(l + 1, (unsigned long long)hi[i]);
+        __syncthreads();
+        for (int i = threadIdx.x; i < 2 * PB; i += AP_THREADS) {
+            long long v = 0;
+            for (int w = 0; w < WARPS; ++w) v += red[2 * w * PB + i];
+            if (v) atomicAdd(p.limbs + 2 * ((size_t)src * P + t0 * C) + i, (unsigned long long)v);
         }
     } else {
-        double* red = reinterpret_cast<double*>(ap_smem);
-        __syncthreads();
-        if (NP == 1) {
-            if (slice < S) red[slice * Pr + pair0] = sum[0];
-            __syncthreads();
-            for (int i = threadIdx.x; i < P; i += AP_THREADS) {
-                double v = 0.0;
-                for (int k = 0; k < S; ++k) v += red[k * Pr + i];
-                p.partials[((size_t)src * AP_PART_BLOCKS + b) * P + i] = v;
-            }
-        } else {
+        float acc[GT];
 #pragma unroll
-            for (int i = 0; i < NP; ++i)
-                if (ok[i]) p.partials[((size_t)src * AP_PART_BLOCKS + b) * P + pair0 + i * AP_THREADS] = sum[i];
+        for (int i = 0; i < GT; ++i) acc[i] = 0.f;
+        if (D.wide)
+            small_walk<uint32_t, GT>(static_cast<const uint32_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, 0, g0, D.Ge,
+                                     gstep, acc);
+        else
+            small_walk<uint8_t, GT>(static_cast<const uint8_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, 0, g0, D.Ge,
+                                    gstep, acc);
+        float* red = reinterpret_cast<float*>(ap_smem);  // WARPS x PB
+#pragma unroll
+        for (int i = 0; i < GT; ++i) {
+            if (i >= nt) break;
+            const float v = warp_slot_sum(acc[i], slot, slots, C, top);
+            if (lane < C) red[warp * PB + i * C + lane] = v;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < PB; i += AP_THREADS) {
+            double v = 0.0;
+            for (int w = 0; w < WARPS; ++w) v += (double)red[w * PB + i];
+            p.partials[((size_t)src * AP_PART_BLOCKS + b) * P + t0 * C + i] = v;
         }
     }
     __threadfence();
@@ -450,23 +513,29 @@ __global__ void __launch_bounds__(AP_THREADS) ap_small_kernel(ApSmall<T> p, ApSm
     double* fold = tot + P;                                      // AP_THREADS
     unsigned long long* cmax = reinterpret_cast<unsigned long long*>(fold + AP_THREADS);  // C
     unsigned long long* wmax = cmax + C;                                                  // 8
-    for (int i = threadIdx.x; i < P; i += AP_THREADS) tot[i] = 0.0;
+    const int Pr = min(AP_THREADS, (P + 31) & ~31);
+    for (int i = threadIdx.x; i < P; i += AP_THREADS) {
+        double v = 0.0;
+        for (int e = 0; e < p.n_kept; ++e) v += p.kept[e][i];
+        tot[i] = v;
+    }
     for (int i = threadIdx.x; i < C; i += AP_THREADS) cmax[i] = 0ULL;
     __syncthreads();
     for (int e = 0; e < p.n_src; ++e) {
-        if (sizeof(T) == 8 && ((gr.fixed_mask >> e) & 1u)) {
-            const int eb = fix_bits(AP_FLUSH, p.src[e].max_count);
+        if constexpr (FIX) {
             for (int i = threadIdx.x; i < P; i += AP_THREADS) {
                 unsigned long long* l = p.limbs + 2 * ((size_t)e * P + i);
-                const long long l0 = (long long)__ldcg(l), l1 = (long long)__ldcg(l + 1);
+                const FixSum f{(long long)__ldcg(l + 1), (long long)__ldcg(l)};
                 l[0] = 0ULL;
                 l[1] = 0ULL;
-                tot[i] += ((double)l1 * 4294967296.0 + (double)l0) * unfix_factor(p.src[e].amax[i % C], eb);
+                const double v = fix_value(f, p.src[e].amax[i % C]);
+                p.src_sums[e][i] = v;
+                tot[i] += v;
             }
             __syncthreads();
             continue;
         }
-        const int nparts = gr.first[e + 1] - gr.first[e];  // at most AP_PART_BLOCKS
+        const int nparts = gr.first[e * gr.halves + 1] - gr.first[e * gr.halves];  // of every half
         const double* part = p.partials + (size_t)e * AP_PART_BLOCKS * P;
         for (int i0 = 0; i0 < P; i0 += Pr) {  // Pr pairs at a time, AP_THREADS / Pr slices of the blocks
             const int ns = AP_THREADS / Pr;
@@ -481,6 +550,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_small_kernel(ApSmall<T> p, ApSm
             if (sl == 0 && i < P) {
                 double w = 0.0;
                 for (int k = 0; k < ns; ++k) w += fold[k * Pr + threadIdx.x];
+                p.src_sums[e][i] = w;
                 tot[i] += w;
             }
             __syncthreads();
@@ -614,6 +684,8 @@ __global__ void __launch_bounds__(256) count_small_kernel(const int32_t* __restr
 
 // largest value the shared memory of a visit may take
 constexpr int AP_SMEM = 200 * 1024;
+// per-warp sums of the widest half of a small dimension (32 groups, 32 columns)
+constexpr size_t AP_SMALL_SMEM = 132 * 1024;
 
 unsigned ap_row_blocks(long long G, int C) {
     const int rps = AP_THREADS / C;
@@ -627,16 +699,12 @@ template <typename T>
 int launch_ap_visit(const ApVisit<T>& p, cudaStream_t s) {
     if (p.t.G <= 0) return 0;
     if (p.t.C > 32) return set_error("group-table projection: %d columns", p.t.C);
-    unsigned mask = 0;
-    size_t smem = sizeof(unsigned long long) * AP_THREADS;
-    for (int e = 0; e < p.n_dense; ++e) {
-        if (sizeof(T) == 8 && !p.dense[e].wide && fix_ok(p.dense[e].Gs, p.dense[e].max_count)) mask |= 1u << e;
-        smem += sizeof(T) * (size_t)p.dense[e].Gs * p.t.C;
-    }
+    size_t smem = sizeof(unsigned long long) * (AP_THREADS + 32);
+    for (int e = 0; e < p.n_dense && !p.small_known; ++e) smem += sizeof(T) * (size_t)p.dense[e].pitch * p.t.C;
     static const cudaError_t attr =
         cudaFuncSetAttribute(ap_visit_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM);
     if (attr != cudaSuccess) return set_cuda_error(attr, "group-table projection attr");
-    ap_visit_kernel<T><<<ap_row_blocks(p.t.G, p.t.C), AP_THREADS, smem, s>>>(p, mask);
+    ap_visit_kernel<T><<<ap_row_blocks(p.t.G, p.t.C), AP_THREADS, smem, s>>>(p);
     FEGB_LAUNCH_CHECK("group-table projection");
     return 0;
 }
@@ -655,12 +723,12 @@ template int launch_ap_repeat<double>(const ApTables<double>&, int, const ApCtl*
 
 size_t ap_small_scratch(int Gs, int C, int n_src) { return (size_t)Gs * C * AP_PART_BLOCKS * std::max(1, n_src); }
 
-template <typename T, int NP>
-int launch_ap_small_np(const ApSmall<T>& p, const ApSmallGrid& gr, size_t smem, cudaStream_t s) {
+template <typename T, int GT>
+int launch_ap_small_gt(const ApSmall<T>& p, const ApSmallGrid& gr, size_t smem, cudaStream_t s) {
     static const cudaError_t attr =
-        cudaFuncSetAttribute(ap_small_kernel<T, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM);
+        cudaFuncSetAttribute(ap_small_kernel<T, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMALL_SMEM);
     if (attr != cudaSuccess) return set_cuda_error(attr, "small-dimension projection attr");
-    ap_small_kernel<T, NP><<<gr.first[p.n_src], AP_THREADS, smem, s>>>(p, gr);
+    ap_small_kernel<T, GT><<<gr.first[p.n_src * gr.halves], AP_THREADS, smem, s>>>(p, gr);
     FEGB_LAUNCH_CHECK("small-dimension projection");
     return 0;
 }
@@ -671,22 +739,20 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s) {
     if (Gs <= 0) return 0;
     if (Gs > DENSE_SMALL_MAX_G || C > 32 || p.n_src < 1) return set_error("small-dimension projection: G=%d C=%d", Gs, C);
     ApSmallGrid gr{};
-    size_t smem = 0;
-    for (int e = 0; e < p.n_src; ++e) {
-        const ApDense<T>& D = p.src[e];
-        const bool fx = sizeof(T) == 8 && !D.wide && fix_ok(AP_FLUSH, D.max_count);
-        if (fx) gr.fixed_mask |= 1u << e;
-        const int tiles = (D.Ge + AP_TILE - 1) / AP_TILE;
-        gr.first[e + 1] = gr.first[e] + std::max(1, std::min(tiles, fx ? AP_FIX_BLOCKS : AP_PART_BLOCKS));
-        smem = std::max(smem, 2 * (sizeof(T) * (size_t)AP_TILE * p.t.ld + (size_t)AP_TILE * Gs * (D.wide ? 4 : 1)));
-    }
+    gr.halves = Gs > AP_HALF ? 2 : 1;
     // the fold: totals, one value per thread, column and warp maxima
-    smem = std::max(smem, sizeof(double) * ((size_t)P + AP_THREADS + C + 8));
-    smem = std::max(smem, sizeof(double) * (size_t)AP_THREADS);
-    if (P <= AP_THREADS) return launch_ap_small_np<T, 1>(p, gr, smem, s);
-    if (P <= 2 * AP_THREADS) return launch_ap_small_np<T, 2>(p, gr, smem, s);
-    if (P <= 4 * AP_THREADS) return launch_ap_small_np<T, 4>(p, gr, smem, s);
-    return launch_ap_small_np<T, 8>(p, gr, smem, s);
+    const size_t per_warp = (sizeof(T) == 8 ? 2 * sizeof(long long) : sizeof(float)) * (size_t)std::min(Gs, AP_HALF) * C;
+    const size_t smem = std::max(sizeof(double) * ((size_t)P + AP_THREADS + C + 8), per_warp * (AP_THREADS / 32));
+    const long long per_block = (long long)(AP_THREADS / 32) * (32 / C) * AP_DEPTH;
+    for (int e = 0; e < p.n_src; ++e) {
+        const long long want = (p.src[e].Ge + per_block - 1) / per_block;
+        const int nb = (int)std::max(1LL, std::min<long long>(want, sizeof(T) == 8 ? AP_FIX_BLOCKS : AP_PART_BLOCKS));
+        for (int h = 0; h < gr.halves; ++h) gr.first[e * gr.halves + h + 1] = gr.first[e * gr.halves + h] + nb;
+    }
+    if (Gs <= 8) return launch_ap_small_gt<T, 8>(p, gr, smem, s);
+    if (Gs <= 16) return launch_ap_small_gt<T, 16>(p, gr, smem, s);
+    if (Gs <= 24) return launch_ap_small_gt<T, 24>(p, gr, smem, s);
+    return launch_ap_small_gt<T, AP_HALF>(p, gr, smem, s);
 }
 template int launch_ap_small<float>(const ApSmall<float>&, cudaStream_t);
 template int launch_ap_small<double>(const ApSmall<double>&, cudaStream_t);
@@ -704,8 +770,8 @@ int launch_ap_check(const ApSlot* slots, int n_fe, int half, ApCtl* ctl, cudaStr
     return 0;
 }
 
-int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int Gs, uint8_t* N8, uint32_t* N32,
-                       unsigned* mx, cudaStream_t s) {
+int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int Gs, uint8_t* N8,
+                       uint32_t* N32, unsigned* mx, cudaStream_t s) {
     FEGB_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned), s), "count max reset");
     if (Ge <= 0 || n <= 0) return 0;
     // about 4096 rows a block, at most 32 KB of counts and 8 KB of offsets

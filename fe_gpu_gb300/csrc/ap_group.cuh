@@ -11,8 +11,8 @@
 // the number of iterations; an iteration moves the group tables, the id tuples
 // and the count matrices.
 // FP64 form, whole fits, rows -> tables: 13M rows over 4142/13/12 groups, 4
-// columns 64.7 -> 12.3 ms; 2M rows over 100k/12k/20 groups, 12 columns 281 -> 63
-// ms; 5M rows over 940k/13/12, 4 columns 40.0 -> 20.6 ms; 800 rows 6.6 -> 1.8 ms.
+// columns 72 -> 12.4 ms; 2M rows over 100k/12k/20 groups, 12 columns 180 -> 24
+// ms; 5M rows over 940k/13/12, 4 columns 39 -> 15.8 ms; 800 rows 6.4 -> 1.9 ms.
 //
 // A visit of a dimension evaluates the coupling sum once and runs one
 // projection; the symmetric order projects its end dimensions twice in a row,
@@ -51,12 +51,15 @@ struct ApCtl {
     int stop;           // set when an iteration stayed below tol: later launches return at once
 };
 
-// Count matrix of a small dimension s against a dimension e, G_e x Gs.
+// Count matrix of a small dimension s against a dimension e: entry (g, t) at
+// N[g * pitch + t], pitch = ap_count_pitch(Gs), so that rows start on 4 bytes.
+inline int ap_count_pitch(int Gs) { return (Gs + 3) & ~3; }
 template <typename T>
 struct ApDense {
     const void* N;     // uint8, or uint32 when wide
     int wide;
     int Gs;
+    int pitch;
     int max_count;
     const T* tab;      // visit: the small dimension's table; small: the table of e
     const unsigned long long* amax;  // per column: bits of max |tab| so far
@@ -81,6 +84,10 @@ struct ApVisit {
     ApTables<T> t;
     int slot;
     const ApCtl* ctl;
+    // the small sources' coupling sums (G x C): stored by a visit that computes
+    // them, read instead by one that finds the small dimensions unchanged
+    double* small_sums;
+    int small_known;
     // swept sources: complete sums of -(weighted source rows) (G x C), or the
     // group's positions (off set), or neither
     const T* sums;
@@ -99,10 +106,13 @@ struct ApSmall {
     int slot;
     int projections;  // 1 or 2 in a row
     const ApCtl* ctl;
-    int n_src;
+    int n_src;                   // the sources that changed since the last visit (at least one)
     ApDense<T> src[SWEEP_MAXP];
+    double* src_sums[SWEEP_MAXP];  // Gs x C: coupling sums of each source, written
+    int n_kept;                  // the other sources: their sums of an earlier visit
+    const double* kept[SWEEP_MAXP];
     double* partials;            // ap_small_scratch() doubles
-    unsigned long long* limbs;   // 2 x Gs x C, zero between launches
+    unsigned long long* limbs;   // 2 x Gs x C per source, zero between launches
     unsigned* counter;           // zero between launches
 };
 
@@ -123,18 +133,19 @@ int launch_ap_reset(ApSlot* slots, const double* relax, const double* prev_chang
 // largest update against the tolerance.
 int launch_ap_check(const ApSlot* slots, int n_fe, int half, ApCtl* ctl, cudaStream_t s);
 
-// Row counts of the (group of e, group of s) pairs, N[g * Gs + t], s with at
-// most DENSE_SMALL_MAX_G groups; *mx (device) = the largest count.
+// Row counts of the (group of e, group of s) pairs, N[g * pitch + t], s with at
+// most DENSE_SMALL_MAX_G groups (pitch >= Gs, entries past Gs zero); *mx
+// (device) = the largest count.
 // Sorted form: off (G_e + 1) are e's groups in the row order of gid_s, no group
 // longer than AP_COUNT_LONGEST rows. N8 receives the counts, clamped to 255
 // (exact when *mx < 256); N32, when set, the counts as they are.
 constexpr int AP_COUNT_LONGEST = 1 << 16;
-int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int Gs, uint8_t* N8, uint32_t* N32,
-                       unsigned* mx, cudaStream_t s);
+int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int pitch, uint8_t* N8,
+                       uint32_t* N32, unsigned* mx, cudaStream_t s);
 // Form for matrices of at most AP_COUNT_SMALL entries, any row order; N is
 // zeroed by the call.
 constexpr int AP_COUNT_SMALL = 12 * 1024;
-int count_pairs_small(const int32_t* gid_e, int Ge, const int32_t* gid_s, long long n, int Gs, uint32_t* N,
+int count_pairs_small(const int32_t* gid_e, int Ge, const int32_t* gid_s, long long n, int pitch, uint32_t* N,
                       cudaStream_t s);
 
 }  // namespace fegb

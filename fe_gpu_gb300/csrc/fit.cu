@@ -1324,13 +1324,14 @@ int cg_schur_precond(Problem& P, CGBuffers<T>& B) {
     return 0;
 }
 
-// Count matrix of a small dimension d and a dimension e (G_e x G_d), uint8 when
-// every count is below 256. mx: a device word.
+// Count matrix of a small dimension d and a dimension e (G_e rows of `pitch`
+// counts, the first G_d used), uint8 when every count is below 256. mx: a
+// device word.
 template <typename T>
-int count_matrix(Problem& P, CGBuffers<T>& B, int d, int e, unsigned* mx) {
+int count_matrix(Problem& P, CGBuffers<T>& B, int d, int e, int pitch, unsigned* mx) {
     Scratch& scr = *P.scr;
     const Dim &De = P.dims[e], &Dd = P.dims[d];
-    const size_t cnt = (size_t)De.G * Dd.G;
+    const size_t cnt = (size_t)De.G * pitch;
     unsigned hmx = 0;
     // the primary's rows are in storage order: counted block by block without
     // the 4-byte matrix in between, unless one group holds very many rows
@@ -1339,22 +1340,22 @@ int count_matrix(Problem& P, CGBuffers<T>& B, int d, int e, unsigned* mx) {
         FEGB_TRY(max_group_length(De.off, De.G, &longest, P.s));
     if (longest <= AP_COUNT_LONGEST) {
         FEGB_TRY(dalloc(scr, &B.N8[d][e], cnt, "count matrix (uint8)"));
-        FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, Dd.G, B.N8[d][e], nullptr, mx, P.s));
+        FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, pitch, B.N8[d][e], nullptr, mx, P.s));
         FEGB_TRY(d2h_sync(&hmx, mx, sizeof(hmx), P.s, "count max copy"));
         if (hmx >= 256) {
             B.N8[d][e] = nullptr;
             FEGB_TRY(dalloc(scr, &B.N32[d][e], cnt, "count matrix (uint32)"));
-            FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, Dd.G, nullptr, B.N32[d][e], mx, P.s));
+            FEGB_TRY(count_pairs_sorted(De.off, De.G, Dd.gid, P.n, pitch, nullptr, B.N32[d][e], mx, P.s));
         }
     } else {
         Scratch tmp(P.s);  // the uint32 counts, released once narrowed or copied
         uint32_t* N = nullptr;
         FEGB_TRY(tmp.alloc(&N, cnt, "count matrix"));
         if (cnt <= (size_t)AP_COUNT_SMALL) {
-            FEGB_TRY(count_pairs_small(De.gid, De.G, Dd.gid, P.n, Dd.G, N, P.s));
+            FEGB_TRY(count_pairs_small(De.gid, De.G, Dd.gid, P.n, pitch, N, P.s));
         } else {
             FEGB_CUDA(cudaMemsetAsync(N, 0, sizeof(uint32_t) * cnt, P.s), "count matrix zero");
-            FEGB_TRY(launch_count_pairs(De.gid, Dd.gid, P.n, Dd.G, N, P.s));
+            FEGB_TRY(launch_count_pairs(De.gid, Dd.gid, P.n, pitch, N, P.s));
         }
         FEGB_TRY(launch_count_max(N, (long long)cnt, mx, P.s));
         FEGB_TRY(d2h_sync(&hmx, mx, sizeof(hmx), P.s, "count max copy"));
@@ -1498,7 +1499,7 @@ int cg_alloc(Problem& P, CGBuffers<T>& B) {
                 sums += (long long)P.dims[d].G * C;
                 for (int e = 0; e < P.n_fe; ++e) {
                     if (e == d || P.dims[e].G <= 0) continue;
-                    FEGB_TRY(count_matrix(P, B, d, e, mx));
+                    FEGB_TRY(count_matrix(P, B, d, e, P.dims[d].G, mx));
                     parts += (long long)dense_chunks(P.dims[e].G) * P.dims[d].G * C;
                 }
             }
@@ -2102,6 +2103,15 @@ struct ApGroups {
     unsigned long long* limbs = nullptr;
     unsigned* counter = nullptr;
     std::vector<std::vector<int>> max_count;  // [small][e]
+    // Coupling sums kept between visits. A dimension between the end ones is
+    // visited from both sides, so at each visit only the side it comes from has
+    // changed: version[e] counts the projections of e, seen[d][e] is the version
+    // that d's kept sums of e were formed from.
+    std::vector<long long> version;
+    std::vector<std::vector<long long>> seen;
+    std::vector<std::vector<double*>> pair_sums;  // [small][e]: Gs x C
+    std::vector<double*> small_sums;              // [swept]: its sums over the small dimensions (G x C)
+    std::vector<T*> swept_sums;                   // [swept]: its sums over the swept ones, chunked streams (G x C)
     ApPoll poll;
 
     int build(Problem& P) {
@@ -2113,6 +2123,10 @@ struct ApGroups {
         B.N8.assign(P.n_fe, std::vector<uint8_t*>(P.n_fe, nullptr));
         B.N32.assign(P.n_fe, std::vector<uint32_t*>(P.n_fe, nullptr));
         max_count.assign(P.n_fe, std::vector<int>(P.n_fe, 0));
+        pair_sums.assign(P.n_fe, std::vector<double*>(P.n_fe, nullptr));
+        seen.assign(P.n_fe, std::vector<long long>(P.n_fe, -1));
+        small_sums.assign(P.n_fe, nullptr);
+        swept_sums.assign(P.n_fe, nullptr);
         std::vector<int> Gd(P.n_fe);
         for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
         const std::vector<char> plan = cg_dense_plan(Gd, C, P.n);
@@ -2125,14 +2139,22 @@ struct ApGroups {
             B.any_dense = true;
             for (int e = 0; e < P.n_fe; ++e) {
                 if (e == d || P.dims[e].G <= 0) continue;
-                FEGB_TRY(count_matrix(P, B, d, e, mx));
+                FEGB_TRY(count_matrix(P, B, d, e, ap_count_pitch(Gd[d]), mx));
                 max_count[d][e] = P.pair_max[d][e];
+                FEGB_TRY(dalloc(scr, &pair_sums[d][e], (size_t)Gd[d] * C, "small coupling sums"));
             }
             part = std::max(part, ap_small_scratch(Gd[d], C, P.n_fe - 1));
             limb = std::max(limb, (size_t)2 * Gd[d] * C * std::max(1, P.n_fe - 1));
         }
         FEGB_TRY(operator_streams(P, B));
         FEGB_TRY(operator_sums(P, B));
+        // dimensions visited from both sides, with sources of both kinds
+        for (int d = 0; d < P.n_fe; ++d) {
+            const auto& st = B.stream[d];
+            if (B.dense[d] || Gd[d] <= 0 || st.n_src == 0 || st.short_groups) continue;
+            FEGB_TRY(dalloc(scr, &swept_sums[d], (size_t)Gd[d] * C, "swept coupling sums"));
+            if (B.any_dense) FEGB_TRY(dalloc(scr, &small_sums[d], (size_t)Gd[d] * C, "small coupling sums"));
+        }
         const size_t np = (size_t)std::max(1LL, P.Gt) * B.ld;
         FEGB_TRY(dalloc(scr, &B.p, np, "group tables"));
         FEGB_TRY(dalloc(scr, &base, (size_t)std::max(1LL, P.Gt) * C, "coupling sums"));
@@ -2170,6 +2192,7 @@ struct ApGroups {
         m.wide = B.N8[s][e] ? 0 : 1;
         m.N = B.N8[s][e] ? static_cast<const void*>(B.N8[s][e]) : static_cast<const void*>(B.N32[s][e]);
         m.Gs = P.dims[s].G;
+        m.pitch = ap_count_pitch(m.Gs);
         m.Ge = P.dims[e].G;
         m.max_count = max_count[s][e];
         m.tab = B.p + P.goff[of] * B.ld;
@@ -2181,6 +2204,7 @@ struct ApGroups {
     int visit(Problem& P, int d, int slot, int projections) {
         if (P.dims[d].G <= 0) return 0;
         P.projections += projections;
+        version[d] += projections;
         if (B.dense[d]) {
             ApSmall<T> q{};
             q.t = tables(P, d);
@@ -2191,11 +2215,22 @@ struct ApGroups {
             q.limbs = limbs;
             q.counter = counter;
             double bytes = 0.0;
+            int last = -1;  // with nothing changed, one source is formed again
             for (int e = 0; e < P.n_fe; ++e)
-                if (e != d && P.dims[e].G > 0) {
-                    q.src[q.n_src++] = matrix(P, d, e, e);
-                    bytes += (double)P.dims[e].G * ((B.N8[d][e] ? 1.0 : 4.0) * P.dims[d].G + (double)P.C * sizeof(T));
+                if (e != d && P.dims[e].G > 0) last = e;
+            bool changed = false;
+            for (int e = 0; e < P.n_fe; ++e) changed = changed || (e != d && P.dims[e].G > 0 && seen[d][e] != version[e]);
+            for (int e = 0; e < P.n_fe; ++e) {
+                if (e == d || P.dims[e].G <= 0) continue;
+                if (seen[d][e] == version[e] && (changed || e != last)) {
+                    q.kept[q.n_kept++] = pair_sums[d][e];
+                    continue;
                 }
+                q.src_sums[q.n_src] = pair_sums[d][e];
+                q.src[q.n_src++] = matrix(P, d, e, e);
+                seen[d][e] = version[e];
+                bytes += (double)P.dims[e].G * ((B.N8[d][e] ? 1.0 : 4.0) * P.dims[d].G + (double)P.C * sizeof(T));
+            }
             if (q.n_src > 0) {
                 CGTimer tm(P);
                 FEGB_TRY(tm.begin(6 + (sizeof(T) == 4 ? 1 : 0), bytes));
@@ -2222,14 +2257,26 @@ struct ApGroups {
                 v.weight = st.weight;
                 bytes += (double)st.m * (4.0 * st.n_src + (st.weight ? 4.0 : 0.0) + (double)st.n_src * P.C * sizeof(T));
             } else {
-                int n_src = 0;
-                FEGB_TRY(cg_sweep<T>(P, B, d, &n_src, &ctl->stop));
-                v.sums = B.sums;
+                bool known = true;
+                for (int i = 0; i < st.n_src; ++i) known = known && seen[d][st.src_dim[i]] == version[st.src_dim[i]];
+                if (!known) {
+                    int n_src = 0;
+                    std::swap(B.sums, swept_sums[d]);
+                    const int rc = cg_sweep<T>(P, B, d, &n_src, &ctl->stop);
+                    std::swap(B.sums, swept_sums[d]);
+                    FEGB_TRY(rc);
+                    for (int i = 0; i < st.n_src; ++i) seen[d][st.src_dim[i]] = version[st.src_dim[i]];
+                }
+                v.sums = swept_sums[d];
             }
         }
+        v.small_sums = small_sums[d];
+        v.small_known = small_sums[d] ? 1 : 0;
         for (int s = 0; s < P.n_fe; ++s)
             if (s != d && B.dense[s] && P.dims[s].G > 0) {
                 v.dense[v.n_dense++] = matrix(P, s, d, s);
+                if (seen[d][s] != version[s]) v.small_known = 0;
+                seen[d][s] = version[s];
                 bytes += (double)P.dims[d].G * (B.N8[s][d] ? 1.0 : 4.0) * P.dims[s].G;
             }
         CGTimer tm(P);
@@ -2254,6 +2301,7 @@ struct ApGroups {
         for (; i < seq.size() && seq[i] == P.order[0]; ++i) {
             const int d = seq[i];
             FEGB_TRY(launch_ap_repeat<T>(tables(P, d), next[d]++, ctl, P.s));
+            version[d] += 1;
             P.projections += P.dims[d].G > 0;
         }
         while (i < seq.size()) {
@@ -2277,6 +2325,8 @@ struct ApGroups {
         if (sizeof(T) == 4)
             FEGB_CUDA(cudaMemsetAsync(P.alpha_all, 0, sizeof(double) * (size_t)std::max(1LL, P.Gt) * C, P.s),
                       "alpha zero");
+        version.assign(P.n_fe, 0);
+        for (auto& v : seen) std::fill(v.begin(), v.end(), -1);
         const int d0 = P.order[0];  // no updates yet: its coupling sums are zero
         FEGB_CUDA(cudaMemcpyAsync(base + P.goff[d0] * C, P.dims[d0].mu, sizeof(double) * (size_t)P.dims[d0].G * C,
                                   cudaMemcpyDeviceToDevice, P.s),
