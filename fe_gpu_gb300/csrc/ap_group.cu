@@ -110,11 +110,18 @@ __device__ __forceinline__ unsigned long long update_bits(double v) {
 }
 
 // One projection of element idx = (g, c): the new table value; mixed -> *upd.
+// With t.means set, the residual's new mean instead.
 template <typename T>
 __device__ __forceinline__ double ap_update(const ApTables<T>& t, long long g, int c, double base, double relax,
                                             double* upd) {
     const long long idx = g * t.C + c;
     T* slot = t.tab + g * t.ld + c;
+    if (t.means) {
+        const double m = t.inv[g] != 0.0 ? base - (double)*slot : 0.0;
+        t.means[idx] = m;
+        *upd = m;
+        return 0.0;
+    }
     const double a = sizeof(T) == 8 ? (double)*slot : t.alpha64[idx];
     const double mean = base - a;
     const double pv = t.prev[idx];
@@ -175,29 +182,51 @@ __device__ __forceinline__ T dense_dot(const CT* __restrict__ N, int Gs, const T
     for (; t < Gs; ++t) a = fma((T)N[t], tab[t * C + c], a);
     return a;
 }
-// the same in fixed point; rows of N start on 4 counts and are zero past Gs, as
-// the table is up to a multiple of four rows
-__device__ __forceinline__ void dense_dot_fixed(const uint8_t* __restrict__ N, int pitch,
-                                                const FixDigits* __restrict__ tab, int C, int c, FixSum& a) {
-#pragma unroll 2
-    for (int t = 0; t < pitch; t += 4) {
-        const unsigned w = *reinterpret_cast<const unsigned*>(N + t);
-        fix_add(a, w & 255u, tab[t * C + c]);
-        fix_add(a, (w >> 8) & 255u, tab[(t + 1) * C + c]);
-        fix_add(a, (w >> 16) & 255u, tab[(t + 2) * C + c]);
-        fix_add(a, w >> 24, tab[(t + 3) * C + c]);
+// the 16 counts of piece w of a row, in order
+struct Counts16 {
+    unsigned n[AP_PART];
+};
+__device__ __forceinline__ Counts16 load_counts(const uint8_t* row, int w) {
+    const uint4 x = reinterpret_cast<const uint4*>(row)[w];
+    const unsigned q[4] = {x.x, x.y, x.z, x.w};
+    Counts16 r;
+#pragma unroll
+    for (int i = 0; i < AP_PART; ++i) r.n[i] = (q[i / 4] >> (8 * (i % 4))) & 255u;
+    return r;
+}
+__device__ __forceinline__ Counts16 load_counts(const uint32_t* row, int w) {
+    Counts16 r;
+#pragma unroll
+    for (int i = 0; i < AP_PART / 4; ++i) {
+        const uint4 x = reinterpret_cast<const uint4*>(row)[w * (AP_PART / 4) + i];
+        r.n[4 * i] = x.x;
+        r.n[4 * i + 1] = x.y;
+        r.n[4 * i + 2] = x.z;
+        r.n[4 * i + 3] = x.w;
+    }
+    return r;
+}
+
+// the same in fixed point; tab is zero past Gs, up to a multiple of four rows
+template <typename CT>
+__device__ __forceinline__ void dense_dot_fixed(const void* N, long long g, int Gs, const FixDigits* __restrict__ tab,
+                                                int C, int c, FixSum& a) {
+    const CT* row = static_cast<const CT*>(N) + g * ap_count_pitch(Gs);
+    for (int t0 = 0; t0 < Gs; t0 += AP_PART) {
+        const Counts16 n = load_counts(row, t0 / AP_PART);
+#pragma unroll
+        for (int i = 0; i < AP_PART; i += 4) {
+            if (t0 + i >= Gs) break;
+            const FixDigits* __restrict__ q = tab + (t0 + i) * C + c;
+            fix_add(a, n.n[i], q[0]);
+            fix_add(a, n.n[i + 1], q[C]);
+            fix_add(a, n.n[i + 2], q[2 * C]);
+            fix_add(a, n.n[i + 3], q[3 * C]);
+        }
     }
 }
-__device__ __forceinline__ void dense_dot_fixed(const uint32_t* __restrict__ N, int pitch,
-                                                const FixDigits* __restrict__ tab, int C, int c, FixSum& a) {
-    for (int t = 0; t < pitch; t += 4) {
-        const uint4 w = *reinterpret_cast<const uint4*>(N + t);
-        fix_add(a, w.x, tab[t * C + c]);
-        fix_add(a, w.y, tab[(t + 1) * C + c]);
-        fix_add(a, w.z, tab[(t + 2) * C + c]);
-        fix_add(a, w.w, tab[(t + 3) * C + c]);
-    }
-}
+
+__host__ __device__ constexpr int four_rows(int Gs) { return (Gs + 3) & ~3; }
 
 // One visit: thread (r, c) takes column c of the block's groups r, r + rps, ...
 // The small sources' tables sit in shared memory, in the FP64 form as
@@ -220,7 +249,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
     const int c = (int)threadIdx.x - rr * C;
     const bool active = rr < rps;
     const bool small = p.n_dense > 0 && !p.small_known;
-    // small tables: entry (t, c) at dst[t * C + c], pitch rows (zero past Gs)
+    // small tables: entry (t, c) at dst[t * C + c], a multiple of four rows (zero past Gs)
     if (small) {
         if (FIX) {
             for (int i = threadIdx.x; i < C; i += AP_THREADS) {
@@ -233,7 +262,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
         T* dst = reinterpret_cast<T*>(tabs);
         for (int e = 0; e < p.n_dense; ++e) {
             const ApDense<T>& D = p.dense[e];
-            for (int i = threadIdx.x; i < D.pitch * C; i += AP_THREADS) {
+            for (int i = threadIdx.x; i < four_rows(D.Gs) * C; i += AP_THREADS) {
                 const int tt = i / C, cc = i - tt * C;
                 const T v = tt < D.Gs ? D.tab[tt * t.ld + cc] : T(0);
                 if (FIX)
@@ -241,7 +270,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
                 else
                     dst[i] = v;
             }
-            dst += D.pitch * C;
+            dst += four_rows(D.Gs) * C;
         }
     }
     const double relax = ap_relax(t.slots, p.slot);
@@ -288,10 +317,10 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
                     for (int e = 0; e < p.n_dense; ++e) {
                         const ApDense<T>& D = p.dense[e];
                         if (D.wide)
-                            dense_dot_fixed(static_cast<const uint32_t*>(D.N) + g * D.pitch, D.pitch, st, C, c, f);
+                            dense_dot_fixed<uint32_t>(D.N, g, D.Gs, st, C, c, f);
                         else
-                            dense_dot_fixed(static_cast<const uint8_t*>(D.N) + g * D.pitch, D.pitch, st, C, c, f);
-                        st += D.pitch * C;
+                            dense_dot_fixed<uint8_t>(D.N, g, D.Gs, st, C, c, f);
+                        st += four_rows(D.Gs) * C;
                     }
                     sm = fix_value(f, cmax[c]);
                 } else {
@@ -300,10 +329,10 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
                     for (int e = 0; e < p.n_dense; ++e) {
                         const ApDense<T>& D = p.dense[e];
                         if (D.wide)
-                            f += dense_dot<T>(static_cast<const uint32_t*>(D.N) + g * D.pitch, D.Gs, st, C, c);
+                            f += dense_dot<T>(static_cast<const uint32_t*>(D.N) + g * ap_count_pitch(D.Gs), D.Gs, st, C, c);
                         else
-                            f += dense_dot<T>(static_cast<const uint8_t*>(D.N) + g * D.pitch, D.Gs, st, C, c);
-                        st += D.pitch * C;
+                            f += dense_dot<T>(static_cast<const uint8_t*>(D.N) + g * ap_count_pitch(D.Gs), D.Gs, st, C, c);
+                        st += four_rows(D.Gs) * C;
                     }
                     sm = (double)f;
                 }
@@ -311,7 +340,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
                 cpl = (p.sums || p.off) ? cpl + sm : sm;
             }
             const double base = fma(-cpl, t.inv[g], t.mu[idx]);
-            t.base[idx] = base;
+            if (!t.means) t.base[idx] = base;
             double u;
             const double an = ap_update(t, g, c, base, relax, &u);
             upd = umax64(upd, update_bits(u));
@@ -348,11 +377,15 @@ __global__ void __launch_bounds__(AP_THREADS) ap_repeat_kernel(ApTables<T> t, in
 constexpr int AP_DEPTH = 4;
 constexpr int AP_PART_BLOCKS = 152;
 constexpr int AP_FIX_BLOCKS = 304;
-constexpr int AP_HALF = 32;  // groups of the small dimension per block: two blocks share a larger one
+
+// A block takes all groups of a small dimension of up to AP_WHOLE groups (what the
+// registers hold), else one part of AP_PART of them.
+constexpr int AP_WHOLE = 24;
+constexpr int AP_PARTS = DENSE_SMALL_MAX_G / AP_PART;
 
 struct ApSmallGrid {
-    int first[2 * SWEEP_MAXP + 1];  // first block of each (source, half)
-    int halves;
+    int first[AP_PARTS * SWEEP_MAXP + 1];  // first block of each (source, part of the small dimension)
+    int parts;                            // parts of the small dimension
 };
 
 // sums over a warp's slots (lane = slot * C + c): valid in the lanes of slot 0
@@ -365,51 +398,45 @@ __device__ __forceinline__ V warp_slot_sum(V v, int slot, int slots, int C, int 
     return v;
 }
 
-// the four counts at N[4 w .. 4 w + 3] of a row
-__device__ __forceinline__ uint4 four_counts(const uint8_t* row, int w) {
-    const unsigned x = reinterpret_cast<const unsigned*>(row)[w];
-    return make_uint4(x & 255u, (x >> 8) & 255u, (x >> 16) & 255u, x >> 24);
-}
-__device__ __forceinline__ uint4 four_counts(const uint32_t* row, int w) { return reinterpret_cast<const uint4*>(row)[w]; }
-
-// acc[t] += N[g][t] * tab[g][c] over this lane's groups
+// acc[t] += N[g][t] * tab[g][c] over this lane's groups, t from piece w of the rows on
 template <typename CT, int GT>
-__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int t0, int words,
-                                           const double* __restrict__ tab, int ld, int c, int k, long long g,
-                                           long long Ge, long long gstep, FixSum (&acc)[GT]) {
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const double* __restrict__ tab,
+                                           int ld, int c, int k, long long g, long long Ge, long long gstep,
+                                           FixSum (&acc)[GT]) {
 #pragma unroll 2
     for (; g < Ge; g += gstep) {
-        const CT* __restrict__ row = N + g * pitch + t0;
         const FixDigits a = fix_digits(to_fixed(tab[g * ld + c], k));
 #pragma unroll
-        for (int w = 0; w < GT / 4; ++w) {
-            if (w >= words) break;
-            const uint4 x = four_counts(row, w);
-            fix_add(acc[4 * w], x.x, a);
-            fix_add(acc[4 * w + 1], x.y, a);
-            fix_add(acc[4 * w + 2], x.z, a);
-            fix_add(acc[4 * w + 3], x.w, a);
+        for (int q = 0; q < GT; q += AP_PART) {
+            const Counts16 n = load_counts(N + g * pitch, w + q / AP_PART);
+#pragma unroll
+            for (int i = 0; i < AP_PART && q + i < GT; ++i) fix_add(acc[q + i], n.n[i], a);
         }
     }
 }
 template <typename CT, int GT>
-__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int t0, int words,
-                                           const float* __restrict__ tab, int ld, int c, int, long long g,
-                                           long long Ge, long long gstep, float (&acc)[GT]) {
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const float* __restrict__ tab,
+                                           int ld, int c, int, long long g, long long Ge, long long gstep,
+                                           float (&acc)[GT]) {
 #pragma unroll 2
     for (; g < Ge; g += gstep) {
-        const CT* __restrict__ row = N + g * pitch + t0;
         const float a = tab[g * ld + c];
 #pragma unroll
-        for (int w = 0; w < GT / 4; ++w) {
-            if (w >= words) break;
-            const uint4 x = four_counts(row, w);
-            acc[4 * w] = fmaf((float)x.x, a, acc[4 * w]);
-            acc[4 * w + 1] = fmaf((float)x.y, a, acc[4 * w + 1]);
-            acc[4 * w + 2] = fmaf((float)x.z, a, acc[4 * w + 2]);
-            acc[4 * w + 3] = fmaf((float)x.w, a, acc[4 * w + 3]);
+        for (int q = 0; q < GT; q += AP_PART) {
+            const Counts16 n = load_counts(N + g * pitch, w + q / AP_PART);
+#pragma unroll
+            for (int i = 0; i < AP_PART && q + i < GT; ++i) acc[q + i] = fmaf((float)n.n[i], a, acc[q + i]);
         }
     }
+}
+template <int GT, typename T, typename A>
+__device__ __forceinline__ void small_walk_any(const ApDense<T>& D, int w, int ld, int c, int k, long long g,
+                                               long long gstep, A (&acc)[GT]) {
+    const int pitch = ap_count_pitch(D.Gs);
+    if (D.wide)
+        small_walk<uint32_t, GT>(static_cast<const uint32_t*>(D.N), pitch, w, D.tab, ld, c, k, g, D.Ge, gstep, acc);
+    else
+        small_walk<uint8_t, GT>(static_cast<const uint8_t*>(D.N), pitch, w, D.tab, ld, c, k, g, D.Ge, gstep, acc);
 }
 
 // Small dimension: sum_g N[g][t] tab[g][c] of one source for up to GT of its
@@ -424,7 +451,7 @@ __device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, 
 // 100k x 20 and 12k x 20 counts, 12 columns: 81 us with FP64 sums of both
 // operands in shared memory, 41 us in this form; 940k x 13, 4 columns: 75 -> 44.
 template <typename T, int GT>
-__global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2) ap_small_kernel(ApSmall<T> p, ApSmallGrid gr) {
+__global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > AP_PART ? 1 : 2) ap_small_kernel(ApSmall<T> p, ApSmallGrid gr) {
     if (p.ctl->stop) return;
     extern __shared__ __align__(16) unsigned char ap_smem[];
     __shared__ bool s_last;
@@ -434,10 +461,10 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
     const int C = t.C, Gs = t.G;
     const int P = Gs * C;
     int part = 0;
-    while (part + 1 < p.n_src * gr.halves && (int)blockIdx.x >= gr.first[part + 1]) ++part;
-    const int src = part / gr.halves;
-    const int t0 = (part - src * gr.halves) * AP_HALF;
-    const int nt = min(Gs - t0, gr.halves > 1 ? AP_HALF : Gs);
+    while (part + 1 < p.n_src * gr.parts && (int)blockIdx.x >= gr.first[part + 1]) ++part;
+    const int src = part / gr.parts;
+    const int t0 = (part - src * gr.parts) * AP_PART;
+    const int nt = gr.parts > 1 ? min(Gs - t0, AP_PART) : Gs;
     const ApDense<T>& D = p.src[src];
     const int nb = gr.first[part + 1] - gr.first[part], b = (int)blockIdx.x - gr.first[part];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -446,7 +473,6 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
     int top = 1;
     while (top < slots) top <<= 1;
     top >>= 1;
-    const int words = (nt + 3) / 4;
     const long long gstep = (long long)nb * WARPS * slots;
     const long long g0 = slot < slots ? ((long long)b * WARPS + warp) * slots + slot : D.Ge;
     const int PB = nt * C;  // sums of this block
@@ -455,12 +481,7 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
 #pragma unroll
         for (int i = 0; i < GT; ++i) acc[i] = FixSum{0, 0};
         const int k = fix_exponent(D.amax[c]);
-        if (D.wide)
-            small_walk<uint32_t, GT>(static_cast<const uint32_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, k, g0, D.Ge,
-                                     gstep, acc);
-        else
-            small_walk<uint8_t, GT>(static_cast<const uint8_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, k, g0, D.Ge,
-                                    gstep, acc);
+        small_walk_any<GT>(D, t0 / AP_PART, t.ld, c, k, g0, gstep, acc);
         long long* red = reinterpret_cast<long long*>(ap_smem);  // WARPS x PB x 2
 #pragma unroll
         for (int i = 0; i < GT; ++i) {
@@ -482,12 +503,7 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
         float acc[GT];
 #pragma unroll
         for (int i = 0; i < GT; ++i) acc[i] = 0.f;
-        if (D.wide)
-            small_walk<uint32_t, GT>(static_cast<const uint32_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, 0, g0, D.Ge,
-                                     gstep, acc);
-        else
-            small_walk<uint8_t, GT>(static_cast<const uint8_t*>(D.N), D.pitch, t0, words, D.tab, t.ld, c, 0, g0, D.Ge,
-                                    gstep, acc);
+        small_walk_any<GT>(D, t0 / AP_PART, t.ld, c, 0, g0, gstep, acc);
         float* red = reinterpret_cast<float*>(ap_smem);  // WARPS x PB
 #pragma unroll
         for (int i = 0; i < GT; ++i) {
@@ -535,7 +551,7 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
             __syncthreads();
             continue;
         }
-        const int nparts = gr.first[e * gr.halves + 1] - gr.first[e * gr.halves];  // of every half
+        const int nparts = gr.first[e * gr.parts + 1] - gr.first[e * gr.parts];  // of every part
         const double* part = p.partials + (size_t)e * AP_PART_BLOCKS * P;
         for (int i0 = 0; i0 < P; i0 += Pr) {  // Pr pairs at a time, AP_THREADS / Pr slices of the blocks
             const int ns = AP_THREADS / Pr;
@@ -565,8 +581,8 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
             const int g = i / C, c = i - g * C;
             double base;
             if (j == 0) {
-                base = t.mu[i] - tot[i] * t.inv[g];
-                t.base[i] = base;
+                base = fma(-tot[i], t.inv[g], t.mu[i]);
+                if (!t.means) t.base[i] = base;
             } else {
                 base = t.base[i];
             }
@@ -591,6 +607,30 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > 24 ? 1 : 2)
     }
     for (int i = threadIdx.x; i < C; i += AP_THREADS)
         if (cmax[i] > t.amax[i]) t.amax[i] = cmax[i];
+}
+
+__global__ void __launch_bounds__(AP_THREADS) ap_load_kernel(const double* __restrict__ inc, long long G, int C, int ld,
+                                                             double* __restrict__ tab, double* __restrict__ total,
+                                                             unsigned long long* __restrict__ amax) {
+    __shared__ unsigned long long red[AP_THREADS];
+    const int rps = AP_THREADS / C;
+    const int rr = (int)threadIdx.x / C;
+    const int c = (int)threadIdx.x - rr * C;
+    unsigned long long m = 0;
+    if (rr < rps)
+        for (long long g = (long long)blockIdx.x * rps + rr; g < G; g += (long long)gridDim.x * rps) {
+            const double v = inc[g * C + c];
+            tab[g * ld + c] = v;
+            total[g * C + c] += v;
+            m = umax64(m, abs_bits(v));
+        }
+    red[threadIdx.x] = m;
+    __syncthreads();
+    if ((int)threadIdx.x < C) {
+        m = 0;
+        for (int j = 0; j < rps; ++j) m = umax64(m, red[j * C + threadIdx.x]);
+        if (m) atomicMax(amax + threadIdx.x, m);
+    }
 }
 
 __global__ void ap_reset_kernel(ApSlot* slots, const double* relax, const double* prev_change, int n_fe, ApCtl* ctl,
@@ -667,6 +707,17 @@ __global__ void __launch_bounds__(256) count_sorted_kernel(const int32_t* __rest
     if ((threadIdx.x & 31) == 0 && m) atomicMax(mx, m);
 }
 
+template <typename CT>
+__global__ void pad_counts_kernel(const CT* __restrict__ src, long long Ge, int Gs, int pitch, CT* __restrict__ dst) {
+    const long long total = Ge * pitch;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long g = i / pitch;
+        const int t = (int)(i - g * pitch);
+        dst[i] = t < Gs ? src[g * Gs + t] : CT(0);
+    }
+}
+
 // Pair counts of a small matrix: a table per block in shared memory, added to
 // the global one once (integers: the order does not matter).
 __global__ void __launch_bounds__(256) count_small_kernel(const int32_t* __restrict__ gid_e, int Ge,
@@ -684,8 +735,8 @@ __global__ void __launch_bounds__(256) count_small_kernel(const int32_t* __restr
 
 // largest value the shared memory of a visit may take
 constexpr int AP_SMEM = 200 * 1024;
-// per-warp sums of the widest half of a small dimension (32 groups, 32 columns)
-constexpr size_t AP_SMALL_SMEM = 132 * 1024;
+// per-warp sums of the widest block of a small dimension (24 groups, 32 columns)
+constexpr size_t AP_SMALL_SMEM = 100 * 1024;
 
 unsigned ap_row_blocks(long long G, int C) {
     const int rps = AP_THREADS / C;
@@ -700,7 +751,7 @@ int launch_ap_visit(const ApVisit<T>& p, cudaStream_t s) {
     if (p.t.G <= 0) return 0;
     if (p.t.C > 32) return set_error("group-table projection: %d columns", p.t.C);
     size_t smem = sizeof(unsigned long long) * (AP_THREADS + 32);
-    for (int e = 0; e < p.n_dense && !p.small_known; ++e) smem += sizeof(T) * (size_t)p.dense[e].pitch * p.t.C;
+    for (int e = 0; e < p.n_dense && !p.small_known; ++e) smem += sizeof(T) * (size_t)four_rows(p.dense[e].Gs) * p.t.C;
     static const cudaError_t attr =
         cudaFuncSetAttribute(ap_visit_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM);
     if (attr != cudaSuccess) return set_cuda_error(attr, "group-table projection attr");
@@ -728,7 +779,7 @@ int launch_ap_small_gt(const ApSmall<T>& p, const ApSmallGrid& gr, size_t smem, 
     static const cudaError_t attr =
         cudaFuncSetAttribute(ap_small_kernel<T, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMALL_SMEM);
     if (attr != cudaSuccess) return set_cuda_error(attr, "small-dimension projection attr");
-    ap_small_kernel<T, GT><<<gr.first[p.n_src * gr.halves], AP_THREADS, smem, s>>>(p, gr);
+    ap_small_kernel<T, GT><<<gr.first[p.n_src * gr.parts], AP_THREADS, smem, s>>>(p, gr);
     FEGB_LAUNCH_CHECK("small-dimension projection");
     return 0;
 }
@@ -739,23 +790,33 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s) {
     if (Gs <= 0) return 0;
     if (Gs > DENSE_SMALL_MAX_G || C > 32 || p.n_src < 1) return set_error("small-dimension projection: G=%d C=%d", Gs, C);
     ApSmallGrid gr{};
-    gr.halves = Gs > AP_HALF ? 2 : 1;
+    gr.parts = Gs <= AP_WHOLE ? 1 : (Gs + AP_PART - 1) / AP_PART;
     // the fold: totals, one value per thread, column and warp maxima
-    const size_t per_warp = (sizeof(T) == 8 ? 2 * sizeof(long long) : sizeof(float)) * (size_t)std::min(Gs, AP_HALF) * C;
+    const size_t per_warp = (sizeof(T) == 8 ? 2 * sizeof(long long) : sizeof(float)) * (size_t)std::min(Gs, AP_WHOLE) * C;
     const size_t smem = std::max(sizeof(double) * ((size_t)P + AP_THREADS + C + 8), per_warp * (AP_THREADS / 32));
     const long long per_block = (long long)(AP_THREADS / 32) * (32 / C) * AP_DEPTH;
     for (int e = 0; e < p.n_src; ++e) {
         const long long want = (p.src[e].Ge + per_block - 1) / per_block;
         const int nb = (int)std::max(1LL, std::min<long long>(want, sizeof(T) == 8 ? AP_FIX_BLOCKS : AP_PART_BLOCKS));
-        for (int h = 0; h < gr.halves; ++h) gr.first[e * gr.halves + h + 1] = gr.first[e * gr.halves + h] + nb;
+        for (int h = 0; h < gr.parts; ++h) gr.first[e * gr.parts + h + 1] = gr.first[e * gr.parts + h] + nb;
     }
+    if (Gs <= 4) return launch_ap_small_gt<T, 4>(p, gr, smem, s);
     if (Gs <= 8) return launch_ap_small_gt<T, 8>(p, gr, smem, s);
-    if (Gs <= 16) return launch_ap_small_gt<T, 16>(p, gr, smem, s);
-    if (Gs <= 24) return launch_ap_small_gt<T, 24>(p, gr, smem, s);
-    return launch_ap_small_gt<T, AP_HALF>(p, gr, smem, s);
+    if (Gs <= 12) return launch_ap_small_gt<T, 12>(p, gr, smem, s);
+    if (Gs <= AP_PART || Gs > AP_WHOLE) return launch_ap_small_gt<T, AP_PART>(p, gr, smem, s);
+    return launch_ap_small_gt<T, AP_WHOLE>(p, gr, smem, s);
 }
 template int launch_ap_small<float>(const ApSmall<float>&, cudaStream_t);
 template int launch_ap_small<double>(const ApSmall<double>&, cudaStream_t);
+
+int launch_ap_load(const double* inc, long long G, int C, int ld, double* tab, double* total,
+                   unsigned long long* amax, cudaStream_t s) {
+    if (G <= 0) return 0;
+    if (C > 32) return set_error("group tables: %d columns", C);
+    ap_load_kernel<<<ap_row_blocks(G, C), AP_THREADS, 0, s>>>(inc, G, C, ld, tab, total, amax);
+    FEGB_LAUNCH_CHECK("group tables of an increment");
+    return 0;
+}
 
 int launch_ap_reset(ApSlot* slots, const double* relax, const double* prev_change, int n_fe, ApCtl* ctl, double tol,
                     cudaStream_t s) {
@@ -782,6 +843,17 @@ int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long lo
     FEGB_LAUNCH_CHECK("count pairs (sorted)");
     return 0;
 }
+
+template <typename CT>
+int launch_pad_counts(const CT* src, long long Ge, int Gs, CT* dst, cudaStream_t s) {
+    if (Ge <= 0) return 0;
+    const int pitch = ap_count_pitch(Gs);
+    pad_counts_kernel<CT><<<grid_stride_blocks(Ge * pitch, 256), 256, 0, s>>>(src, Ge, Gs, pitch, dst);
+    FEGB_LAUNCH_CHECK("padded counts");
+    return 0;
+}
+template int launch_pad_counts<uint8_t>(const uint8_t*, long long, int, uint8_t*, cudaStream_t);
+template int launch_pad_counts<uint32_t>(const uint32_t*, long long, int, uint32_t*, cudaStream_t);
 
 int count_pairs_small(const int32_t* gid_e, int Ge, const int32_t* gid_s, long long n, int Gs, uint32_t* N,
                       cudaStream_t s) {

@@ -52,15 +52,16 @@ struct ApCtl {
 };
 
 // Count matrix of a small dimension s against a dimension e: entry (g, t) at
-// N[g * pitch + t], pitch = ap_count_pitch(Gs), so that rows start on 4 bytes.
-inline int ap_count_pitch(int Gs) { return (Gs + 3) & ~3; }
+// N[g * ap_count_pitch(Gs) + t], zero past Gs: rows of whole 16-count pieces, one
+// load each. (Rows of Gs bytes read in 4-byte pieces: three times the
+// instructions of the whole walk at 700k x 30 counts.)
+constexpr int AP_PART = 16;
+__host__ __device__ inline int ap_count_pitch(int Gs) { return (Gs + AP_PART - 1) / AP_PART * AP_PART; }
 template <typename T>
 struct ApDense {
     const void* N;     // uint8, or uint32 when wide
     int wide;
     int Gs;
-    int pitch;
-    int max_count;
     const T* tab;      // visit: the small dimension's table; small: the table of e
     const unsigned long long* amax;  // per column: bits of max |tab| so far
     int Ge;            // small: groups of e
@@ -77,6 +78,10 @@ struct ApTables {
     double* base;                // G x C: mu - coupling sum / n of the last visit
     unsigned long long* amax;    // C: bits of the running max |tab| per column
     ApSlot* slots;
+    // set: no projection; the table is an increment taken out of the residual,
+    // whose new means mu - coupling sum / n - tab go here, the largest of them
+    // into the slot's change
+    double* means;
 };
 
 template <typename T>
@@ -125,6 +130,11 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s);
 // doubles of ApSmall::partials for a dimension of Gs groups with n_src sources
 size_t ap_small_scratch(int Gs, int C, int n_src);
 
+// The FP64 tables of an increment: tab (row stride ld) = inc, total += inc (G x C,
+// compact) and the columns' maxima of |inc| into amax (zeroed by the caller).
+int launch_ap_load(const double* inc, long long G, int C, int ld, double* tab, double* total,
+                   unsigned long long* amax, cudaStream_t s);
+
 // Slots of all dimensions for a start from relaxation `relax` and last change
 // `prev_change` per dimension (device arrays of n_fe).
 int launch_ap_reset(ApSlot* slots, const double* relax, const double* prev_change, int n_fe, ApCtl* ctl, double tol,
@@ -142,6 +152,9 @@ int launch_ap_check(const ApSlot* slots, int n_fe, int half, ApCtl* ctl, cudaStr
 constexpr int AP_COUNT_LONGEST = 1 << 16;
 int count_pairs_sorted(const int32_t* off, int Ge, const int32_t* gid_s, long long n, int pitch, uint8_t* N8,
                        uint32_t* N32, unsigned* mx, cudaStream_t s);
+// dst (pitch ap_count_pitch(Gs), zero past Gs) = src (pitch Gs)
+template <typename CT>
+int launch_pad_counts(const CT* src, long long Ge, int Gs, CT* dst, cudaStream_t s);
 // Form for matrices of at most AP_COUNT_SMALL entries, any row order; N is
 // zeroed by the call.
 constexpr int AP_COUNT_SMALL = 12 * 1024;

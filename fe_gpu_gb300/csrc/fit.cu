@@ -1004,6 +1004,24 @@ int fp64_mean_pass(Problem& P, bool apply_alpha, double* mu_max) {
 
 // ----------------------- conjugate gradients (alpha space) -----------------------
 
+// The operator sweep of a many-group dimension d: positions in d's group
+// order, either the rows or (compressed) the distinct id tuples of the
+// many-group dimensions, each weighted by its row count.
+struct OpStream {
+    long long m = 0;
+    const int32_t* gseq = nullptr;
+    const int32_t* off = nullptr;  // G_d + 1 offsets over the positions
+    int n_src = 0;
+    const int32_t* src_gid[SWEEP_MAXP] = {};
+    int src_dim[SWEEP_MAXP] = {};
+    const float* weight = nullptr;
+    const int32_t* long_list = nullptr;
+    int n_long = 0;
+    const int32_t* multi_list = nullptr;
+    int n_multi = 0;
+    bool short_groups = false;  // every group short: the one-thread-per-group sweep applies
+};
+
 // Scratch of the CG solve in storage type T.
 template <typename T>
 struct CGBuffers {
@@ -1028,24 +1046,7 @@ struct CGBuffers {
     double* dense_sums = nullptr;
     T* extra = nullptr;  // Gt x C: the dense dimensions' share of each swept dimension's q
     bool any_dense = false;
-    // the operator sweep of each many-group dimension d: positions in d's group
-    // order, either the rows or (compressed) the distinct id tuples of the
-    // many-group dimensions, each weighted by its row count
-    struct Stream {
-        long long m = 0;
-        const int32_t* gseq = nullptr;
-        const int32_t* off = nullptr;  // G_d + 1 offsets over the positions
-        int n_src = 0;
-        const int32_t* src_gid[SWEEP_MAXP] = {};
-        int src_dim[SWEEP_MAXP] = {};
-        const float* weight = nullptr;
-        const int32_t* long_list = nullptr;
-        int n_long = 0;
-        const int32_t* multi_list = nullptr;
-        int n_multi = 0;
-        bool short_groups = false;  // every group short: the one-thread-per-group sweep applies
-    };
-    std::vector<Stream> stream;
+    std::vector<OpStream> stream;  // per many-group dimension
     bool compressed = false;
     // Schur-complement form: the primary (largest) dimension is eliminated, the
     // CG vectors span the other dimensions only (off[d]: their rows, Gv in all),
@@ -1100,7 +1101,7 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
     for (int d = 0; d < P.n_fe; ++d)
         if (P.dims[d].G > 0 && !B.dense[d] && d != P.primary) sw.push_back(d);
     if (P.primary >= 0 && P.dims[P.primary].G > 0 && !B.dense[P.primary]) sw.push_back(P.primary);
-    B.stream.assign(P.n_fe, typename CGBuffers<T>::Stream());
+    B.stream.assign(P.n_fe, OpStream());
     // rows, in each dimension's group order
     for (int d : sw) {
         Dim& D = P.dims[d];
@@ -1207,7 +1208,7 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
             const int d = sw[jd];
             const int G = P.dims[d].G;
             auto& st = B.stream[d];
-            st = typename CGBuffers<T>::Stream();
+            st = OpStream();
             st.m = m;
             int32_t* order = nullptr;  // tuple index at each position (null: identity)
             if (d == in_order) {
@@ -1994,65 +1995,6 @@ int cg_solve_host(Problem& P, CGBuffers<T>& B, double inner_tol, int max_it, int
     return cg_finish<T>(P, B);
 }
 
-// FP64 refinement loop around a CG inner solve in storage type T.
-template <typename T>
-int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update, int* outer) {
-    *iterations = 0;
-    *converged = 1;
-    *max_update = 0.0;
-    *outer = 0;
-    if (P.n_fe == 0 || P.n == 0) return 0;
-    CGBuffers<T> B;
-    FEGB_TRY(cg_alloc<T>(P, B));
-    CGGraph<T> G;
-    bool use_graph = false;
-    if (!P.profile && tuning(TUNE_CG_GRAPH)) {
-        FEGB_TRY(dalloc(*P.scr, &G.ctl, 1, "cg loop state"));
-        use_graph = cg_build_graph<T>(P, B, G) == 0;
-        if (!use_graph) {
-            cudaGetLastError();  // the host loop takes over
-            set_ok();
-        }
-    }
-    const int max_outer = 12;
-    double mu = 0.0, mu_prev = DBL_MAX;
-    int total = 0, hit = 0;
-    bool apply_alpha = false;
-    for (int round = 0; round < max_outer; ++round) {
-        FEGB_TRY(fp64_mean_pass(P, apply_alpha, &mu));
-        *outer = round + 1;
-        if (trace_enabled() && (mu < tol || round + 1 == max_outer))
-            std::fprintf(stderr, "fegb cg: outer %d max group mean %.3e (tolerance %.1e)\n", round + 1, mu, tol);
-        if (mu < tol) {
-            hit = 1;
-            break;
-        }
-        if (total >= max_iter) break;
-        if (round > 2 && mu > 0.5 * mu_prev) break;
-        mu_prev = mu;
-        const double inner_tol =
-            sizeof(T) == 4 ? std::max(0.5 * tol, 2e-6 * mu) : std::max(0.5 * tol, 1e-12 * mu);
-        int it = 0;
-        double zm = 0.0;
-        FEGB_TRY(cg_solve<T>(P, B, inner_tol, max_iter - total, &it, &zm, use_graph ? &G : nullptr));
-        if (trace_enabled())
-            std::fprintf(stderr, "fegb cg: outer %d max group mean %.3e inner tol %.3e: %d iterations, max |z| %.3e\n",
-                         round + 1, mu, inner_tol, it, zm);
-        total += it;
-        apply_alpha = true;
-    }
-    if (sizeof(T) == 4 && B.any_dense) {
-        // the tensor-core count-matrix passes record a wait that ran out of time
-        int umma_err = 0;
-        FEGB_TRY(dense_umma_error(&umma_err, true, P.s));
-        if (umma_err) return set_error("CG operator: a tensor-core count-matrix pass timed out waiting on its copies");
-    }
-    *iterations = total;
-    *converged = hit;
-    *max_update = mu;
-    return 0;
-}
-
 // ------------------- alternating projections on group tables -------------------
 
 // Host poll of a loop that runs ahead of it: AP_AHEAD iterations may be queued
@@ -2091,6 +2033,12 @@ struct ApPoll {
 // position's gather as long as the row itself.
 bool ap_on_groups(int C, int n_fe, long long n) { return C <= 32 && n_fe > 0 && n > 0; }
 
+// The group tables carry the means of the rows as they stand, to FP64 rounding:
+// 2^-53 of the largest mean, some 64 of them over the sums. While that is not far
+// below the tolerance (columns with a large level) the work stays on the rows,
+// whose level the first pass over them takes out.
+bool level_fits(double level, double tol) { return 64.0 * 0x1p-53 * level <= 1e-3 * tol; }
+
 // The group tables of an AP run in storage type T, with what they gather from.
 template <typename T>
 struct ApGroups {
@@ -2102,7 +2050,6 @@ struct ApGroups {
     double* partials = nullptr;
     unsigned long long* limbs = nullptr;
     unsigned* counter = nullptr;
-    std::vector<std::vector<int>> max_count;  // [small][e]
     // Coupling sums kept between visits. A dimension between the end ones is
     // visited from both sides, so at each visit only the side it comes from has
     // changed: version[e] counts the projections of e, seen[d][e] is the version
@@ -2113,40 +2060,85 @@ struct ApGroups {
     std::vector<double*> small_sums;              // [swept]: its sums over the small dimensions (G x C)
     std::vector<T*> swept_sums;                   // [swept]: its sums over the swept ones, chunked streams (G x C)
     ApPoll poll;
+    // refinement (FP64 tables): the increments taken out of the residual so far
+    bool refine = false;
+    double* total = nullptr;  // Gt x C
 
     int build(Problem& P) {
         Scratch& scr = *P.scr;
         const int C = P.C;
-        B.ld = cg_row_stride(C, (int)sizeof(T));
-        B.off.assign(P.goff.begin(), P.goff.end() - 1);
         B.dense.assign(P.n_fe, 0);
         B.N8.assign(P.n_fe, std::vector<uint8_t*>(P.n_fe, nullptr));
         B.N32.assign(P.n_fe, std::vector<uint32_t*>(P.n_fe, nullptr));
-        max_count.assign(P.n_fe, std::vector<int>(P.n_fe, 0));
-        pair_sums.assign(P.n_fe, std::vector<double*>(P.n_fe, nullptr));
-        seen.assign(P.n_fe, std::vector<long long>(P.n_fe, -1));
-        small_sums.assign(P.n_fe, nullptr);
-        swept_sums.assign(P.n_fe, nullptr);
         std::vector<int> Gd(P.n_fe);
         for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
         const std::vector<char> plan = cg_dense_plan(Gd, C, P.n);
         unsigned* mx = nullptr;
         FEGB_TRY(dalloc(scr, &mx, 1, "count max"));
-        size_t part = 1, limb = 2;
         for (int d = 0; d < P.n_fe; ++d) {
             if (!plan[d]) continue;
             B.dense[d] = 1;
             B.any_dense = true;
+            for (int e = 0; e < P.n_fe; ++e)
+                if (e != d && P.dims[e].G > 0) FEGB_TRY(count_matrix(P, B, d, e, ap_count_pitch(Gd[d]), mx));
+        }
+        FEGB_TRY(operator_streams(P, B));
+        FEGB_TRY(alloc(P));
+        return poll.open();
+    }
+
+    // The couplings of a CG operator (count rows without padding).
+    template <typename S>
+    int adopt(Problem& P, const CGBuffers<S>& O) {
+        FEGB_TRY(share(P, O));
+        for (int d = 0; d < P.n_fe; ++d)
             for (int e = 0; e < P.n_fe; ++e) {
-                if (e == d || P.dims[e].G <= 0) continue;
-                FEGB_TRY(count_matrix(P, B, d, e, ap_count_pitch(Gd[d]), mx));
-                max_count[d][e] = P.pair_max[d][e];
-                FEGB_TRY(dalloc(scr, &pair_sums[d][e], (size_t)Gd[d] * C, "small coupling sums"));
+                const long long Ge = P.dims[e].G;
+                const int Gs = P.dims[d].G, pitch = ap_count_pitch(Gs);
+                if (pitch == Gs) continue;
+                if (B.N8[d][e]) {
+                    FEGB_TRY(dalloc(*P.scr, &B.N8[d][e], (size_t)Ge * pitch, "padded counts"));
+                    FEGB_TRY(launch_pad_counts<uint8_t>(O.N8[d][e], Ge, Gs, B.N8[d][e], P.s));
+                }
+                if (B.N32[d][e]) {
+                    FEGB_TRY(dalloc(*P.scr, &B.N32[d][e], (size_t)Ge * pitch, "padded counts"));
+                    FEGB_TRY(launch_pad_counts<uint32_t>(O.N32[d][e], Ge, Gs, B.N32[d][e], P.s));
+                }
             }
+        return 0;
+    }
+    // The couplings as they are.
+    template <typename S>
+    int share(Problem& P, const CGBuffers<S>& O) {
+        B.dense = O.dense;
+        B.any_dense = O.any_dense;
+        B.N8 = O.N8;
+        B.N32 = O.N32;
+        B.stream = O.stream;
+        return alloc(P);
+    }
+
+    int alloc(Problem& P) {
+        Scratch& scr = *P.scr;
+        const int C = P.C;
+        B.ld = cg_row_stride(C, (int)sizeof(T));
+        B.off.assign(P.goff.begin(), P.goff.end() - 1);
+        pair_sums.assign(P.n_fe, std::vector<double*>(P.n_fe, nullptr));
+        seen.assign(P.n_fe, std::vector<long long>(P.n_fe, -1));
+        version.assign(P.n_fe, 0);
+        small_sums.assign(P.n_fe, nullptr);
+        swept_sums.assign(P.n_fe, nullptr);
+        std::vector<int> Gd(P.n_fe);
+        for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
+        size_t part = 1, limb = 2;
+        for (int d = 0; d < P.n_fe; ++d) {
+            if (!B.dense[d]) continue;
+            for (int e = 0; e < P.n_fe; ++e)
+                if (e != d && P.dims[e].G > 0)
+                    FEGB_TRY(dalloc(scr, &pair_sums[d][e], (size_t)Gd[d] * C, "small coupling sums"));
             part = std::max(part, ap_small_scratch(Gd[d], C, P.n_fe - 1));
             limb = std::max(limb, (size_t)2 * Gd[d] * C * std::max(1, P.n_fe - 1));
         }
-        FEGB_TRY(operator_streams(P, B));
         FEGB_TRY(operator_sums(P, B));
         // dimensions visited from both sides, with sources of both kinds
         for (int d = 0; d < P.n_fe; ++d) {
@@ -2166,7 +2158,7 @@ struct ApGroups {
         FEGB_TRY(dalloc(scr, &counter, 1, "small-dimension counter"));
         FEGB_CUDA(cudaMemsetAsync(limbs, 0, sizeof(unsigned long long) * limb, P.s), "small-dimension sums zero");
         FEGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), P.s), "small-dimension counter zero");
-        return poll.open();
+        return 0;
     }
 
     ApTables<T> tables(const Problem& P, int d) const {
@@ -2183,6 +2175,7 @@ struct ApGroups {
         t.base = base + P.goff[d] * P.C;
         t.amax = amax + (size_t)d * P.C;
         t.slots = slots + (size_t)d * AP_SLOTS;
+        t.means = refine ? D.mu : nullptr;
         return t;
     }
 
@@ -2192,9 +2185,7 @@ struct ApGroups {
         m.wide = B.N8[s][e] ? 0 : 1;
         m.N = B.N8[s][e] ? static_cast<const void*>(B.N8[s][e]) : static_cast<const void*>(B.N32[s][e]);
         m.Gs = P.dims[s].G;
-        m.pitch = ap_count_pitch(m.Gs);
         m.Ge = P.dims[e].G;
-        m.max_count = max_count[s][e];
         m.tab = B.p + P.goff[of] * B.ld;
         m.amax = amax + (size_t)of * P.C;
         return m;
@@ -2357,7 +2348,135 @@ struct ApGroups {
             FEGB_TRY(launch_to_f64<double>(reinterpret_cast<const double*>(B.p), B.ld, P.alpha_all, C, P.Gt, P.s));
         return 0;
     }
+
+    // ---- refinement: the means of the residual as increments leave it ----
+
+    // mu_all holds the means of the rows; nothing taken out yet.
+    int refine_start(Problem& P) {
+        refine = true;
+        if (!total) FEGB_TRY(dalloc(*P.scr, &total, (size_t)std::max(1LL, P.Gt) * P.C, "increments taken out"));
+        FEGB_CUDA(cudaMemsetAsync(total, 0, sizeof(double) * (size_t)std::max(1LL, P.Gt) * P.C, P.s),
+                  "increments zero");
+        FEGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ApCtl), P.s), "refinement state");
+        return 0;
+    }
+
+    // Takes the increments alpha_all out of the residual: mu_all becomes the
+    // means of what is left; their largest -> *mu_max.
+    int refine_step(Problem& P, double* mu_max) {
+        const int C = P.C;
+        FEGB_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (size_t)P.n_fe * C, P.s), "table maxima zero");
+        FEGB_CUDA(cudaMemsetAsync(slots, 0, sizeof(ApSlot) * (size_t)P.n_fe * AP_SLOTS, P.s), "refinement slots");
+        for (int d = 0; d < P.n_fe; ++d)
+            FEGB_TRY(launch_ap_load(P.alpha_all + P.goff[d] * C, P.dims[d].G, C, B.ld,
+                                    reinterpret_cast<double*>(B.p) + P.goff[d] * B.ld, total + P.goff[d] * C,
+                                    amax + (size_t)d * C, P.s));
+        for (auto& v : seen) std::fill(v.begin(), v.end(), -1);
+        const int proj = P.projections;
+        for (int d = 0; d < P.n_fe; ++d) FEGB_TRY(visit(P, d, 0, 1));
+        P.projections = proj;
+        std::vector<ApSlot> h((size_t)P.n_fe * AP_SLOTS);
+        FEGB_TRY(d2h_sync(h.data(), slots, sizeof(ApSlot) * h.size(), P.s, "refinement maxima copy"));
+        double m = 0.0;
+        for (int d = 0; d < P.n_fe; ++d) m = std::max(m, bits_to_double(h[(size_t)d * AP_SLOTS].change));
+        *mu_max = m;
+        return 0;
+    }
+
+    // All increments out of the rows.
+    int refine_finish(Problem& P) {
+        FEGB_CUDA(cudaMemcpyAsync(P.alpha_all, total, sizeof(double) * (size_t)std::max(1LL, P.Gt) * P.C,
+                                  cudaMemcpyDeviceToDevice, P.s),
+                  "increments copy");
+        refine = false;
+        return apply_alpha_rows(P);
+    }
 };
+
+// The FP64 refinement around an inner solve: group means of the residual, on the
+// rows at first and, once their level allows it (level_fits), on FP64 group
+// tables; there the rows are read once and written once, whatever the rounds.
+struct Refinement {
+    ApGroups<double> A;
+    bool possible = false, on_tables = false;
+
+    // means of the residual after the increments alpha_all of the previous round (if any)
+    int means(Problem& P, bool increments, double tol, double* mu) {
+        if (on_tables) return A.refine_step(P, mu);
+        FEGB_TRY(fp64_mean_pass(P, increments, mu));
+        if (possible && level_fits(*mu, tol)) {
+            on_tables = true;
+            FEGB_TRY(A.refine_start(P));
+        }
+        return 0;
+    }
+    int finish(Problem& P, bool increments) { return on_tables && increments ? A.refine_finish(P) : 0; }
+};
+
+// FP64 refinement loop around a CG inner solve in storage type T.
+template <typename T>
+int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update, int* outer) {
+    *iterations = 0;
+    *converged = 1;
+    *max_update = 0.0;
+    *outer = 0;
+    if (P.n_fe == 0 || P.n == 0) return 0;
+    CGBuffers<T> B;
+    FEGB_TRY(cg_alloc<T>(P, B));
+    CGGraph<T> G;
+    bool use_graph = false;
+    if (!P.profile && tuning(TUNE_CG_GRAPH)) {
+        FEGB_TRY(dalloc(*P.scr, &G.ctl, 1, "cg loop state"));
+        use_graph = cg_build_graph<T>(P, B, G) == 0;
+        if (!use_graph) {
+            cudaGetLastError();  // the host loop takes over
+            set_ok();
+        }
+    }
+    Refinement R;
+    if (ap_on_groups(P.C, P.n_fe, P.n)) {
+        FEGB_TRY(R.A.adopt(P, B));
+        R.possible = true;
+    }
+    const int max_outer = 12;
+    double mu = 0.0, mu_prev = DBL_MAX;
+    int total = 0, hit = 0;
+    bool apply_alpha = false;
+    for (int round = 0; round < max_outer; ++round) {
+        FEGB_TRY(R.means(P, apply_alpha, tol, &mu));
+        *outer = round + 1;
+        if (trace_enabled() && (mu < tol || round + 1 == max_outer))
+            std::fprintf(stderr, "fegb cg: outer %d max group mean %.3e (tolerance %.1e)\n", round + 1, mu, tol);
+        if (mu < tol) {
+            hit = 1;
+            break;
+        }
+        if (total >= max_iter) break;
+        if (round > 2 && mu > 0.5 * mu_prev) break;
+        mu_prev = mu;
+        const double inner_tol =
+            sizeof(T) == 4 ? std::max(0.5 * tol, 2e-6 * mu) : std::max(0.5 * tol, 1e-12 * mu);
+        int it = 0;
+        double zm = 0.0;
+        FEGB_TRY(cg_solve<T>(P, B, inner_tol, max_iter - total, &it, &zm, use_graph ? &G : nullptr));
+        if (trace_enabled())
+            std::fprintf(stderr, "fegb cg: outer %d max group mean %.3e inner tol %.3e: %d iterations, max |z| %.3e\n",
+                         round + 1, mu, inner_tol, it, zm);
+        total += it;
+        apply_alpha = true;
+    }
+    FEGB_TRY(R.finish(P, apply_alpha));
+    if (sizeof(T) == 4 && B.any_dense) {
+        // the tensor-core count-matrix passes record a wait that ran out of time
+        int umma_err = 0;
+        FEGB_TRY(dense_umma_error(&umma_err, true, P.s));
+        if (umma_err) return set_error("CG operator: a tensor-core count-matrix pass timed out waiting on its copies");
+    }
+    *iterations = total;
+    *converged = hit;
+    *max_update = mu;
+    return 0;
+}
 
 int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* converged, double* max_update) {
     *iterations = 0;
@@ -2369,12 +2488,7 @@ int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* con
     ProjectionOpts o;
     int hit = 0;
     double mu = 0.0;
-    // The group tables carry the means of the rows as they stand, to FP64
-    // rounding: 2^-53 of the largest mean, some 64 of them over the sums. While
-    // that is not far below the tolerance (columns with a large level) the
-    // projections run on the rows, whose level the first iteration takes out.
-    constexpr double AP_ROUND = 64.0 * 0x1p-53;
-    constexpr int AP_ROW_ITERATIONS = 3;
+    constexpr int AP_ROW_ITERATIONS = 3;  // on the rows before the tables are given up
     int iter = 0;
     if (ap_on_groups(P.C, P.n_fe, P.n)) {
         ApGroups<double> A;
@@ -2382,7 +2496,7 @@ int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* con
         while (iter < max_iter && iter <= AP_ROW_ITERATIONS) {
             double level = 0.0;
             FEGB_TRY(fp64_mean_pass(P, false, &level));
-            if (AP_ROUND * level <= 1e-3 * tol) {
+            if (level_fits(level, tol)) {
                 int it = 0;
                 FEGB_TRY(A.run(P, tol, max_iter - iter, &it, &mu));
                 FEGB_TRY(apply_alpha_rows(P));
@@ -2456,9 +2570,14 @@ int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* con
     int hit = 0;
     const bool groups = ap_on_groups(P.C, P.n_fe, P.n);
     ApGroups<float> A;
-    if (groups) FEGB_TRY(A.build(P));
+    Refinement R;
+    if (groups) {
+        FEGB_TRY(A.build(P));
+        FEGB_TRY(R.A.share(P, A.B));
+        R.possible = true;
+    }
     for (int round = 0; round < max_outer; ++round) {
-        FEGB_TRY(fp64_mean_pass(P, apply_alpha, &mu));
+        FEGB_TRY(R.means(P, apply_alpha, tol, &mu));
         *outer = round + 1;
         if (mu < tol) {
             hit = 1;
@@ -2478,6 +2597,7 @@ int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* con
         total_iter += it;
         apply_alpha = true;
     }
+    FEGB_TRY(R.finish(P, apply_alpha));
     *iterations = total_iter;
     *converged = hit;
     *max_update = mu;
@@ -2520,13 +2640,17 @@ void finalize_stats(fegb_result* r, long long n_obs) {
         r->f_stat = 0.0;
 }
 
-__global__ void tss_partials_kernel(const double* __restrict__ y, long long n, double mean, double* partials,
-                                    double* sums) {
+// element i of y at y[i * stride]
+__global__ void tss_partials_kernel(const double* __restrict__ y, long long stride, long long n, double mean,
+                                    double* partials, double* sums) {
     __shared__ double red[256 / 32];
     double a = 0.0;
     long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     const long long st = (long long)gridDim.x * 256;
-    for (; i < n; i += st) a += sums ? y[i] : (y[i] - mean) * (y[i] - mean);
+    for (; i < n; i += st) {
+        const double v = y[i * stride];
+        a += sums ? v : (v - mean) * (v - mean);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
@@ -2540,20 +2664,20 @@ __global__ void tss_partials_kernel(const double* __restrict__ y, long long n, d
 
 // Total sum of squares around the mean of the raw y (compute_tss,
 // fe_pipeline.f90:1935-1955), with a fixed reduction order.
-int compute_tss_dev(const double* y, long long n, double* out, cudaStream_t s, Scratch& scr) {
+int compute_tss_dev(const double* y, long long stride, long long n, double* out, cudaStream_t s, Scratch& scr) {
     *out = 0.0;
     if (n <= 0) return 0;
     int nb = (int)std::min<long long>((long long)num_sms() * 4, (n + 255) / 256);
     double* part = nullptr;
     FEGB_TRY(scr.alloc(&part, (size_t)nb, "tss partials"));
     std::vector<double> h(nb);
-    tss_partials_kernel<<<nb, 256, 0, s>>>(y, n, 0.0, nullptr, part);
+    tss_partials_kernel<<<nb, 256, 0, s>>>(y, stride, n, 0.0, nullptr, part);
     FEGB_LAUNCH_CHECK("tss sum");
     FEGB_TRY(d2h_sync(h.data(), part, sizeof(double) * nb, s, "tss sum copy"));
     double sum = 0.0;
     for (double v : h) sum += v;
     double mean = sum / (double)n;
-    tss_partials_kernel<<<nb, 256, 0, s>>>(y, n, mean, part, nullptr);
+    tss_partials_kernel<<<nb, 256, 0, s>>>(y, stride, n, mean, part, nullptr);
     FEGB_LAUNCH_CHECK("tss");
     FEGB_TRY(d2h_sync(h.data(), part, sizeof(double) * nb, s, "tss copy"));
     double t = 0.0;
@@ -3232,18 +3356,11 @@ int estimate_device_impl(const fegb_config* cfg_in, long long n, int k, int l, i
     // TSS of the raw y over the rows used
     double tss = 0.0;
     {
-        double* ycol = nullptr;
-        FEGB_TRY(scr.alloc(&ycol, (size_t)std::max(1LL, P.n), "y column"));
-        // copy the strided column 0 of the data block into a contiguous vector
-        // (or the raw y when the block was demeaned beforehand)
-        if (y_raw && P.n > 0) {
-            FEGB_CUDA(cudaMemcpyAsync(ycol, y_raw, sizeof(double) * P.n, cudaMemcpyDeviceToDevice, s), "raw y copy");
-        } else if (P.n > 0) {
-            FEGB_CUDA(cudaMemcpy2DAsync(ycol, sizeof(double), P.X, sizeof(double) * P.C, sizeof(double), (size_t)P.n,
-                                        cudaMemcpyDeviceToDevice, s),
-                      "y column copy");
-        }
-        FEGB_TRY(compute_tss_dev(ycol, P.n, &tss, s, scr));
+        // all rows used: the caller's y (a sum over them needs no order), or the
+        // raw y when the block was demeaned beforehand; else column 0 of the data block
+        const double* yv = y_raw ? y_raw : (P.n == n ? y : P.X);
+        const long long stride = yv == P.X ? P.C : 1;
+        FEGB_TRY(compute_tss_dev(yv, stride, P.n, &tss, s, scr));
     }
     trace_phase(s, t0, "problem and tss");
     FEGB_CUDA(cudaStreamSynchronize(s), "prep sync");
@@ -3309,7 +3426,7 @@ int reconstruct_fe_impl(const fegb_config& cfg, long long n, int k, int n_fe, co
         int nb = (int)std::min<long long>((long long)num_sms() * 4, (n + 255) / 256);
         double* part = nullptr;
         FEGB_TRY(scr.alloc(&part, (size_t)nb, "fe mean partials"));
-        tss_partials_kernel<<<nb, 256, 0, s>>>(r, n, 0.0, nullptr, part);
+        tss_partials_kernel<<<nb, 256, 0, s>>>(r, 1, n, 0.0, nullptr, part);
         FEGB_LAUNCH_CHECK("fe mean");
         std::vector<double> h(nb);
         FEGB_TRY(d2h_sync(h.data(), part, sizeof(double) * nb, s, "fe mean copy"));
