@@ -83,6 +83,7 @@ struct Dim {
     float* pend32 = nullptr;
     double* alpha = nullptr;
     double* mu = nullptr;
+    bool order_deferred = false;  // perm, gseq, off not built (the runs serve instead): order_rows builds them
 };
 
 struct Problem {
@@ -133,6 +134,20 @@ struct Problem {
     // tuple at each position, null = identity), their group ids and offsets
     std::vector<const int32_t*> tuple_dim_order, tuple_dim_gseq, tuple_dim_off;
     double* inc_tab = nullptr;                 // m x C
+    // The tuples are runs: maximal stretches of consecutive storage rows with equal
+    // ids in the primary and the one other swept dimension, found without sorting
+    // the rows. A pair of groups that a primary group returns to gives more than one
+    // run; the distinct pairs are the segments pair_off of the runs in the other
+    // dimension's order (pair_gseq: pair of each position), pair_m in all.
+    bool runs = false;
+    int run_dim = -1;                        // the other swept dimension
+    const int32_t* run_sorted = nullptr;     // its group at each position of its order
+    const int32_t* run_order = nullptr;      // run at each position
+    const int32_t* run_primary = nullptr;    // the primary group at each position
+    const float* run_weight = nullptr;       // rows of each run
+    const int32_t* pair_gseq = nullptr;
+    const int32_t* pair_off = nullptr;
+    int pair_m = 0;
     // long-group lists of persistent offset arrays (the tuple streams), found
     // once: offsets array, group count -> list, list length
     struct LongCache {
@@ -295,15 +310,15 @@ __global__ void gather_i32_kernel(const int32_t* __restrict__ src, const int32_t
 }
 
 // Distinct id tuples of the swept dimensions: tuple k covers the key-sorted
-// rows [off[k], off[k + 1]); its weight is that row count and its ids are
-// those of its first row.
+// rows [off[k], off[k + 1]) (perm null: of the storage order); its weight is that
+// row count and its ids are those of its first row.
 __global__ void tuple_build_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ perm, long long m,
                                    int nd, const int32_t* const* __restrict__ gids, int32_t* const* __restrict__ tgid,
                                    float* __restrict__ weight) {
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long st = (long long)gridDim.x * blockDim.x;
     for (; k < m; k += st) {
-        const int r = perm[off[k]];
+        const int r = perm ? perm[off[k]] : off[k];
         weight[k] = (float)(off[k + 1] - off[k]);
         for (int j = 0; j < nd; ++j) tgid[j][k] = gids[j][r];
     }
@@ -427,6 +442,164 @@ std::vector<char> cg_dense_plan(const std::vector<int>& G, int C, long long n) {
     return dense;
 }
 
+// flags[i] = 1 where the pair (ga, gb) changes along an ordered list of rows
+__global__ void pair_flags_kernel(const int32_t* __restrict__ ga, const int32_t* __restrict__ gb, long long n,
+                                  uint32_t* __restrict__ flags) {
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (; i < n; i += st) flags[i] = (i == 0 || ga[i] != ga[i - 1] || gb[i] != gb[i - 1]) ? 1u : 0u;
+}
+
+// rank[i] = the run of position i; off[run] = its first position
+__global__ void run_ranks_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ excl, long long n,
+                                 int32_t* __restrict__ off, int32_t* __restrict__ rank) {
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (; i < n; i += st) {
+        const int32_t r = (int32_t)(excl[i] + flags[i]) - 1;
+        rank[i] = r;
+        if (flags[i]) off[r] = (int32_t)i;
+    }
+}
+
+// ids and length of each run of storage rows [off[k], off[k + 1])
+__global__ void run_build_kernel(const int32_t* __restrict__ off, long long m, const int32_t* __restrict__ gw,
+                                 const int32_t* __restrict__ ge, int32_t* __restrict__ tw, int32_t* __restrict__ te,
+                                 float* __restrict__ len) {
+    long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (; k < m; k += st) {
+        const int r = off[k];
+        len[k] = (float)(off[k + 1] - r);
+        tw[k] = gw[r];
+        te[k] = ge[r];
+    }
+}
+
+// counts[g] += rows of each run of group g
+__global__ void run_counts_kernel(const int32_t* __restrict__ gid, const int32_t* __restrict__ off, long long m,
+                                  int32_t* __restrict__ counts) {
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (; i < m; i += st) atomicAdd(counts + gid[i], off[i + 1] - off[i]);  // integer: order-free
+}
+
+// Runs of the primary and dimension e over the storage order (Problem::runs),
+// taken as the tuples of the operator when they are at most three quarters of the
+// rows and at most a quarter more than the distinct pairs (rows of a primary
+// group in no order of e would give many runs for one pair). What remains is
+// sorted run by run: the rows themselves are neither sorted by e nor gathered in
+// that order (150M rows, 12M runs: 10 digit passes of 4 ms over the rows become
+// three of 0.4 ms over the runs; fit 165 -> RUNS_MS ms).
+int build_runs(Problem& P, int e) {
+    Scratch& scr = *P.scr;
+    cudaStream_t s = P.s;
+    const long long n = P.n;
+    const int32_t *gw = P.dims[P.primary].gid, *ge = P.dims[e].gid;
+    Scratch tmp(s);
+    uint32_t *flags = nullptr, *excl = nullptr, *total = nullptr;
+    FEGB_TRY(tmp.alloc(&flags, (size_t)n, "run flags"));
+    FEGB_TRY(tmp.alloc(&excl, (size_t)n, "run scan"));
+    FEGB_TRY(tmp.alloc(&total, 1, "run count"));
+    pair_flags_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(gw, ge, n, flags);
+    FEGB_LAUNCH_CHECK("run flags");
+    FEGB_TRY(scan_exclusive_u32(flags, excl, n, total, s, tmp));
+    uint32_t hm = 0;
+    FEGB_TRY(d2h_sync(&hm, total, sizeof(hm), s, "run count copy"));
+    const int m = (int)hm;
+    if ((double)m > 0.75 * (double)n) return 0;
+    int32_t *off = nullptr, *row_run = nullptr, *tw = nullptr, *te = nullptr, *order = nullptr, *wj = nullptr;
+    float* w = nullptr;
+    uint32_t* sorted = nullptr;
+    FEGB_TRY(dalloc(scr, &off, (size_t)m + 1, "run offsets"));
+    FEGB_TRY(dalloc(scr, &row_run, (size_t)n, "run of each row"));
+    run_ranks_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(flags, excl, n, off, row_run);
+    FEGB_LAUNCH_CHECK("runs");
+    const int32_t n32 = (int32_t)n;
+    FEGB_TRY(h2d_sync(off + m, &n32, sizeof(n32), s, "run end"));
+    FEGB_TRY(dalloc(scr, &tw, (size_t)m, "run ids"));
+    FEGB_TRY(dalloc(scr, &te, (size_t)m, "run ids"));
+    FEGB_TRY(dalloc(scr, &w, (size_t)m, "run lengths"));
+    run_build_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(off, m, gw, ge, tw, te, w);
+    FEGB_LAUNCH_CHECK("run ids");
+    FEGB_TRY(dalloc(scr, &sorted, (size_t)m, "run order ids"));
+    FEGB_TRY(dalloc(scr, &order, (size_t)m, "run order"));
+    FEGB_TRY(radix_sort_u32(reinterpret_cast<const uint32_t*>(te), nullptr, sorted, order, m,
+                            bits_for((unsigned long long)P.dims[e].G), s, tmp));
+    FEGB_TRY(dalloc(scr, &wj, (size_t)m, "run primary ids"));
+    gather_i32_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(tw, order, m, wj);
+    FEGB_LAUNCH_CHECK("run id gather");
+    // the distinct pairs: the runs in (group of e, primary group) order
+    int32_t *pgs = nullptr, *pof = nullptr;
+    FEGB_TRY(dalloc(scr, &pgs, (size_t)m, "pair ranks"));
+    FEGB_TRY(dalloc(scr, &pof, (size_t)m + 1, "pair offsets"));
+    pair_flags_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(reinterpret_cast<const int32_t*>(sorted), wj, m, flags);
+    FEGB_LAUNCH_CHECK("pair flags");
+    FEGB_TRY(scan_exclusive_u32(flags, excl, m, total, s, tmp));
+    run_ranks_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(flags, excl, m, pof, pgs);
+    FEGB_LAUNCH_CHECK("pair ranks");
+    FEGB_TRY(d2h_sync(&hm, total, sizeof(hm), s, "pair count copy"));
+    const int mp = (int)hm;
+    if ((double)m > 1.25 * (double)mp) return 0;
+    const int32_t m32 = m;
+    FEGB_TRY(h2d_sync(pof + mp, &m32, sizeof(m32), s, "pair end"));
+    P.runs = true;
+    P.run_dim = e;
+    P.run_sorted = reinterpret_cast<const int32_t*>(sorted);
+    P.run_order = order;
+    P.run_primary = wj;
+    P.run_weight = w;
+    P.pair_gseq = pgs;
+    P.pair_off = pof;
+    P.pair_m = mp;
+    P.row_tuple = row_run;
+    P.tuple_perm = nullptr;
+    P.tuple_off = off;
+    P.tuple_gseq = row_run;
+    P.tuple_m = m;
+    P.tuple_n = n;
+    P.tuple_sw = {e, P.primary};
+    P.tuple_ids = {te, tw};
+    P.tuple_dims = {std::min(e, P.primary), std::max(e, P.primary)};
+    P.tuple_gid = {P.dims[P.tuple_dims[0]].gid, P.dims[P.tuple_dims[1]].gid};
+    return 0;
+}
+
+// Group order of the rows of dimension d: perm, gseq, offsets, long groups.
+int order_rows(Problem& P, int d) {
+    Dim& D = P.dims[d];
+    Scratch& scr = *P.scr;
+    uint32_t* sorted = nullptr;
+    FEGB_TRY(dalloc(scr, &sorted, (size_t)P.n, "gather gseq"));
+    FEGB_TRY(dalloc(scr, &D.perm, (size_t)P.n, "gather perm"));
+    FEGB_TRY(radix_sort_u32(reinterpret_cast<const uint32_t*>(D.gid), nullptr, sorted, D.perm, P.n,
+                            bits_for((unsigned long long)D.G), P.s, scr));
+    D.gseq = reinterpret_cast<int32_t*>(sorted);
+    return 0;
+}
+
+// What order_deferred left out, for the row sweeps.
+int order_deferred_rows(Problem& P) {
+    for (int d = 0; d < P.n_fe; ++d) {
+        Dim& D = P.dims[d];
+        if (!D.order_deferred) continue;
+        FEGB_TRY(order_rows(P, d));
+        FEGB_TRY(dalloc(*P.scr, &D.off, (size_t)D.G + 1, "offsets"));
+        FEGB_TRY(segment_offsets(reinterpret_cast<const uint32_t*>(D.gseq), P.n, D.G, D.off, P.s));
+        FEGB_TRY(dalloc(*P.scr, &D.long_list, (size_t)D.G, "long groups"));
+        FEGB_TRY(find_long_groups(D.off, D.G, CHUNK_R, D.long_list, &D.n_long, P.s));
+        for (int e = 0; e < P.n_fe; ++e) {
+            if (e == d) continue;
+            FEGB_TRY(dalloc(*P.scr, &D.gid_at_perm[e], (size_t)P.n, "gid at perm"));
+            gather_i32_kernel<<<grid_stride_blocks(P.n, 256), 256, 0, P.s>>>(P.dims[e].gid, D.perm, P.n,
+                                                                            D.gid_at_perm[e]);
+            FEGB_LAUNCH_CHECK("gid at perm");
+        }
+        D.order_deferred = false;
+    }
+    return 0;
+}
+
 int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const double* y, const double* W, const double* Z,
                   const int32_t* const* ids, const int* G_in, bool drop_singletons, bool mixed, long long* n_single,
                   bool sorted_all = false) {
@@ -491,6 +664,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     for (int d = 0; d < n_fe; ++d) P.dims[d].G = G[d];
     // storage order: stable sort by the primary id
     int32_t* row_of = nullptr;
+    bool in_primary_order = false;
     if (P.primary >= 0 && n > 0) {
         uint32_t *keys = nullptr, *sorted = nullptr;
         int32_t* vals = nullptr;
@@ -508,6 +682,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
         FEGB_LAUNCH_CHECK("primary order check");
         int h_unsorted = 1;
         FEGB_TRY(d2h_sync(&h_unsorted, unsorted, sizeof(int), s, "order flag copy"));
+        in_primary_order = !h_unsorted;
         if (!h_unsorted) {
             row_of = rows ? vals : nullptr;
             P.dims[P.primary].gid = reinterpret_cast<int32_t*>(keys);
@@ -552,6 +727,21 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
                 FEGB_LAUNCH_CHECK("gid gather");
             }
         }
+    }
+    // rows that come in the primary's order, and one other swept dimension: its
+    // runs may serve instead of its row order
+    if (sorted_all && in_primary_order && n >= 4096) {
+        const std::vector<char> dense = cg_dense_plan(G, C, n);
+        int other = -1, swept = 0;
+        for (int d = 0; d < n_fe; ++d)
+            if (!dense[d] && G[d] > 0) {
+                ++swept;
+                if (d != P.primary) other = d;
+            }
+        if (swept == 2 && other >= 0 && !dense[P.primary]) FEGB_TRY(build_runs(P, other));
+    }
+    for (int d = 0; d < n_fe; ++d) {
+        Dim& D = P.dims[d];
         if (d == P.primary) {
             D.mode = MODE_CONTIG;
             D.gseq = D.gid;
@@ -560,16 +750,14 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
         } else {
             D.mode = MODE_GATHER;
         }
-        const bool need_sorted = D.mode == MODE_GATHER || cg_sorted[d];
-        if (need_sorted && n > 0) {
-            uint32_t* sorted = nullptr;
-            FEGB_TRY(dalloc(scr, &sorted, (size_t)n, "gather gseq"));
-            FEGB_TRY(dalloc(scr, &D.perm, (size_t)n, "gather perm"));
-            FEGB_TRY(radix_sort_u32(reinterpret_cast<const uint32_t*>(D.gid), nullptr, sorted, D.perm, n,
-                                    bits_for((unsigned long long)D.G), s, scr));
-            D.gseq = reinterpret_cast<int32_t*>(sorted);
-        }
-        if (D.mode != MODE_SMALLG || need_sorted) {
+        D.order_deferred = P.runs && d == P.run_dim;
+        const bool need_sorted = (D.mode == MODE_GATHER || cg_sorted[d]) && !D.order_deferred;
+        if (need_sorted && n > 0) FEGB_TRY(order_rows(P, d));
+        if (D.order_deferred) {
+            run_counts_kernel<<<grid_stride_blocks(P.tuple_m, 256), 256, 0, s>>>(P.tuple_ids[0], P.tuple_off,
+                                                                                P.tuple_m, D.counts);
+            FEGB_LAUNCH_CHECK("run counts");
+        } else if (D.mode != MODE_SMALLG || need_sorted) {
             FEGB_TRY(dalloc(scr, &D.off, (size_t)D.G + 1, "offsets"));
             if (n > 0) {
                 FEGB_TRY(segment_offsets(reinterpret_cast<const uint32_t*>(D.gseq), n, D.G, D.off, s));
@@ -590,7 +778,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
             }
         }
         if (D.mode == MODE_SMALLG) {
-            if (!need_sorted) {  // sorted dimensions already have counts from their offsets
+            if (!need_sorted && !D.order_deferred) {  // sorted dimensions already have counts from their offsets
                 FEGB_CUDA(cudaMemsetAsync(D.counts, 0, sizeof(int32_t) * (size_t)D.G, s), "counts zero");
                 if (n > 0 && D.G > 0) {
                     count_ids_kernel<<<std::min<unsigned>(grid_stride_blocks(n, 256), 4u * (unsigned)num_sms()), 256,
@@ -611,7 +799,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     for (int d = 0; d < n_fe; ++d) {
         Dim& D = P.dims[d];
         D.gid_at_perm.assign(n_fe, nullptr);
-        if (!(D.mode == MODE_GATHER || cg_sorted[d]) || n == 0) continue;
+        if (!(D.mode == MODE_GATHER || cg_sorted[d]) || n == 0 || D.order_deferred) continue;
         for (int e = 0; e < n_fe; ++e) {
             if (e == d) continue;
             FEGB_TRY(dalloc(scr, &D.gid_at_perm[e], (size_t)n, "gid at perm"));
@@ -1068,27 +1256,51 @@ __global__ void scatter_tuple_kernel(const int32_t* __restrict__ perm, const int
     for (; i < n; i += st) row_tuple[perm[i]] = rank[i];
 }
 
-// flags[i] = 1 where the pair (ga, gb) changes along an ordered list of rows
-__global__ void pair_flags_kernel(const int32_t* __restrict__ ga, const int32_t* __restrict__ gb, long long n,
-                                  uint32_t* __restrict__ flags) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long st = (long long)gridDim.x * blockDim.x;
-    for (; i < n; i += st) flags[i] = (i == 0 || ga[i] != ga[i - 1] || gb[i] != gb[i - 1]) ? 1u : 0u;
+// Long and multi-chunk groups of a stream over st.m positions of dimension d.
+int stream_groups(Problem& P, int d, OpStream& st) {
+    const int G = P.dims[d].G;
+    int32_t *off = nullptr, *ll = nullptr, *ml = nullptr;
+    FEGB_TRY(dalloc(*P.scr, &off, (size_t)G + 1, "tuple group offsets"));
+    FEGB_TRY(segment_offsets(reinterpret_cast<const uint32_t*>(st.gseq), st.m, G, off, P.s));
+    FEGB_TRY(dalloc(*P.scr, &ll, (size_t)G, "tuple long groups"));
+    FEGB_TRY(find_long_groups(off, G, CG_CHUNK, ll, &st.n_long, P.s));
+    FEGB_TRY(dalloc(*P.scr, &ml, (size_t)G, "tuple multi-chunk groups"));
+    FEGB_TRY(find_multi_groups(off, G, CG_CHUNK, ml, &st.n_multi, P.s));
+    st.off = off;
+    st.long_list = ll;
+    st.multi_list = ml;
+    return 0;
 }
 
-// rank[i] = the run of position i; off[run] = its first position
-__global__ void run_ranks_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ excl, long long n,
-                                 int32_t* __restrict__ off, int32_t* __restrict__ rank) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long st = (long long)gridDim.x * blockDim.x;
-    for (; i < n; i += st) {
-        const int32_t r = (int32_t)(excl[i] + flags[i]) - 1;
-        rank[i] = r;
-        if (flags[i]) off[r] = (int32_t)i;
+// The two swept dimensions' streams over the runs (Problem::runs).
+int run_streams(Problem& P, std::vector<OpStream>& streams) {
+    const int pd = P.primary, e = P.run_dim;
+    const long long m = P.tuple_m;
+    FEGB_TRY(dalloc(*P.scr, &P.inc_tab, (size_t)m * P.C, "combined increments"));
+    P.tuple_dim_order.assign(P.n_fe, nullptr);
+    P.tuple_dim_gseq.assign(P.n_fe, nullptr);
+    P.tuple_dim_off.assign(P.n_fe, nullptr);
+    float* we = nullptr;
+    FEGB_TRY(dalloc(*P.scr, &we, (size_t)m, "run lengths (sorted)"));
+    gather_f32_kernel<<<grid_stride_blocks(m, 256), 256, 0, P.s>>>(P.run_weight, P.run_order, m, we);
+    FEGB_LAUNCH_CHECK("run length gather");
+    for (int d : {pd, e}) {
+        OpStream& st = streams[d];
+        st.m = m;
+        st.gseq = d == pd ? P.tuple_ids[1] : P.run_sorted;
+        st.n_src = 1;
+        st.src_gid[0] = d == pd ? P.tuple_ids[0] : P.run_primary;
+        st.src_dim[0] = d == pd ? e : pd;
+        st.weight = d == pd ? P.run_weight : we;
+        FEGB_TRY(stream_groups(P, d, st));
+        P.tuple_dim_order[d] = d == pd ? nullptr : P.run_order;
+        P.tuple_dim_gseq[d] = st.gseq;
+        P.tuple_dim_off[d] = st.off;
     }
+    return 0;
 }
 
-// Position streams of the CG operator sweeps (see CGBuffers::Stream). The
+// Position streams of the CG operator sweeps (see OpStream). The
 // rows are compressed into distinct id tuples of the many-group dimensions
 // when that removes at least a quarter of the positions: the operator carries
 // no row data, so rows with equal ids contribute equally (weight x one row).
@@ -1102,6 +1314,11 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
         if (P.dims[d].G > 0 && !B.dense[d] && d != P.primary) sw.push_back(d);
     if (P.primary >= 0 && P.dims[P.primary].G > 0 && !B.dense[P.primary]) sw.push_back(P.primary);
     B.stream.assign(P.n_fe, OpStream());
+    if (P.runs) {
+        FEGB_TRY(run_streams(P, B.stream));
+        B.compressed = true;
+        return 0;
+    }
     // rows, in each dimension's group order
     for (int d : sw) {
         Dim& D = P.dims[d];
@@ -1240,20 +1457,11 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
                 }
                 st.src_dim[st.n_src++] = sw[je];
             }
-            int32_t *off = nullptr, *ll = nullptr, *ml = nullptr;
-            FEGB_TRY(dalloc(scr, &off, (size_t)G + 1, "tuple group offsets"));
-            FEGB_TRY(segment_offsets(reinterpret_cast<const uint32_t*>(st.gseq), m, G, off, s));
-            FEGB_TRY(dalloc(scr, &ll, (size_t)G, "tuple long groups"));
-            FEGB_TRY(find_long_groups(off, G, CG_CHUNK, ll, &st.n_long, s));
-            FEGB_TRY(dalloc(scr, &ml, (size_t)G, "tuple multi-chunk groups"));
-            FEGB_TRY(find_multi_groups(off, G, CG_CHUNK, ml, &st.n_multi, s));
-            st.off = off;
-            st.long_list = ll;
-            st.multi_list = ml;
+            FEGB_TRY(stream_groups(P, d, st));
             // the SEs sum the scores of this dimension's clusters from the tuples' sums
             P.tuple_dim_order[d] = order;
             P.tuple_dim_gseq[d] = st.gseq;
-            P.tuple_dim_off[d] = off;
+            P.tuple_dim_off[d] = st.off;
         }
         FEGB_CUDA(cudaStreamSynchronize(s), "tuple streams sync");
     }
@@ -1266,8 +1474,9 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
 // primary group) pairs, instead of the group counts n_g (which overstate S_gg
 // by up to n_g / S_gg: the inner solve's max |z| stop would then end it early).
 // The pairs come from the dimension's compressed stream when its positions are
-// exactly those pairs (one other swept dimension), from a sort of the rows by
-// pair otherwise, and from the count matrices for the small dimensions.
+// those pairs (one other swept dimension; a pair of several runs then counts a
+// little more than it should, which a preconditioner may), from a sort of the rows
+// by pair otherwise, and from the count matrices for the small dimensions.
 template <typename T>
 int cg_schur_precond(Problem& P, CGBuffers<T>& B) {
     const int pd = B.prim;
@@ -2505,6 +2714,7 @@ int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* con
                 *max_update = mu;
                 return 0;
             }
+            FEGB_TRY(order_deferred_rows(P));
             FEGB_TRY(ap_iteration<double>(P, P.X, pl, o, &mu));
             ++iter;
             FEGB_TRY(apply_all_pending<double>(P, P.X, pl));
@@ -3123,11 +3333,8 @@ int estimate_on_problem(Problem& P, const fegb_config& cfg, const int* G_all, lo
             } else if (tuple_single) {
                 n_cl = P.dims[sd[0]].G;
             } else if (tuples) {
-                // the clusters are the CG operator's id tuples: its row sort serves
-                perm = P.tuple_perm;
-                gseq = P.tuple_gseq;
-                off = P.tuple_off;
-                n_cl = P.tuple_m;
+                // the clusters are the CG operator's id tuples (with runs, the distinct pairs among them)
+                n_cl = P.runs ? P.pair_m : P.tuple_m;
             } else if (smallg_single) {
                 n_cl = P.dims[sd[0]].G;  // sums from per-block tables in storage order, no sort
             } else if (m == 1 && P.dims[sd[0]].mode != MODE_SMALLG) {
@@ -3208,11 +3415,15 @@ int estimate_on_problem(Problem& P, const fegb_config& cfg, const int* G_all, lo
             } else {
                 double* Sc = nullptr;
                 if (tuples || tuple_single) FEGB_TRY(tuple_sums());
-                if (tuples)
+                const bool merge = tuples && n_cl != P.tuple_m;
+                if (tuples && !merge)
                     Sc = tuple_scores;  // the clusters are the tuples
                 else
                     FEGB_TRY(sub.alloc(&Sc, (size_t)n_cl * ns, "cluster scores"));
-                if (tuples) {
+                if (merge) {
+                    FEGB_TRY(cluster_score_sums(P, tuple_scores, ns, P.run_order, P.pair_gseq, P.pair_off, n_cl, Sc, sub,
+                                                P.tuple_m, -1, true));
+                } else if (tuples) {
                 } else if (tuple_single) {
                     // n rows -> m tuple sums -> G cluster sums: the second pass reads m positions
                     FEGB_TRY(cluster_score_sums(P, tuple_scores, ns, P.tuple_dim_order[sd[0]],
