@@ -490,7 +490,7 @@ __global__ void run_counts_kernel(const int32_t* __restrict__ gid, const int32_t
 // group in no order of e would give many runs for one pair). What remains is
 // sorted run by run: the rows themselves are neither sorted by e nor gathered in
 // that order (150M rows, 12M runs: 10 digit passes of 4 ms over the rows become
-// three of 0.4 ms over the runs; fit 165 -> RUNS_MS ms).
+// three of 0.4 ms over the runs; preparation 27.6 -> 11.9 ms).
 int build_runs(Problem& P, int e) {
     Scratch& scr = *P.scr;
     cudaStream_t s = P.s;
