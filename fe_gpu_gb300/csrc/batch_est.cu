@@ -333,8 +333,12 @@ __global__ void __launch_bounds__(DN_THREADS)
     double* Pi = Pi_out + (long long)blockIdx.x * Kb * Kb;
     double* Qiz = Qzx + Kb * Kb;
     double* Qinv = Qinv_out + (long long)blockIdx.x * Kb * Kb;
-    double* work = Qiz + Kb * Kb;  // 2 Kb^2
-    double* b = work + 2 * Kb * Kb;
+    // work matrices of the factorisations: shared memory where they fit (launched
+    // with dn_work_bytes(Kb)), else 2 Kb^2 of the scratch
+    extern __shared__ __align__(16) unsigned char dn_smem[];
+    const bool fits = dn_fits(Kb);
+    double* work = fits ? reinterpret_cast<double*>(dn_smem) : Qiz + Kb * Kb;
+    double* b = Qiz + 3 * Kb * Kb;
     double* zy = b + Kb;
     double* rhs = zy + Kb;
     double* bsel = rhs + Kb;
@@ -373,7 +377,7 @@ __global__ void __launch_bounds__(DN_THREADS)
         for (int e = t; e < na * k; e += DN_THREADS) Qzx[e] = gram_at(G, S.za[e % na], 1 + e / na);
         for (int j = t; j < na; j += DN_THREADS) zy[j] = gram_at(G, S.za[j], 0);
         __syncthreads();
-        chol_solve_inv_block(na, Qzz, na, nullptr, zy, rhs, Qiz, &s_info, work);
+        chol_solve_inv_block(na, Qzz, na, nullptr, zy, rhs, Qiz, &s_info, work, fits ? dn_stride(na) : na);
         __syncthreads();
         if (s_info != 0) {
             if (t == 0) S.info = s_info;
@@ -420,7 +424,7 @@ __global__ void __launch_bounds__(DN_THREADS)
     __syncthreads();
     const int kk = s_kk;
     if (kk == 0) return;
-    chol_solve_inv_block(kk, Q, k, s_kept, b, bsel, Qinv, &s_info, work);
+    chol_solve_inv_block(kk, Q, k, s_kept, b, bsel, Qinv, &s_info, work, fits ? dn_stride(kk) : kk);
     __syncthreads();
     if (s_info != 0) {
         if (t == 0) S.info = s_info;
@@ -684,10 +688,13 @@ __global__ void __launch_bounds__(DN_THREADS)
     if (S.info != 0 || S.kk == 0) return;
     const int kk = S.kk;
     double* sel = scratch + (long long)s * be_scratch_per_spec(Kb);
-    double* work = sel + Kb;
+    extern __shared__ __align__(16) unsigned char dn_smem[];
+    const bool fits = dn_fits(Kb);
+    double* work = fits ? reinterpret_cast<double*>(dn_smem) : sel + Kb;
     if (scalar[s] > 0.0) {
         __shared__ int s_psd;
-        finalize_cov_block(kk, acc_all + (long long)s * Kb * Kb, scalar[s], 1, sel, &s_psd, work);
+        finalize_cov_block(kk, acc_all + (long long)s * Kb * Kb, scalar[s], 1, sel, &s_psd, work,
+                           fits ? dn_stride(kk) : kk);
         __syncthreads();
         for (int q = t; q < kk; q += DN_THREADS) se[S.kept[q]] = sel[q];
         if (t == 0) psd[s] = s_psd;
@@ -916,7 +923,14 @@ int estimate_class_batched(const fegb_config& cfg, const std::vector<BeSpecHost>
     ColMajorX X{yb, Wb, N};
     FEGB_TRY(be_gram(X, items, item0, item1, d_width, ns, Cw, d_gram, s, scr));
     FEGB_TRY(phase("gram"));
-    be_solve_kernel<<<ns, DN_THREADS, 0, s>>>(d_specs, d_gram, Cw, Kb, d_scratch, d_beta, d_Qinv, d_Pi);
+    static const cudaError_t solve_attr =
+        cudaFuncSetAttribute(be_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+    static const cudaError_t fin_attr =
+        cudaFuncSetAttribute(be_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+    if (solve_attr != cudaSuccess) return set_cuda_error(solve_attr, "batch solve attr");
+    if (fin_attr != cudaSuccess) return set_cuda_error(fin_attr, "batch finalize attr");
+    const size_t dn_bytes = dn_fits(Kb) ? dn_work_bytes(Kb) : 0;
+    be_solve_kernel<<<ns, DN_THREADS, dn_bytes, s>>>(d_specs, d_gram, Cw, Kb, d_scratch, d_beta, d_Qinv, d_Pi);
     FEGB_LAUNCH_CHECK("batch solve");
     FEGB_CUDA(cudaStreamSynchronize(s), "batch solve sync");
     const double t_regression = be_seconds_since(t0);
@@ -1099,7 +1113,7 @@ int estimate_class_batched(const fegb_config& cfg, const std::vector<BeSpecHost>
     FEGB_TRY(scr.alloc(&d_psd, (size_t)ns, "batch psd"));
     FEGB_CUDA(cudaMemcpyAsync(d_scalar, hscalar.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, s), "scalar copy");
     FEGB_CUDA(cudaMemcpyAsync(d_df, hdf.data(), sizeof(long long) * ns, cudaMemcpyHostToDevice, s), "dof copy");
-    be_finalize_kernel<<<ns, DN_THREADS, 0, s>>>(d_specs, Kb, d_Qinv, d_acc, d_scalar, d_rss, d_df, d_se, d_psd,
+    be_finalize_kernel<<<ns, DN_THREADS, dn_bytes, s>>>(d_specs, Kb, d_Qinv, d_acc, d_scalar, d_rss, d_df, d_se, d_psd,
                                                  d_scratch);
     FEGB_LAUNCH_CHECK("batch finalize");
     std::vector<double> hbeta((size_t)ns * Kb), hse((size_t)ns * Kb);

@@ -227,7 +227,11 @@ __global__ void __launch_bounds__(DN_THREADS)
     chol_solve_inv_kernel(int k, const double* __restrict__ Q, int ldq, const int* __restrict__ idx,
                           const double* __restrict__ b, double* __restrict__ beta, double* __restrict__ Qinv,
                           int* __restrict__ info, double* __restrict__ work) {
-    chol_solve_inv_block(k, Q, ldq, idx, b, beta, Qinv, info, work);
+    extern __shared__ __align__(16) unsigned char dn_smem[];
+    if (dn_fits(k))
+        chol_solve_inv_block(k, Q, ldq, idx, b, beta, Qinv, info, reinterpret_cast<double*>(dn_smem), dn_stride(k));
+    else
+        chol_solve_inv_block(k, Q, ldq, idx, b, beta, Qinv, info, work, k);
 }
 
 __global__ void gemm_small_kernel(int ta, int tb, int m, int n, int k, double alpha, const double* __restrict__ A,
@@ -258,7 +262,11 @@ __global__ void select_kernel(int k, const double* __restrict__ M, int ldm, cons
 __global__ void __launch_bounds__(DN_THREADS)
     finalize_cov_kernel(int k, double* __restrict__ acc, double scalar, int do_psd, double* __restrict__ se,
                         int* __restrict__ psd_applied, double* __restrict__ work) {
-    finalize_cov_block(k, acc, scalar, do_psd, se, psd_applied, work);
+    extern __shared__ __align__(16) unsigned char dn_smem[];
+    if (dn_fits(k))
+        finalize_cov_block(k, acc, scalar, do_psd, se, psd_applied, reinterpret_cast<double*>(dn_smem), dn_stride(k));
+    else
+        finalize_cov_block(k, acc, scalar, do_psd, se, psd_applied, work, k);
 }
 
 }  // namespace
@@ -808,7 +816,10 @@ int residual_scores(const double* X, int C, long long n, const double* beta, int
 int dense_chol_solve_inv(int k, const double* Q, int ldq, const int* idx_dev, const double* b, double* beta_out,
                          double* Qinv, int* info_dev, double* work, cudaStream_t s) {
     if (k <= 0) return 0;
-    chol_solve_inv_kernel<<<1, DN_THREADS, 0, s>>>(k, Q, ldq, idx_dev, b, beta_out, Qinv, info_dev, work);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(chol_solve_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+    if (attr != cudaSuccess) return set_cuda_error(attr, "cholesky attr");
+    chol_solve_inv_kernel<<<1, DN_THREADS, dn_fits(k) ? dn_work_bytes(k) : 0, s>>>(k, Q, ldq, idx_dev, b, beta_out, Qinv, info_dev, work);
     FEGB_LAUNCH_CHECK("cholesky");
     return 0;
 }
@@ -838,7 +849,10 @@ int dense_sandwich_acc(int k, const double* Qinv, const double* M, int ldm, cons
 int dense_finalize_cov(int k, double* acc, double scalar, int do_psd, double* se_out, int* psd_applied, double* work,
                        cudaStream_t s) {
     if (k <= 0) return 0;
-    finalize_cov_kernel<<<1, DN_THREADS, 0, s>>>(k, acc, scalar, do_psd, se_out, psd_applied, work);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(finalize_cov_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+    if (attr != cudaSuccess) return set_cuda_error(attr, "covariance finalize attr");
+    finalize_cov_kernel<<<1, DN_THREADS, dn_fits(k) ? dn_work_bytes(k) : 0, s>>>(k, acc, scalar, do_psd, se_out, psd_applied, work);
     FEGB_LAUNCH_CHECK("covariance finalize");
     return 0;
 }

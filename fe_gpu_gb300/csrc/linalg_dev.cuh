@@ -25,137 +25,153 @@ __device__ __forceinline__ void ds_fma(float2 x, float2 y, float& sh, float& sl)
     sl += err + (pe + cr);
 }
 
-// One block of DN_THREADS threads: Q_sel = Q[idx, idx] (or the leading k x k
-// block), upper Cholesky factor, solve for b_sel and the inverse. info: 0 ok,
-// j > 0 when the leading minor j is not positive definite. work: 2 k^2.
-__device__ inline void chol_solve_inv_block(int k, const double* __restrict__ Q, int ldq, const int* __restrict__ idx,
-                                     const double* __restrict__ b, double* __restrict__ beta,
-                                     double* __restrict__ Qinv, int* __restrict__ info, double* __restrict__ work) {
-    double* U = work;
-    double* Ui = work + (size_t)k * k;
-    __shared__ int s_info;
-    __shared__ double s_d;
-    const int t = threadIdx.x;
-    for (int e = t; e < k * k; e += DN_THREADS) {
-        int i = e % k, j = e / k;
-        int qi = idx ? idx[i] : i, qj = idx ? idx[j] : j;
-        U[e] = Q[qi + (long long)qj * ldq];
-    }
-    if (t == 0) s_info = 0;
+// Row stride and doubles of the two k x k work matrices of the dense routines:
+// odd strides where they sit in shared memory (lanes walk down columns without
+// bank conflicts). One block is bound by the latency of its steps: with the
+// matrices in global memory and a thread per column, k = 90 took 1.08 ms and the
+// eigensolver at k = 29 1.3; in shared memory, with the trailing matrix shared
+// by all warps, k = 100 takes 0.50 ms and a 30-column fit of 38k rows 6.1 -> 5.6.
+constexpr size_t DN_SMEM = 200 * 1024;
+__host__ __device__ inline int dn_stride(int k) { return k | 1; }
+__host__ __device__ inline size_t dn_work_bytes(int k) { return sizeof(double) * 2 * (size_t)k * dn_stride(k); }
+__host__ __device__ inline bool dn_fits(int k) { return dn_work_bytes(k) <= DN_SMEM; }
+
+// Upper Cholesky factor of the k x k matrix in U (row-major, stride ld, upper
+// triangle used), in place: each pivot row is scaled and subtracted from the
+// trailing rows, so an entry receives its terms in pivot order. Returns 0, or
+// j > 0 when the leading minor j is not positive (on every thread).
+__device__ inline int block_chol_factor(int k, double* U, int ld) {
+    __shared__ int s_fail;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    if (t == 0) s_fail = 0;
     __syncthreads();
     for (int j = 0; j < k; ++j) {
-        for (int c = j + t; c < k; c += DN_THREADS) {
-            double v = U[j + c * k];
-            for (int p = 0; p < j; ++p) v -= U[p + j * k] * U[p + c * k];
-            U[j + c * k] = v;
-        }
-        __syncthreads();
-        if (t == 0) {
-            double d = U[j + j * k];
+        double* rj = U + (size_t)j * ld;
+        if (warp == 0) {
+            const double d = rj[j];
             if (!(d > 0.0)) {
-                s_info = j + 1;
+                if (lane == 0) s_fail = j + 1;
             } else {
-                s_d = sqrt(d);
-                U[j + j * k] = s_d;
+                const double r = sqrt(d);
+                __syncwarp();
+                if (lane == 0) rj[j] = r;
+                for (int c = j + 1 + lane; c < k; c += 32) rj[c] /= r;
             }
         }
         __syncthreads();
-        if (s_info) break;
-        for (int c = j + 1 + t; c < k; c += DN_THREADS) U[j + c * k] /= s_d;
+        if (s_fail) break;
+        for (int r = j + 1 + warp; r < k; r += DN_THREADS / 32) {
+            const double f = rj[r];
+            double* row = U + (size_t)r * ld;
+            for (int c = r + lane; c < k; c += 32) row[c] = fma(-f, rj[c], row[c]);
+        }
         __syncthreads();
     }
-    if (s_info) {
-        if (t == 0) *info = s_info;
-        return;
-    }
-    // U^{-1}: column j by thread j (back substitution on the upper factor)
-    for (int j = t; j < k; j += DN_THREADS) {
-        for (int i = 0; i < k; ++i) Ui[i + j * k] = 0.0;
-        Ui[j + j * k] = 1.0 / U[j + j * k];
-        for (int i = j - 1; i >= 0; --i) {
-            double s = 0.0;
-            for (int p = i + 1; p <= j; ++p) s += U[i + p * k] * Ui[p + j * k];
-            Ui[i + j * k] = -s / U[i + i * k];
-        }
+    const int fail = s_fail;
+    __syncthreads();
+    return fail;
+}
+
+// One block of DN_THREADS threads: Q_sel = Q[idx, idx] (or the leading k x k
+// block), upper Cholesky factor, solve for b_sel and the inverse. info: 0 ok,
+// j > 0 when the leading minor j is not positive definite. work: 2 k ld doubles
+// (global or shared), ld >= k.
+__device__ inline void chol_solve_inv_block(int k, const double* __restrict__ Q, int ldq, const int* __restrict__ idx,
+                                     const double* __restrict__ b, double* __restrict__ beta,
+                                     double* __restrict__ Qinv, int* __restrict__ info, double* work, int ld) {
+    double* U = work;
+    double* X = work + (size_t)k * ld;  // U^{-1}, row-major
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (int e = t; e < k * k; e += DN_THREADS) {
+        int i = e % k, j = e / k;
+        int qi = idx ? idx[i] : i, qj = idx ? idx[j] : j;
+        U[(size_t)i * ld + j] = Q[qi + (long long)qj * ldq];
+        X[(size_t)i * ld + j] = 0.0;
     }
     __syncthreads();
-    // beta = U^{-1} U^{-T} b_sel, Qinv = U^{-1} U^{-T}
+    const int fail = block_chol_factor(k, U, ld);
+    if (fail) {
+        if (t == 0) *info = fail;
+        return;
+    }
+    // rows of U^{-1} from the last: X[i][j] gathers sum_p U[i][p] X[p][j] over the
+    // finished rows p > i, then row i is -that / U[i][i]
+    for (int p = k - 1; p >= 0; --p) {
+        double* xp = X + (size_t)p * ld;
+        const double u = U[(size_t)p * ld + p];
+        for (int j = p + t; j < k; j += DN_THREADS) xp[j] = j == p ? 1.0 / u : -xp[j] / u;
+        __syncthreads();
+        for (int i = warp; i < p; i += DN_THREADS / 32) {
+            const double f = U[(size_t)i * ld + p];
+            double* xi = X + (size_t)i * ld;
+            for (int j = p + lane; j < k; j += 32) xi[j] = fma(f, xp[j], xi[j]);
+        }
+        __syncthreads();
+    }
+    // Qinv = U^{-1} U^{-T}
     for (int e = t; e < k * k; e += DN_THREADS) {
         int i = e % k, j = e / k;
         if (i > j) continue;
         double s = 0.0;
-        for (int p = j; p < k; ++p) s += Ui[i + p * k] * Ui[j + p * k];
+        for (int p = j; p < k; ++p) s += X[(size_t)i * ld + p] * X[(size_t)j * ld + p];
         Qinv[i + j * k] = s;
         Qinv[j + i * k] = s;
     }
     __syncthreads();
-    if (t == 0) {
-        // forward then backward substitution (dpotrs order)
+    // beta: forward then backward substitution by one warp, the right-hand side
+    // in place of the first row of X
+    if (warp == 0) {
+        double* v = X;
+        for (int i = lane; i < k; i += 32) v[i] = b[idx ? idx[i] : i];
+        __syncwarp();
         for (int i = 0; i < k; ++i) {
-            double v = b[idx ? idx[i] : i];
-            for (int p = 0; p < i; ++p) v -= U[p + i * k] * beta[p];
-            beta[i] = v / U[i + i * k];
+            const double* ui = U + (size_t)i * ld;
+            const double y = v[i] / ui[i];
+            __syncwarp();
+            if (lane == 0) v[i] = y;
+            for (int c = i + 1 + lane; c < k; c += 32) v[c] = fma(-ui[c], y, v[c]);
+            __syncwarp();
         }
         for (int i = k - 1; i >= 0; --i) {
-            double v = beta[i];
-            for (int p = i + 1; p < k; ++p) v -= U[i + p * k] * beta[p];
-            beta[i] = v / U[i + i * k];
+            const double y = v[i] / U[(size_t)i * ld + i];
+            __syncwarp();
+            if (lane == 0) v[i] = y;
+            for (int c = lane; c < i; c += 32) v[c] = fma(-U[(size_t)c * ld + i], y, v[c]);
+            __syncwarp();
         }
-        *info = 0;
+        for (int i = lane; i < k; i += 32) beta[i] = v[i];
+        if (lane == 0) *info = 0;
     }
+    __syncthreads();
 }
 
 // One block: whether the symmetric k x k matrix A (upper triangle read) has an
 // upper Cholesky factor with positive pivots, i.e. is positive definite; the
-// factor is formed in U (k^2 doubles). The answer is the same on every thread.
-__device__ inline bool block_cholesky_ok(int k, const double* __restrict__ A, double* __restrict__ U) {
-    __shared__ int s_fail;
-    __shared__ double s_d;
+// factor is formed in U (k ld doubles). The answer is the same on every thread.
+__device__ inline bool block_cholesky_ok(int k, const double* __restrict__ A, double* U, int ld) {
     const int t = threadIdx.x;
-    for (int e = t; e < k * k; e += DN_THREADS) U[e] = A[e];
-    if (t == 0) s_fail = 0;
+    for (int e = t; e < k * k; e += DN_THREADS) U[(size_t)(e / k) * ld + e % k] = A[e / k + (long long)(e % k) * k];
     __syncthreads();
-    for (int j = 0; j < k; ++j) {
-        for (int c = j + t; c < k; c += DN_THREADS) {
-            double v = U[j + c * k];
-            for (int p = 0; p < j; ++p) v -= U[p + j * k] * U[p + c * k];
-            U[j + c * k] = v;
-        }
-        __syncthreads();
-        if (t == 0) {
-            const double d = U[j + j * k];
-            if (!(d > 0.0))
-                s_fail = 1;
-            else
-                s_d = sqrt(d);
-        }
-        __syncthreads();
-        if (s_fail) break;
-        for (int c = j + 1 + t; c < k; c += DN_THREADS) U[j + c * k] /= s_d;
-        __syncthreads();
-    }
-    const bool ok = s_fail == 0;
-    __syncthreads();
-    return ok;
+    return block_chol_factor(k, U, ld) == 0;
 }
 
-// Parallel cyclic Jacobi on a k x k symmetric matrix A (in place; global
-// memory), eigenvectors accumulated in V; the round-robin pairing makes all
+// Parallel cyclic Jacobi on a k x k symmetric matrix A (in place, stride
+// ld), eigenvectors accumulated in V (stride ld); the round-robin pairing makes all
 // rotations of one round touch disjoint rows/columns.
-__device__ inline void block_jacobi(int k, double* A, double* V) {
+__device__ inline void block_jacobi(int k, double* A, double* V, int ld) {
     __shared__ int sp[DN_THREADS], sq[DN_THREADS];
     __shared__ double sc[DN_THREADS], ss[DN_THREADS];
     __shared__ double s_off, s_tot;
     __shared__ double red[DN_THREADS / 32];
     const int t = threadIdx.x;
-    for (int e = t; e < k * k; e += DN_THREADS) V[e] = (e % k == e / k) ? 1.0 : 0.0;
+    for (int e = t; e < k * k; e += DN_THREADS) V[e % k + (size_t)(e / k) * ld] = (e % k == e / k) ? 1.0 : 0.0;
     const int kk = (k % 2) ? k + 1 : k;
     const int m = kk / 2;
     __syncthreads();
     for (int sweep = 0; sweep < 60; ++sweep) {
         double off = 0.0, tot = 0.0;
         for (int e = t; e < k * k; e += DN_THREADS) {
-            double a = A[e] * A[e];
+            const double v = A[e % k + (size_t)(e / k) * ld], a = v * v;
             tot += a;
             if (e % k != e / k) off += a;
         }
@@ -193,9 +209,9 @@ __device__ inline void block_jacobi(int k, double* A, double* V) {
                 }
                 double c = 1.0, s = 0.0;
                 if (q < k) {
-                    double apq = A[p + q * k];
+                    double apq = A[p + q * ld];
                     if (apq != 0.0) {
-                        double app = A[p + p * k], aqq = A[q + q * k];
+                        double app = A[p + p * ld], aqq = A[q + q * ld];
                         double theta = (aqq - app) / (2.0 * apq);
                         double tt = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
                         c = 1.0 / sqrt(tt * tt + 1.0);
@@ -214,12 +230,12 @@ __device__ inline void block_jacobi(int k, double* A, double* V) {
                 int p = sp[i], q = sq[i];
                 if (q >= k || ss[i] == 0.0) continue;
                 double c = sc[i], s = ss[i];
-                double arp = A[r + p * k], arq = A[r + q * k];
-                A[r + p * k] = c * arp - s * arq;
-                A[r + q * k] = s * arp + c * arq;
-                double vrp = V[r + p * k], vrq = V[r + q * k];
-                V[r + p * k] = c * vrp - s * vrq;
-                V[r + q * k] = s * vrp + c * vrq;
+                double arp = A[r + p * ld], arq = A[r + q * ld];
+                A[r + p * ld] = c * arp - s * arq;
+                A[r + q * ld] = s * arp + c * arq;
+                double vrp = V[r + p * ld], vrq = V[r + q * ld];
+                V[r + p * ld] = c * vrp - s * vrq;
+                V[r + q * ld] = s * vrp + c * vrq;
             }
             __syncthreads();
             // rows: A <- J^T A
@@ -228,9 +244,9 @@ __device__ inline void block_jacobi(int k, double* A, double* V) {
                 int p = sp[i], q = sq[i];
                 if (q >= k || ss[i] == 0.0) continue;
                 double c = sc[i], s = ss[i];
-                double apc = A[p + col * k], aqc = A[q + col * k];
-                A[p + col * k] = c * apc - s * aqc;
-                A[q + col * k] = s * apc + c * aqc;
+                double apc = A[p + col * ld], aqc = A[q + col * ld];
+                A[p + col * ld] = c * apc - s * aqc;
+                A[q + col * ld] = s * apc + c * aqc;
             }
             __syncthreads();
         }
@@ -239,13 +255,13 @@ __device__ inline void block_jacobi(int k, double* A, double* V) {
 
 // One block: acc *= scalar, then the PSD fix (mirror, Jacobi, clamp
 // negative eigenvalues, rebuild) or the CPU path's symmetrisation; se[i] =
-// sqrt(max(0, acc[i, i])). work: 2 k^2.
+// sqrt(max(0, acc[i, i])). work: 2 k ld doubles, ld >= k.
 __device__ inline void finalize_cov_block(int k, double* __restrict__ acc, double scalar, int do_psd,
                                    double* __restrict__ se, int* __restrict__ psd_applied,
-                                   double* __restrict__ work) {
+                                   double* work, int ld) {
     const int t = threadIdx.x;
     double* A = work;
-    double* V = work + (size_t)k * k;
+    double* V = work + (size_t)k * ld;
     __shared__ int s_applied;
     if (t == 0) s_applied = 0;
     for (int e = t; e < k * k; e += DN_THREADS) acc[e] *= scalar;
@@ -254,10 +270,10 @@ __device__ inline void finalize_cov_block(int k, double* __restrict__ acc, doubl
         // 0.5 (A + A^T), as the CPU path does (fe_pipeline.f90:476)
         for (int e = t; e < k * k; e += DN_THREADS) {
             int i = e % k, j = e / k;
-            A[e] = 0.5 * (acc[i + j * k] + acc[j + i * k]);
+            A[i + (size_t)j * ld] = 0.5 * (acc[i + j * k] + acc[j + i * k]);
         }
         __syncthreads();
-        for (int e = t; e < k * k; e += DN_THREADS) acc[e] = A[e];
+        for (int e = t; e < k * k; e += DN_THREADS) acc[e] = A[e % k + (size_t)(e / k) * ld];
         __syncthreads();
         for (int i = t; i < k; i += DN_THREADS) se[i] = sqrt(fmax(0.0, acc[i + i * k]));
         if (t == 0) *psd_applied = 0;
@@ -269,34 +285,34 @@ __device__ inline void finalize_cov_block(int k, double* __restrict__ acc, doubl
         if (i > j) acc[e] = acc[j + i * k];
     }
     __syncthreads();
-    for (int e = t; e < k * k; e += DN_THREADS) A[e] = acc[e];
+    for (int e = t; e < k * k; e += DN_THREADS) A[e % k + (size_t)(e / k) * ld] = acc[e];
     __syncthreads();
     // A positive definite matrix has no negative eigenvalue to clamp, and its
     // reconstruction V diag(lambda) V' is the matrix itself up to rounding:
     // the eigensolver (about 24 ms at k = 90) runs only when the Cholesky
     // factorisation fails
-    if (block_cholesky_ok(k, A, V)) {
+    if (block_cholesky_ok(k, acc, V, ld)) {
         for (int i = t; i < k; i += DN_THREADS) se[i] = sqrt(fmax(0.0, acc[i + i * k]));
         if (t == 0) *psd_applied = 0;
         return;
     }
-    block_jacobi(k, A, V);
+    block_jacobi(k, A, V, ld);
     __syncthreads();
     // lambda_j = A[j,j]; scale eigenvector columns by sqrt(max(lambda,0))
     for (int e = t; e < k * k; e += DN_THREADS) {
         int j = e / k;
-        double lam = A[j + j * k];
+        double lam = A[j + (size_t)j * ld];
         if (lam < 0.0) {
             s_applied = 1;
             lam = 0.0;
         }
-        V[e] *= lam > 0.0 ? sqrt(lam) : 0.0;
+        V[e % k + (size_t)j * ld] *= lam > 0.0 ? sqrt(lam) : 0.0;
     }
     __syncthreads();
     for (int e = t; e < k * k; e += DN_THREADS) {
         int i = e % k, j = e / k;
         double s = 0.0;
-        for (int p = 0; p < k; ++p) s += V[i + p * k] * V[j + p * k];
+        for (int p = 0; p < k; ++p) s += V[i + (size_t)p * ld] * V[j + (size_t)p * ld];
         acc[e] = s;
     }
     __syncthreads();
