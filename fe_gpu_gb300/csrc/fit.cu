@@ -17,6 +17,7 @@
 #include <thread>
 #include <string>
 #include <mutex>
+#include <condition_variable>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -2087,12 +2088,21 @@ __global__ void cg_loop_check_kernel(const unsigned long long* __restrict__ zmax
     cudaGraphSetConditional(h, stop ? 0u : 1u);
 }
 
+// Loop graphs are captured, instantiated and destroyed by one host thread at a
+// time: threads doing so side by side (the classes of a batch) hung under the
+// activity tracing of a profiler.
+std::mutex& graph_mutex() {
+    static std::mutex mu;
+    return mu;
+}
+
 template <typename T>
 struct CGGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     CGLoopCtl* ctl = nullptr;  // device
     ~CGGraph() {
+        std::lock_guard<std::mutex> lk(graph_mutex());
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
     }
@@ -2102,6 +2112,7 @@ struct CGGraph {
 // refuses any step, in which case the caller keeps the host loop.
 template <typename T>
 int cg_build_graph(Problem& P, CGBuffers<T>& B, CGGraph<T>& G) {
+    std::lock_guard<std::mutex> lk(graph_mutex());
     if (cudaGraphCreate(&G.graph, 0) != cudaSuccess) return 1;
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, G.graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) return 1;
@@ -3745,6 +3756,8 @@ int within_impl(const fegb_config& cfg, long long n, int k, int l, int n_fe, dou
 // on its own rows with the single-fit code, the within-transform skipped.
 
 constexpr int BATCH_MAX_FE = SWEEP_MAXP;
+constexpr int BATCH_CLASS_THREADS = 6;    // classes at a time
+constexpr double BATCH_MEMORY = 0.4;      // of the free memory, for all but the first class at a time
 constexpr int BATCH_FIT_THREADS = 8;  // host threads (one stream each) fitting specifications after the demean
 
 struct BatchSpecDev {
@@ -3861,15 +3874,9 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
     for (int i = 0; i < n_specs; ++i) order.push_back({batch_class(1 + specs[i].k + specs[i].l), i});
     std::stable_sort(order.begin(), order.end(),
                      [](const std::pair<int, int>& a, const std::pair<int, int>& b) { return a.first < b.first; });
-    size_t pos = 0;
-    while (pos < order.size()) {
-        size_t end = pos;
-        while (end < order.size() && order[end].first == order[pos].first) ++end;
-        const int cb = order[pos].first;
+    // one class of specifications (their indices idx) on one stream
+    auto run_class = [&](const int cb, const std::vector<int>& idx, cudaStream_t s) -> int {
         const int kb = cb - 1;
-        std::vector<int> idx;
-        for (size_t t = pos; t < end; ++t) idx.push_back(order[t].second);
-        pos = end;
         const int ns = (int)idx.size();
         Scratch scr(s);
         std::vector<BatchSpecDev> hs(ns);
@@ -4006,7 +4013,7 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
                                  "fegb batch: class of %d columns: %d specs, %lld rows, within-transform %.1f ms "
                                  "(%d CG), batched estimation %.1f ms\n",
                                  cb, ns, N, t_within * 1e3, pre.iterations, seconds_since(tc0) * 1e3);
-                continue;
+                return 0;
             }
         }
         // every specification on its own demeaned rows; the fits are
@@ -4085,6 +4092,92 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
             std::fprintf(stderr, "fegb batch: class of %d columns: %d specs, %lld rows, within-transform %.1f ms (%d CG), "
                                  "per-spec fits %.1f ms\n",
                          cb, ns, N, t_within * 1e3, pre.iterations, seconds_since(tc0) * 1e3);
+        return 0;
+    };
+    // the classes, largest first
+    struct BatchClass {
+        int cb;
+        std::vector<int> idx;
+        double bytes;  // device memory while it runs: the stack, the data block, scores, ids and orders
+    };
+    std::vector<BatchClass> classes;
+    for (size_t pos = 0; pos < order.size();) {
+        BatchClass c{order[pos].first, {}, 0.0};
+        double rows = 0.0;
+        for (; pos < order.size() && order[pos].first == c.cb; ++pos) {
+            c.idx.push_back(order[pos].second);
+            rows += (double)specs[order[pos].second].n;
+        }
+        c.bytes = rows * (8.0 * 5 * c.cb + 4.0 * 40);
+        classes.push_back(std::move(c));
+    }
+    std::stable_sort(classes.begin(), classes.end(),
+                     [](const BatchClass& x, const BatchClass& y) { return x.bytes > y.bytes; });
+    // A class is a chain of some hundred launches and readbacks of its own; a few
+    // classes run side by side, each on a stream and a host thread, as far as
+    // BATCH_MEMORY of the free memory goes (60 specifications of 5k to 200k rows,
+    // six classes: 57 ms one after the other, 31 side by side). Profiled fits run one class at a time: their launch
+    // timings would overlap.
+    const int n_threads = cfg.profile ? 1 : (int)std::min<size_t>(classes.size(), BATCH_CLASS_THREADS);
+    if (n_threads <= 1) {
+        for (const BatchClass& c : classes) FEGB_TRY(run_class(c.cb, c.idx, s));
+        return set_ok();
+    }
+    size_t free_b = 0, total_b = 0;
+    FEGB_CUDA(cudaMemGetInfo(&free_b, &total_b), "batch memory");
+    const double budget = BATCH_MEMORY * (double)free_b;
+    int dev = 0;
+    FEGB_CUDA(cudaGetDevice(&dev), "batch device");
+    cudaEvent_t ready = nullptr;  // the inputs, as far as the caller's stream has them queued
+    FEGB_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "batch event");
+    int st = cudaEventRecord(ready, s) == cudaSuccess ? 0 : set_error("batch: cannot record on the stream");
+    std::mutex mu;
+    std::condition_variable room;
+    double in_use = 0.0;
+    size_t next = 0;
+    int running = 0;
+    std::string message;
+    auto worker = [&]() {
+        cudaStream_t ws = nullptr;
+        int err = 0;
+        if (cudaSetDevice(dev) != cudaSuccess || cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaStreamWaitEvent(ws, ready, 0) != cudaSuccess)
+            err = set_error("batch: cannot create a stream for a class");
+        std::unique_lock<std::mutex> lk(mu);
+        while (!err && !st && next < classes.size()) {
+            const BatchClass& c = classes[next];
+            if (running > 0 && in_use + c.bytes > budget) {
+                room.wait(lk);
+                continue;
+            }
+            ++next;
+            ++running;
+            in_use += c.bytes;
+            lk.unlock();
+            err = run_class(c.cb, c.idx, ws);
+            if (cudaStreamSynchronize(ws) != cudaSuccess && !err) err = set_error("batch: a class failed on the device");
+            lk.lock();
+            --running;
+            in_use -= c.bytes;
+            room.notify_all();
+        }
+        if (err && !st) {
+            st = err;
+            message = last_error();
+            room.notify_all();
+        }
+        lk.unlock();
+        if (ws) cudaStreamDestroy(ws);
+    };
+    if (!st) {
+        std::vector<std::thread> pool;
+        for (int t = 0; t < n_threads; ++t) pool.emplace_back(worker);
+        for (auto& th : pool) th.join();
+    }
+    cudaEventDestroy(ready);
+    if (st) {
+        if (!message.empty()) set_error("%s", message.c_str());
+        return st;
     }
     return set_ok();
 }
