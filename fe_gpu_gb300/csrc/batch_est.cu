@@ -44,7 +44,11 @@ double be_seconds_since(BeClock::time_point t0) {
 }
 
 constexpr int BE_THREADS = 256;
-constexpr int BE_ITEM_ROWS = 16384;  // rows (or clusters) per work item
+// Rows (or clusters) per work item: the class cut into some BE_ITEMS items, so that
+// small classes fill the chip too (0.8M rows of 24 columns in 16384-row items
+// left two thirds of the SMs idle), within these limits.
+constexpr int BE_ITEMS = 1216;
+constexpr int BE_ITEM_MIN = 1024, BE_ITEM_MAX = 16384;
 // rows per shared-memory tile of the Gram: about 4096 values (32 KB as FP64),
 // a multiple of 32 between 32 and 256
 __host__ __device__ inline int be_tile_rows(int Cw) {
@@ -789,9 +793,12 @@ void be_items(const std::vector<long long>& begin, const std::vector<long long>&
     items.clear();
     item0.assign(ns, 0);
     item1.assign(ns, 0);
+    long long total = 0;
+    for (int s = 0; s < ns; ++s) total += std::max(0LL, end[s] - begin[s]);
+    const long long rows = std::min<long long>(BE_ITEM_MAX, std::max<long long>(BE_ITEM_MIN, (total / BE_ITEMS + 255) / 256 * 256));
     for (int s = 0; s < ns; ++s) {
         item0[s] = (int)items.size();
-        for (long long r = begin[s]; r < end[s]; r += BE_ITEM_ROWS) items.push_back({s, r, std::min(end[s], r + BE_ITEM_ROWS)});
+        for (long long r = begin[s]; r < end[s]; r += rows) items.push_back({s, r, std::min(end[s], r + rows)});
         item1[s] = (int)items.size();
     }
 }
