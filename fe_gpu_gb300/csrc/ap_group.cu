@@ -398,14 +398,15 @@ __device__ __forceinline__ V warp_slot_sum(V v, int slot, int slots, int C, int 
     return v;
 }
 
-// acc[t] += N[g][t] * tab[g][c] over this lane's groups, t from piece w of the rows on
-template <typename CT, int GT>
-__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const double* __restrict__ tab,
-                                           int ld, int c, int k, long long g, long long Ge, long long gstep,
-                                           FixSum (&acc)[GT]) {
+// acc[t] += N[g][t] * tab[g][c] over this lane's groups, t from piece w of the rows
+// on. WRITTEN: the table was written by this launch (read past L1).
+template <typename CT, int GT, bool WRITTEN = false>
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const double* tab, int ld, int c,
+                                           int k, long long g, long long Ge, long long gstep, FixSum (&acc)[GT]) {
 #pragma unroll 2
     for (; g < Ge; g += gstep) {
-        const FixDigits a = fix_digits(to_fixed(tab[g * ld + c], k));
+        const double* at = tab + g * ld + c;
+        const FixDigits a = fix_digits(to_fixed(WRITTEN ? __ldcg(at) : *at, k));
 #pragma unroll
         for (int q = 0; q < GT; q += AP_PART) {
             const Counts16 n = load_counts(N + g * pitch, w + q / AP_PART);
@@ -609,6 +610,320 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > AP_PART ? 1
         if (cmax[i] > t.amax[i]) t.amax[i] = cmax[i];
 }
 
+
+// ------------------------ one large dimension, small others ------------------------
+
+// Barrier of all blocks of a cooperative launch, the n-th one. Bounded: after
+// about a second of waiting the error word is set and every block leaves.
+__device__ __forceinline__ bool star_barrier(const ApStar& p, unsigned n, int* s_bad) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned target = n * gridDim.x;
+        atomicAdd(p.arrived, 1u);
+        volatile unsigned* a = p.arrived;
+        volatile int* e = p.error;
+        int bad = 0;
+        for (long long spin = 0; *a < target; ++spin) {
+            if ((spin & 1023) == 1023 && *e) {
+                bad = 1;
+                break;
+            }
+            if (spin > (1LL << 23)) {
+                *e = 1;
+                bad = 1;
+                break;
+            }
+            if (spin > 64) __nanosleep(64);
+        }
+        __threadfence();
+        *s_bad = bad;
+    }
+    __syncthreads();
+    return *s_bad == 0;
+}
+
+// relaxation after a projection whose largest update was cd (fe_gpu_demean.f90:213-218)
+__device__ __forceinline__ void star_relax(double& relax, double& pc, double cd) {
+    if (cd > pc * 1.05)
+        relax = fmax(0.4, relax * 0.5);
+    else if (cd < pc * 0.8)
+        relax = fmin(2.0, relax * 1.10);
+    pc = cd;
+}
+
+__device__ __forceinline__ unsigned long long block_umax(unsigned long long v, unsigned long long* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = umax64(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+#pragma unroll
+    for (int w = 1; w < AP_THREADS / 32; ++w) v = umax64(v, red[w]);
+    return v;
+}
+
+// 28k rows over 3500/15/13 groups, 6 columns, 13 iterations, from host arrays: 3.1 ms
+// with a launch per visit, 2.25 in one.
+__global__ void __launch_bounds__(AP_THREADS, 2) ap_star_kernel(const __grid_constant__ ApStar p) {
+    extern __shared__ __align__(16) unsigned char ap_smem[];
+    __shared__ int s_bad;
+    __shared__ unsigned long long s_red[AP_THREADS / 32];
+    __shared__ double s_relax[SWEEP_MAXP + 1], s_pc[SWEEP_MAXP + 1];  // small dimensions, then the large one
+    const int C = p.w.C, ld = p.w.ld, ns = p.n_small;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int WARPS = AP_THREADS / 32;
+    // shared memory: column maxima | reduction area | per small dimension tab,
+    // prev, mu, sums over w (Gs x C each), inv (Gs) | digit tables
+    unsigned long long* cmax = reinterpret_cast<unsigned long long*>(ap_smem);  // 32
+    long long* red = reinterpret_cast<long long*>(cmax + 32);                   // max(WARPS x AP_PART x C x 2, AP_THREADS)
+    double* f = reinterpret_cast<double*>(red + max(WARPS * AP_PART * C * 2, AP_THREADS));
+    double *tab[SWEEP_MAXP], *prev[SWEEP_MAXP], *mu[SWEEP_MAXP], *tw[SWEEP_MAXP], *inv[SWEEP_MAXP];
+    int sum_at[SWEEP_MAXP];
+    int words = 0;
+    for (int i = 0; i < ns; ++i) {
+        const int P = p.s[i].G * C;
+        tab[i] = f;
+        prev[i] = f + P;
+        mu[i] = f + 2 * P;
+        tw[i] = f + 3 * P;
+        inv[i] = f + 4 * P;
+        f += 4 * P + p.s[i].G;
+        sum_at[i] = words;
+        words += 2 * P;
+        for (int e = threadIdx.x; e < P; e += AP_THREADS) {
+            tab[i][e] = 0.0;
+            prev[i][e] = p.s[i].prev[e];
+            mu[i][e] = p.s[i].mu[e];
+            tw[i][e] = 0.0;
+        }
+        for (int g = threadIdx.x; g < p.s[i].G; g += AP_THREADS) inv[i][g] = p.s[i].inv[g];
+    }
+    FixDigits* digits = reinterpret_cast<FixDigits*>(f);
+    if (threadIdx.x <= ns) {
+        s_relax[threadIdx.x] = p.relax[p.relax_at[threadIdx.x]];
+        s_pc[threadIdx.x] = p.prev_change[p.relax_at[threadIdx.x]];
+    }
+    __syncthreads();
+    // this block's groups of the large dimension
+    const int G = p.w.G;
+    const int gb0 = (int)((long long)G * blockIdx.x / gridDim.x), gb1 = (int)((long long)G * (blockIdx.x + 1) / gridDim.x);
+    const int rps = AP_THREADS / C;
+    const int rr = (int)threadIdx.x / C;
+    const int c = (int)threadIdx.x - rr * C;
+    const bool active = rr < rps;
+    const int slots = 32 / C, slot = lane / C, sc = lane - slot * C;
+    int top = 1;
+    while (top < slots) top <<= 1;
+    top >>= 1;
+    unsigned long long it_max = 0;  // largest update of the iteration
+    unsigned barrier = 0;
+    int turn = 0;     // projections of w so far (ring of change)
+    int visit = 0;    // visits of w so far (ring of sums)
+    int iter = 0;
+    bool stop = false, ok = true;
+
+    // n projections in a row of small dimension i, by every block alike
+    auto small_visit = [&](int i, int n) {
+        const int Gi = p.s[i].G, P = Gi * C;
+        for (int j = 0; j < n; ++j) {
+            unsigned long long upd = 0;
+            const double relax = s_relax[i];
+            for (int e = threadIdx.x; e < P; e += AP_THREADS) {
+                const int t = e / C, cc = e - t * C;
+                double T = tw[i][e];
+                for (int o = 0; o < ns; ++o) {
+                    if (o == i) continue;
+                    const ApDense<double>& D = p.ss[i][o];
+                    const int pitch = ap_count_pitch(Gi);
+                    const double* to = tab[o] + cc;
+                    if (D.wide) {
+                        const uint32_t* N = static_cast<const uint32_t*>(D.N) + t;
+                        for (int g = 0; g < D.Ge; ++g) T = fma((double)N[g * pitch], to[g * C], T);
+                    } else {
+                        const uint8_t* N = static_cast<const uint8_t*>(D.N) + t;
+                        for (int g = 0; g < D.Ge; ++g) T = fma((double)N[g * pitch], to[g * C], T);
+                    }
+                }
+                const double a = tab[i][e];
+                const double mean = fma(-T, inv[i][t], mu[i][e]) - a;
+                const double pv = prev[i][e];
+                const double mixed = pv + relax * (mean - pv);
+                prev[i][e] = mixed;
+                tab[i][e] = a + mixed;
+                upd = umax64(upd, update_bits(mixed));
+            }
+            upd = block_umax(upd, s_red);
+            it_max = umax64(it_max, upd);
+            if (threadIdx.x == 0) star_relax(s_relax[i], s_pc[i], bits_dbl(upd));
+            __syncthreads();
+        }
+    };
+    // the largest update of the projection of w in `turn`, once all blocks are in
+    auto close_projection = [&](unsigned long long upd) {
+        upd = block_umax(upd, s_red);
+        unsigned long long* ch = p.change + turn % AP_STAR_RING;
+        if (threadIdx.x == 0) {
+            if (upd) atomicMax(ch, upd);
+            if (blockIdx.x == 0) p.change[(turn + 2) % AP_STAR_RING] = 0ULL;  // last read two projections ago
+        }
+        if (!star_barrier(p, ++barrier, &s_bad)) return false;
+        const unsigned long long all = __ldcg(ch);
+        it_max = umax64(it_max, all);
+        if (threadIdx.x == 0) star_relax(s_relax[ns], s_pc[ns], bits_dbl(all));
+        ++turn;
+        __syncthreads();
+        return true;
+    };
+    auto visit_w = [&]() {
+        // digits of the small tables, one scale per column over all of them
+        for (int cc = threadIdx.x; cc < C; cc += AP_THREADS) {
+            unsigned long long m = 0;
+            for (int i = 0; i < ns; ++i)
+                for (int t = 0; t < p.s[i].G; ++t) m = umax64(m, abs_bits(tab[i][t * C + cc]));
+            cmax[cc] = m;
+        }
+        __syncthreads();
+        {
+            FixDigits* d = digits;
+            for (int i = 0; i < ns; ++i) {
+                const int Gi = p.s[i].G;
+                for (int e = threadIdx.x; e < four_rows(Gi) * C; e += AP_THREADS) {
+                    const int t = e / C;
+                    d[e] = fix_digits(to_fixed(t < Gi ? tab[i][e] : 0.0, fix_exponent(cmax[e - t * C])));
+                }
+                d += four_rows(Gi) * C;
+            }
+        }
+        if (blockIdx.x == 0) {  // the ring entry after the next one: last read two visits ago
+            unsigned long long* z = p.sums + (size_t)((visit + 2) % AP_STAR_RING) * words;
+            for (int e = threadIdx.x; e < words; e += AP_THREADS) z[e] = 0ULL;
+        }
+        __syncthreads();
+        double relax = s_relax[ns];
+        unsigned long long upd = 0;
+        if (active)
+            for (int g = gb0 + rr; g < gb1; g += rps) {
+                const long long idx = (long long)g * C + c;
+                FixSum fs{0, 0};
+                const FixDigits* d = digits;
+                for (int i = 0; i < ns; ++i) {
+                    if (p.sw[i].wide)
+                        dense_dot_fixed<uint32_t>(p.sw[i].N, g, p.s[i].G, d, C, c, fs);
+                    else
+                        dense_dot_fixed<uint8_t>(p.sw[i].N, g, p.s[i].G, d, C, c, fs);
+                    d += four_rows(p.s[i].G) * C;
+                }
+                const double base = fma(-fix_value(fs, cmax[c]), p.w.inv[g], p.w.mu[idx]);
+                p.w.base[idx] = base;
+                double* a = p.w.tab + (long long)g * ld + c;
+                const double av = *a, pv = p.w.prev[idx];
+                const double mixed = pv + relax * (base - av - pv);
+                p.w.prev[idx] = mixed;
+                *a = av + mixed;
+                upd = umax64(upd, update_bits(mixed));
+            }
+        if (!close_projection(upd)) return false;
+        relax = s_relax[ns];
+        upd = 0;
+        unsigned long long am = 0;
+        if (active)
+            for (int g = gb0 + rr; g < gb1; g += rps) {
+                const long long idx = (long long)g * C + c;
+                double* a = p.w.tab + (long long)g * ld + c;
+                const double av = *a, pv = p.w.prev[idx];
+                const double mixed = pv + relax * (p.w.base[idx] - av - pv);
+                p.w.prev[idx] = mixed;
+                const double an = av + mixed;
+                *a = an;
+                upd = umax64(upd, update_bits(mixed));
+                am = umax64(am, abs_bits(an));
+            }
+        unsigned long long* ured = reinterpret_cast<unsigned long long*>(red);
+        __syncthreads();
+        ured[threadIdx.x] = active ? am : 0ULL;
+        __syncthreads();
+        if ((int)threadIdx.x < C) {
+            unsigned long long m = 0;
+            for (int j = 0; j < rps; ++j) m = umax64(m, ured[j * C + threadIdx.x]);
+            if (m > __ldcg(p.w.amax + threadIdx.x)) atomicMax(p.w.amax + threadIdx.x, m);
+        }
+        if (!close_projection(upd)) return false;
+        // sums over this block's groups for every small dimension, a piece of
+        // AP_PART of its groups at a time
+        unsigned long long* sums = p.sums + (size_t)(visit % AP_STAR_RING) * words;
+        const int k = fix_exponent(__ldcg(p.w.amax + sc));
+        const int g0 = slot < slots ? gb0 + warp * slots + slot : gb1;
+        for (int i = 0; i < ns; ++i) {
+            const int Gi = p.s[i].G;
+            for (int t0 = 0; t0 < Gi; t0 += AP_PART) {
+                FixSum acc[AP_PART];
+#pragma unroll
+                for (int q = 0; q < AP_PART; ++q) acc[q] = FixSum{0, 0};
+                if (p.sw[i].wide)
+                    small_walk<uint32_t, AP_PART, true>(static_cast<const uint32_t*>(p.sw[i].N), ap_count_pitch(Gi),
+                                                  t0 / AP_PART, p.w.tab, ld, sc, k, g0, gb1, WARPS * slots, acc);
+                else
+                    small_walk<uint8_t, AP_PART, true>(static_cast<const uint8_t*>(p.sw[i].N), ap_count_pitch(Gi),
+                                                 t0 / AP_PART, p.w.tab, ld, sc, k, g0, gb1, WARPS * slots, acc);
+                const int nt = min(AP_PART, Gi - t0), PB = nt * C;
+                __syncthreads();  // red of the previous piece has been read
+#pragma unroll
+                for (int q = 0; q < AP_PART; ++q) {
+                    if (q >= nt) break;
+                    const long long lo = warp_slot_sum(acc[q].lo, slot, slots, C, top);
+                    const long long hi = warp_slot_sum(acc[q].hi, slot, slots, C, top);
+                    if (lane < C) {
+                        red[2 * (warp * PB + q * C + lane)] = lo;
+                        red[2 * (warp * PB + q * C + lane) + 1] = hi;
+                    }
+                }
+                __syncthreads();
+                for (int e = threadIdx.x; e < 2 * PB; e += AP_THREADS) {
+                    long long v = 0;
+                    for (int w = 0; w < WARPS; ++w) v += red[2 * w * PB + e];
+                    if (v) atomicAdd(sums + sum_at[i] + 2 * t0 * C + e, (unsigned long long)v);
+                }
+            }
+        }
+        if (!star_barrier(p, ++barrier, &s_bad)) return false;
+        for (int i = 0; i < ns; ++i)
+            for (int e = threadIdx.x; e < p.s[i].G * C; e += AP_THREADS) {
+                const unsigned long long* l = sums + sum_at[i] + 2 * e;
+                const FixSum fs{(long long)__ldcg(l + 1), (long long)__ldcg(l)};
+                tw[i][e] = fix_value(fs, __ldcg(p.w.amax + e % C));
+            }
+        ++visit;
+        __syncthreads();
+        return true;
+    };
+
+    while (iter < p.max_iter && !stop && ok) {
+        it_max = 0;
+        for (int half = 0; half < 2 && ok; ++half) {
+            // up through the small dimensions, the large one twice, and down again;
+            // the first projection after the other half's last is of the same dimension
+            for (int i = 0; i < ns; ++i) small_visit(i, 1);
+            ok = visit_w();
+            if (!ok) break;
+            for (int i = ns - 1; i >= 0; --i) small_visit(i, 1);
+        }
+        ++iter;
+        stop = bits_dbl(it_max) < p.ctl->tol;
+    }
+    if (blockIdx.x == 0) {
+        for (int i = 0; i < ns; ++i)
+            for (int e = threadIdx.x; e < p.s[i].G * C; e += AP_THREADS)
+                p.s[i].tab[(e / C) * p.s[i].ld + e % C] = tab[i][e];
+        if (threadIdx.x == 0) {
+            p.ctl->iterations = iter;
+            p.ctl->max_update = bits_dbl(it_max);
+            p.ctl->stop = stop ? 1 : 0;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(AP_THREADS) ap_load_kernel(const double* __restrict__ inc, long long G, int C, int ld,
                                                              double* __restrict__ tab, double* __restrict__ total,
                                                              unsigned long long* __restrict__ amax) {
@@ -808,6 +1123,44 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s) {
 }
 template int launch_ap_small<float>(const ApSmall<float>&, cudaStream_t);
 template int launch_ap_small<double>(const ApSmall<double>&, cudaStream_t);
+
+size_t ap_star_sums(const ApStar& p) {
+    size_t w = 0;
+    for (int i = 0; i < p.n_small; ++i) w += 2 * (size_t)p.s[i].G * p.w.C;
+    return w;
+}
+size_t ap_star_smem(const ApStar& p) {
+    const int C = p.w.C;
+    size_t b = sizeof(unsigned long long) * 32 +
+               sizeof(long long) * (size_t)std::max((AP_THREADS / 32) * AP_PART * C * 2, AP_THREADS);
+    for (int i = 0; i < p.n_small; ++i)
+        b += sizeof(double) * ((size_t)4 * p.s[i].G * C + p.s[i].G) + sizeof(FixDigits) * (size_t)four_rows(p.s[i].G) * C;
+    return b;
+}
+
+int launch_ap_star(const ApStar& p, cudaStream_t s) {
+    if (p.w.G <= 0 || p.n_small < 1 || p.w.C > 32) return set_error("projections in one launch: invalid sizes");
+    const size_t smem = ap_star_smem(p);
+    if (smem > AP_STAR_SMEM) return set_error("projections in one launch: %zu bytes of shared memory", smem);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(ap_star_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AP_STAR_SMEM);
+    if (attr != cudaSuccess) return set_cuda_error(attr, "projections attr");
+    int per_sm = 0;
+    FEGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ap_star_kernel, AP_THREADS, smem),
+              "projections occupancy");
+    if (per_sm < 1) return set_error("projections in one launch: no block fits");
+    // three steps of 256 / C groups a block while blocks are few (each more block
+    // makes the barriers dearer), else as many as are resident
+    const long long want = ((long long)p.w.G + 3 * (AP_THREADS / p.w.C) - 1) / (3 * (AP_THREADS / p.w.C));
+    const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(want, (long long)per_sm * num_sms()));
+    ApStar q = p;
+    void* args[] = {&q};
+    FEGB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(ap_star_kernel), dim3(blocks), dim3(AP_THREADS), args,
+                                          smem, s),
+              "projections in one launch");
+    FEGB_LAUNCH_CHECK("projections in one launch");
+    return 0;
+}
 
 int launch_ap_load(const double* inc, long long G, int C, int ld, double* tab, double* total,
                    unsigned long long* amax, cudaStream_t s) {

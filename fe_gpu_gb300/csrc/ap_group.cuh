@@ -130,6 +130,40 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s);
 // doubles of ApSmall::partials for a dimension of Gs groups with n_src sources
 size_t ap_small_scratch(int Gs, int C, int n_src);
 
+// All iterations of a problem with one large dimension and otherwise small ones
+// (at most DENSE_SMALL_MAX_G groups each) in one cooperative launch, FP64: a block
+// owns a range of the large dimension's groups and a copy of the small tables.
+// Everything between two visits of the large dimension then happens inside
+// every block alike; the blocks meet only for the largest updates of the large
+// dimension and for its sums over the small groups, six times an iteration.
+struct ApStar {
+    ApTables<double> w;          // the large dimension (amax: running column maxima, zeroed)
+    int n_small;
+    ApTables<double> s[SWEEP_MAXP];        // small dimensions in sweep order
+    ApDense<double> sw[SWEEP_MAXP];        // counts of small i against the large dimension (Ge = w.G)
+    ApDense<double> ss[SWEEP_MAXP][SWEEP_MAXP];  // counts of small i against small j (Ge = groups of j)
+    unsigned long long* sums;    // AP_STAR_RING x ap_star_sums() words, zeroed
+    unsigned long long* change;  // AP_STAR_RING words, zeroed: largest update of a projection of w
+    unsigned* arrived;           // zeroed: the barrier's count
+    int* error;                  // zeroed: a barrier ran out of time
+    ApCtl* ctl;                  // tol in; iterations, max_update, stop out
+    const double* relax;         // starting relaxation and last change of the small dimensions, then of w
+    const double* prev_change;
+    int relax_at[SWEEP_MAXP + 1];
+    int max_iter;
+};
+// Up to this many elements of the large dimension's table: the launches of an
+// iteration (eight or more, several us each) weigh less beyond, and one launch
+// keeps only two blocks an SM (whole fits, 4 columns, 6 rows a group: 20k groups
+// 4.05 -> 2.70 ms, 150k 5.79 -> 4.24, 400k 8.52 -> 7.29; 940k 15.0 -> 15.7).
+constexpr double AP_STAR_ELEMENTS = 2.0e6;
+constexpr int AP_STAR_RING = 4;
+// 64-bit words of one ring entry of ApStar::sums; shared memory the kernel needs
+size_t ap_star_sums(const ApStar& p);
+size_t ap_star_smem(const ApStar& p);
+constexpr size_t AP_STAR_SMEM = 96 * 1024;
+int launch_ap_star(const ApStar& p, cudaStream_t s);
+
 // The FP64 tables of an increment: tab (row stride ld) = inc, total += inc (G x C,
 // compact) and the columns' maxima of |inc| into amax (zeroed by the caller).
 int launch_ap_load(const double* inc, long long G, int C, int ld, double* tab, double* total,

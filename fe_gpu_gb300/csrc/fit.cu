@@ -2526,6 +2526,62 @@ struct ApGroups {
         return launch_ap_check(slots, P.n_fe, half, ctl, P.s);
     }
 
+    // The problem as one large dimension and small ones (ap_group.cuh, ApStar);
+    // false when it is not one or its small tables are too large. (Profiled fits
+    // take the launches one by one, to time them.)
+    bool star_of(const Problem& P, int max_iter, ApStar* star) const {
+        ApStar& a = *star;
+        std::memset(&a, 0, sizeof(a));
+        int large = -1;
+        for (int d : P.order) {
+            if (P.dims[d].G <= 0) return false;
+            if (B.dense[d]) {
+                a.relax_at[a.n_small] = d;
+                a.s[a.n_small++] = tables(P, d);
+            } else if (large < 0) {
+                large = d;
+            } else {
+                return false;
+            }
+        }
+        // the sweep order ends with the large dimension
+        if (large < 0 || a.n_small < 1 || P.order[P.n_fe - 1] != large) return false;
+        a.w = tables(P, large);
+        a.relax_at[a.n_small] = large;
+        for (int i = 0; i < a.n_small; ++i) {
+            a.sw[i] = matrix(P, P.order[i], large, large);
+            for (int j = 0; j < a.n_small; ++j)
+                if (j != i) a.ss[i][j] = matrix(P, P.order[i], P.order[j], P.order[j]);
+        }
+        a.relax = P.relax;
+        a.prev_change = P.prev_change;
+        a.ctl = ctl;
+        a.max_iter = max_iter;
+        return (double)a.w.G * P.C <= AP_STAR_ELEMENTS && ap_star_smem(a) <= AP_STAR_SMEM;
+    }
+
+    int run_star(Problem& P, ApStar& a, int* iterations, double* max_update) {
+        Scratch tmp(P.s);
+        const size_t words = ap_star_sums(a) * AP_STAR_RING + AP_STAR_RING + 1;
+        unsigned long long* w = nullptr;
+        FEGB_TRY(tmp.alloc(&w, words, "projection exchange"));
+        FEGB_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long) * words, P.s), "projection exchange zero");
+        a.change = w;
+        a.arrived = reinterpret_cast<unsigned*>(w + AP_STAR_RING);
+        a.error = reinterpret_cast<int*>(a.arrived + 1);
+        a.sums = w + AP_STAR_RING + 1;
+        FEGB_TRY(launch_ap_star(a, P.s));
+        ApCtl last{};
+        int bad = 0;
+        FEGB_CUDA(cudaMemcpyAsync(&last, ctl, sizeof(last), cudaMemcpyDeviceToHost, P.s), "projection state copy");
+        FEGB_TRY(d2h_sync(&bad, a.error, sizeof(bad), P.s, "projection error copy"));
+        if (bad) return set_error("alternating projections: a barrier of the one-launch form ran out of time");
+        *iterations = last.iterations;
+        *max_update = last.max_update;
+        P.projections += 4 * P.n_fe * last.iterations;
+        return 0;
+    }
+
     // Iterations from the means mu_all (of the current rows) until the largest
     // update stays below tol; the relaxation state continues from P.relax,
     // P.prev_change and the prev tables. Leaves the updates in alpha_all.
@@ -2543,6 +2599,13 @@ struct ApGroups {
                                   cudaMemcpyDeviceToDevice, P.s),
                   "coupling sums start");
         FEGB_TRY(launch_ap_reset(slots, P.relax, P.prev_change, P.n_fe, ctl, tol, P.s));
+        if constexpr (sizeof(T) == 8) {
+            ApStar star;
+            if (!P.profile && star_of(P, max_iter, &star)) {
+                FEGB_TRY(run_star(P, star, iterations, max_update));
+                return launch_to_f64<double>(reinterpret_cast<const double*>(B.p), B.ld, P.alpha_all, C, P.Gt, P.s);
+            }
+        }
         ApCtl last{};
         int queued = 0;
         const int proj0 = P.projections;

@@ -38,6 +38,10 @@ CASES = [
     (5000, (800, 64, 17), 31),           # 32 columns
     (5000, (800, 64, 17), 32),           # 33 columns: projections on the rows
     (60000, (12000, 3000, 11), 2),       # short groups and chunked groups
+    (3000, (200, 9), 2),                 # one large dimension and small ones: one launch, one block
+    (30000, (5000, 17, 64, 2), 8),       # the same over many blocks, pieces of 16 and their remainders
+    (700, (65, 33), 31),                 # 32 columns: one slot a warp
+    (3000000, (600000, 5), 3),           # more elements than the one-launch form takes
 ]
 
 
