@@ -347,10 +347,10 @@ __device__ __forceinline__ void column_partials(A prod, long long base, int C, A
 }
 
 // ---- row-tiled CG vector kernels ----
-// A block covers VEC_STEPS steps of rps = 256 / C rows of a G x C table
+// A block covers `steps` steps of rps = 256 / C rows of a G x C table
 // (C <= 256); thread t handles column c = t % C of rows g0 + t / C + rps * k,
 // so its column is fixed: products accumulate in one register per thread (in
-// T, VEC_STEPS terms at most) and each block writes one FP64 partial per
+// T, `steps` terms at most) and each block writes one FP64 partial per
 // column, folded in row order. 32-bit index arithmetic per thread.
 struct VecLane {
     int c;       // column
@@ -392,16 +392,16 @@ __device__ __forceinline__ void vec_block_max(double m, double* red8, double* ou
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) cg_q_rows_kernel(FinalizeParams src, int C, const T* __restrict__ p, int pld,
+__global__ void __launch_bounds__(256) cg_q_rows_kernel(FinalizeParams src, int steps, int C, const T* __restrict__ p, int pld,
                                                         T* __restrict__ q, double* __restrict__ pq_partials,
                                                         const T* __restrict__ extra) {
     __shared__ double red[256];
     const VecLane v = vec_lane(C);
     T prod = T(0);
     if (v.active) {
-        const long long g0 = (long long)blockIdx.x * v.rps * VEC_STEPS + v.rr;
+        const long long g0 = (long long)blockIdx.x * v.rps * steps + v.rr;
 #pragma unroll 4
-        for (int k = 0; k < VEC_STEPS; ++k) {
+        for (int k = 0; k < steps; ++k) {
             const long long gl = g0 + (long long)k * v.rps;
             if (gl >= src.G) break;
             const int g = (int)gl;
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) cg_q_rows_kernel(FinalizeParams src, int 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) cg_update_rows_kernel(long long Gt, int C, const T* __restrict__ inv_counts,
+__global__ void __launch_bounds__(256) cg_update_rows_kernel(long long Gt, int steps, int C, const T* __restrict__ inv_counts,
                                                              const double* __restrict__ rz,
                                                              const double* __restrict__ pq, const T* __restrict__ p,
                                                              int pld, const T* __restrict__ q, T* __restrict__ x,
@@ -435,9 +435,9 @@ __global__ void __launch_bounds__(256) cg_update_rows_kernel(long long Gt, int C
     if (v.active) {
         const double den = pq[v.c];
         const T a = (T)(den != 0.0 ? rz[v.c] / den : 0.0);
-        const long long g0 = (long long)blockIdx.x * v.rps * VEC_STEPS + v.rr;
+        const long long g0 = (long long)blockIdx.x * v.rps * steps + v.rr;
 #pragma unroll 4
-        for (int k = 0; k < VEC_STEPS; ++k) {
+        for (int k = 0; k < steps; ++k) {
             const long long g = g0 + (long long)k * v.rps;
             if (g >= Gt) break;
             const long long idx = g * C + v.c;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) cg_update_rows_kernel(long long Gt, int C
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) cg_init_rows_kernel(long long Gt, int C, const int32_t* __restrict__ counts,
+__global__ void __launch_bounds__(256) cg_init_rows_kernel(long long Gt, int steps, int C, const int32_t* __restrict__ counts,
                                                            const double* __restrict__ mu, T* __restrict__ r,
                                                            T* __restrict__ z, T* __restrict__ p, int pld,
                                                            T* __restrict__ x, double* __restrict__ rz_partials,
@@ -466,8 +466,8 @@ __global__ void __launch_bounds__(256) cg_init_rows_kernel(long long Gt, int C, 
     const VecLane v = vec_lane(C);
     T prod = T(0), az = T(0);
     if (v.active) {
-        const long long g0 = (long long)blockIdx.x * v.rps * VEC_STEPS + v.rr;
-        for (int k = 0; k < VEC_STEPS; ++k) {
+        const long long g0 = (long long)blockIdx.x * v.rps * steps + v.rr;
+        for (int k = 0; k < steps; ++k) {
             const long long g = g0 + (long long)k * v.rps;
             if (g >= Gt) break;
             const long long idx = g * C + v.c;
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256) cg_init_rows_kernel(long long Gt, int C, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) cg_init_rhs_rows_kernel(long long Gt, int C, const int32_t* __restrict__ counts,
+__global__ void __launch_bounds__(256) cg_init_rhs_rows_kernel(long long Gt, int steps, int C, const int32_t* __restrict__ counts,
                                                                const double* __restrict__ mu, const T* __restrict__ qb,
                                                                const T* __restrict__ inv, T* __restrict__ r,
                                                                T* __restrict__ z, T* __restrict__ p, int pld,
@@ -499,8 +499,8 @@ __global__ void __launch_bounds__(256) cg_init_rhs_rows_kernel(long long Gt, int
     const VecLane v = vec_lane(C);
     T prod = T(0), az = T(0);
     if (v.active) {
-        const long long g0 = (long long)blockIdx.x * v.rps * VEC_STEPS + v.rr;
-        for (int k = 0; k < VEC_STEPS; ++k) {
+        const long long g0 = (long long)blockIdx.x * v.rps * steps + v.rr;
+        for (int k = 0; k < steps; ++k) {
             const long long g = g0 + (long long)k * v.rps;
             if (g >= Gt) break;
             const long long idx = g * C + v.c;
@@ -890,9 +890,17 @@ int launch_convert_f64_f32(const double* src, float* dst, long long n, cudaStrea
 }
 
 
+int cg_vec_steps(long long G, int C) {
+    constexpr long long FILL = 304;  // blocks that fill the chip (a constant: the same sums on any GPU)
+    const long long rps = std::max(1, 256 / C);
+    int steps = 16;
+    while (steps > 1 && G < FILL * rps * steps) steps /= 4;
+    return steps;
+}
+
 int cg_partial_blocks(long long G, int C) {
     if (C <= 256) {
-        const long long rows = (long long)(256 / C) * VEC_STEPS;
+        const long long rows = (long long)(256 / C) * cg_vec_steps(G, C);
         return (int)((G + rows - 1) / rows);
     }
     return (int)((G * C + FIN_THREADS - 1) / FIN_THREADS);
@@ -905,7 +913,7 @@ int launch_cg_q(const FinalizeParams& src, int C, const T* p, int pld, T* q, dou
     if (total <= 0) return 0;
     const int nb = cg_partial_blocks(src.G, C);
     if (C <= 256)
-        cg_q_rows_kernel<T><<<nb, 256, 0, s>>>(src, C, p, pld, q, pq_partials, extra);
+        cg_q_rows_kernel<T><<<nb, 256, 0, s>>>(src, cg_vec_steps(src.G, C), C, p, pld, q, pq_partials, extra);
     else
         cg_q_kernel<T><<<nb, FIN_THREADS, 0, s>>>(src, C, p, pld, q, pq_partials, extra);
     FEGB_LAUNCH_CHECK("cg q");
@@ -1004,7 +1012,7 @@ int launch_cg_update(long long Gt, int C, const T* inv_counts, const double* rz,
     if (total <= 0) return 0;
     const int nb = cg_partial_blocks(Gt, C);
     if (C <= 256)
-        cg_update_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, C, inv_counts, rz, pq, p, pld, q, x, r, z, rz_partials,
+        cg_update_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, inv_counts, rz, pq, p, pld, q, x, r, z, rz_partials,
                                                     zmax_partials);
     else
         cg_update_kernel<T><<<nb, FIN_THREADS, 0, s>>>(Gt, C, inv_counts, rz, pq, p, pld, q, x, r, z, rz_partials,
@@ -1036,7 +1044,7 @@ int launch_cg_init(long long Gt, int C, const int32_t* counts, const double* mu,
     if (total <= 0) return 0;
     const int nb = cg_partial_blocks(Gt, C);
     if (C <= 256)
-        cg_init_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, C, counts, mu, r, z, p, pld, x, rz_partials, zmax_partials);
+        cg_init_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, counts, mu, r, z, p, pld, x, rz_partials, zmax_partials);
     else
         cg_init_kernel<T><<<nb, FIN_THREADS, 0, s>>>(Gt, C, counts, mu, r, z, p, pld, x, rz_partials,
                                                      zmax_partials);
@@ -1053,7 +1061,7 @@ int launch_cg_init_rhs(long long Gt, int C, const int32_t* counts, const double*
     if (Gt * C <= 0) return 0;
     if (C > 256) return set_error("cg: %d columns exceed the right-hand-side initialisation", C);
     const int nb = cg_partial_blocks(Gt, C);
-    cg_init_rhs_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, C, counts, mu, qb, inv, r, z, p, pld, x, rz_partials,
+    cg_init_rhs_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, counts, mu, qb, inv, r, z, p, pld, x, rz_partials,
                                                   zmax_partials);
     FEGB_LAUNCH_CHECK("cg init (rhs)");
     fold_max_kernel<<<1, FIN_THREADS, 0, s>>>(zmax_partials, nb, zmax);
@@ -1263,7 +1271,6 @@ __global__ void __launch_bounds__(256) dense_pair_kernel(const CT* __restrict__ 
     const size_t m_bytes = ((sizeof(CT) * (size_t)DENSE_TILE * Gs + 15) / 16) * 16;
     unsigned char* const buf0 = dense_smem + s_bytes + u_bytes;
     unsigned char* const buf1 = buf0 + p_bytes + m_bytes;
-    double* red = reinterpret_cast<double*>(dense_smem);  // Gs x C (after the tiles)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (extra || sch.sums)
         for (int i = threadIdx.x; i < Gs * CQ; i += 256) {
@@ -1342,22 +1349,28 @@ __global__ void __launch_bounds__(256) dense_pair_kernel(const CT* __restrict__ 
         }
         __syncthreads();  // this buffer is refilled two tiles on
     }
-    // fold the warps' small-side sums in warp order (FP64); red overlays sS
+    // fold the warps' small-side sums in warp order (FP64): every warp leaves its
+    // sums in shared memory (over the tiles), then a thread per sum adds the eight
+    // (warp after warp into one FP64 table, eight barriers, was half of a launch
+    // of 74 blocks with 30 columns: 22 us, 5.5 now)
+    if (!small_side) return;
     __syncthreads();
-    for (int w = 0; w < DENSE_WARPS; ++w) {
-        if (warp == w) {
+    T* const wsum = reinterpret_cast<T*>(dense_smem);  // DENSE_WARPS x Gs x C
+    const int GC = Gs * C;
 #pragma unroll
-            for (int c = 0; c < CQ; ++c) {
-                if (c >= C) break;
-                if (lane < Gs) red[lane * C + c] = (w ? red[lane * C + c] : 0.0) + (double)acc0[c];
-                if constexpr (TWO)
-                    if (lane + 32 < Gs) red[(lane + 32) * C + c] = (w ? red[(lane + 32) * C + c] : 0.0) + (double)acc1[c];
-            }
-        }
-        __syncthreads();
+    for (int c = 0; c < CQ; ++c) {
+        if (c >= C) break;
+        if (lane < Gs) wsum[warp * GC + lane * C + c] = acc0[c];
+        if constexpr (TWO)
+            if (lane + 32 < Gs) wsum[warp * GC + (lane + 32) * C + c] = acc1[c];
     }
-    if (small_side)
-        for (int i = threadIdx.x; i < Gs * C; i += 256) partials[(long long)blockIdx.x * Gs * C + i] = red[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < GC; i += 256) {
+        double v = (double)wsum[i];
+#pragma unroll
+        for (int w = 1; w < DENSE_WARPS; ++w) v += (double)wsum[w * GC + i];
+        partials[(long long)blockIdx.x * GC + i] = v;
+    }
 }
 
 template <typename T, typename CT, int CQ, bool TWO>
@@ -1372,7 +1385,7 @@ int dense_pair_cq(const CT* M, long long Ge, int Gs, const T* pe, const T* ps, i
     const size_t p_bytes = dense_slot_bytes<T>(ld, C);
     const size_t m_bytes = ((sizeof(CT) * (size_t)DENSE_TILE * Gs + 15) / 16) * 16;
     const size_t smem = std::max(sizeof(T) * (size_t)(DENSE_SMALL_MAX_G + DENSE_TILE) * CQ + 2 * (p_bytes + m_bytes),
-                                 sizeof(double) * (size_t)Gs * C);
+                                 sizeof(T) * (size_t)DENSE_WARPS * Gs * C);
     dense_pair_kernel<T, CT, CQ, TWO><<<nb, 256, smem, s>>>(M, Ge, Gs, pe, ps, ld, C, per, partials, extra,
                                                             accumulate, sch);
     FEGB_LAUNCH_CHECK("dense small-G pair product");

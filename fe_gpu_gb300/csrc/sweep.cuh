@@ -324,9 +324,12 @@ int launch_inv_diag(const unsigned long long* acc, const int32_t* counts, long l
 // sums[t * C + c] = -(sum over parts of partials[part][t][c]), parts in order
 int launch_fold_dense(const double* partials, int nparts, int Gs, int C, double* sums, cudaStream_t s);
 // Partial blocks (one FP64 partial per column each) of the CG vector kernels
-// over a G x C table: VEC_STEPS steps of 256 / C rows per block (C <= 256),
-// else one block per 256 elements.
-constexpr int VEC_STEPS = 16;
+// over a G x C table: cg_vec_steps(G, C) steps of 256 / C rows per block
+// (C <= 256), else one block per 256 elements. Sixteen steps a block for large
+// tables; fewer where that would leave most of the chip idle and each block a
+// chain of sixteen dependent loads (2,000 groups, 5 columns: update 14 -> 6
+// us a launch, q 7.5 -> 4.3).
+int cg_vec_steps(long long G, int C);
 int cg_partial_blocks(long long G, int C);
 
 // out[c] = sum_b partials[b * C + c] for b < nb (fixed order)
