@@ -167,6 +167,19 @@ __device__ __forceinline__ void ap_open_slot(ApSlot* slots, int slot, double rel
     slots[(slot + 1) % AP_SLOTS].change = 0ULL;
 }
 
+// The relaxation for a whole block, by one thread (the rule is eight FP64
+// instructions, 128 cycles of an SM's FP64 pipe a warp), recorded by the first.
+__device__ __forceinline__ double ap_block_relax(ApSlot* slots, int slot) {
+    __shared__ double s_relax;
+    if (threadIdx.x == 0) {
+        const double r = ap_relax(slots, slot);
+        s_relax = r;
+        if (blockIdx.x == 0) ap_open_slot(slots, slot, r);
+    }
+    __syncthreads();
+    return s_relax;
+}
+
 // sum over t of N[g][t] * tab[t][c], small source, FP64/FP32 arithmetic
 template <typename T, typename CT>
 __device__ __forceinline__ T dense_dot(const CT* __restrict__ N, int Gs, const T* __restrict__ tab, int C, int c) {
@@ -182,30 +195,23 @@ __device__ __forceinline__ T dense_dot(const CT* __restrict__ N, int Gs, const T
     for (; t < Gs; ++t) a = fma((T)N[t], tab[t * C + c], a);
     return a;
 }
-// the 16 counts of piece w of a row, in order
-struct Counts16 {
-    unsigned n[AP_PART];
-};
-__device__ __forceinline__ Counts16 load_counts(const uint8_t* row, int w) {
-    const uint4 x = reinterpret_cast<const uint4*>(row)[w];
-    const unsigned q[4] = {x.x, x.y, x.z, x.w};
-    Counts16 r;
+// piece w (16 counts) of a row: the loads, and the counts in order
+template <typename CT>
+struct Piece {
+    uint4 x[AP_PART * sizeof(CT) / 16];
+    __device__ __forceinline__ void load(const CT* row, int w) {
+        constexpr int V = AP_PART * sizeof(CT) / 16;
 #pragma unroll
-    for (int i = 0; i < AP_PART; ++i) r.n[i] = (q[i / 4] >> (8 * (i % 4))) & 255u;
-    return r;
-}
-__device__ __forceinline__ Counts16 load_counts(const uint32_t* row, int w) {
-    Counts16 r;
-#pragma unroll
-    for (int i = 0; i < AP_PART / 4; ++i) {
-        const uint4 x = reinterpret_cast<const uint4*>(row)[w * (AP_PART / 4) + i];
-        r.n[4 * i] = x.x;
-        r.n[4 * i + 1] = x.y;
-        r.n[4 * i + 2] = x.z;
-        r.n[4 * i + 3] = x.w;
+        for (int i = 0; i < V; ++i) x[i] = reinterpret_cast<const uint4*>(row)[w * V + i];
     }
-    return r;
-}
+    __device__ __forceinline__ unsigned operator[](int i) const {
+        constexpr int PER = 16 / sizeof(CT), SUB = 4 / sizeof(CT);  // counts per vector, per word
+        const uint4 v = x[i / PER];
+        const int k = i % PER / SUB;
+        const unsigned q = k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
+        return sizeof(CT) == 4 ? q : (q >> (8 * (i % SUB))) & 255u;
+    }
+};
 
 // the same in fixed point; tab is zero past Gs, up to a multiple of four rows
 template <typename CT>
@@ -213,15 +219,16 @@ __device__ __forceinline__ void dense_dot_fixed(const void* N, long long g, int 
                                                 int C, int c, FixSum& a) {
     const CT* row = static_cast<const CT*>(N) + g * ap_count_pitch(Gs);
     for (int t0 = 0; t0 < Gs; t0 += AP_PART) {
-        const Counts16 n = load_counts(row, t0 / AP_PART);
+        Piece<CT> n;
+        n.load(row, t0 / AP_PART);
 #pragma unroll
         for (int i = 0; i < AP_PART; i += 4) {
             if (t0 + i >= Gs) break;
             const FixDigits* __restrict__ q = tab + (t0 + i) * C + c;
-            fix_add(a, n.n[i], q[0]);
-            fix_add(a, n.n[i + 1], q[C]);
-            fix_add(a, n.n[i + 2], q[2 * C]);
-            fix_add(a, n.n[i + 3], q[3 * C]);
+            fix_add(a, n[i], q[0]);
+            fix_add(a, n[i + 1], q[C]);
+            fix_add(a, n[i + 2], q[2 * C]);
+            fix_add(a, n[i + 3], q[3 * C]);
         }
     }
 }
@@ -273,9 +280,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_visit_kernel(ApVisit<T> p) {
             dst += four_rows(D.Gs) * C;
         }
     }
-    const double relax = ap_relax(t.slots, p.slot);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ap_open_slot(t.slots, p.slot, relax);
-    __syncthreads();
+    const double relax = ap_block_relax(t.slots, p.slot);
     unsigned long long upd = 0, av = 0;
     if (active)
         for (long long g = (long long)blockIdx.x * rps + rr; g < t.G; g += (long long)gridDim.x * rps) {
@@ -358,8 +363,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_repeat_kernel(ApTables<T> t, in
     const int rr = (int)threadIdx.x / C;
     const int c = (int)threadIdx.x - rr * C;
     const bool active = rr < rps;
-    const double relax = ap_relax(t.slots, slot);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ap_open_slot(t.slots, slot, relax);
+    const double relax = ap_block_relax(t.slots, slot);
     unsigned long long upd = 0, av = 0;
     if (active)
         for (long long g = (long long)blockIdx.x * rps + rr; g < t.G; g += (long long)gridDim.x * rps) {
@@ -376,7 +380,7 @@ __global__ void __launch_bounds__(AP_THREADS) ap_repeat_kernel(ApTables<T> t, in
 // folded by one block, hence their lower limit.
 constexpr int AP_DEPTH = 4;
 constexpr int AP_PART_BLOCKS = 152;
-constexpr int AP_FIX_BLOCKS = 304;
+constexpr int AP_FIX_BLOCKS = 304;       // two an SM; one (half of them) where the sums of 24 groups fill the registers
 
 // A block takes all groups of a small dimension of up to AP_WHOLE groups (what the
 // registers hold), else one part of AP_PART of them.
@@ -399,35 +403,39 @@ __device__ __forceinline__ V warp_slot_sum(V v, int slot, int slots, int C, int 
 }
 
 // acc[t] += N[g][t] * tab[g][c] over this lane's groups, t from piece w of the rows
-// on. WRITTEN: the table was written by this launch (read past L1).
-template <typename CT, int GT, bool WRITTEN = false>
-__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const double* tab, int ld, int c,
-                                           int k, long long g, long long Ge, long long gstep, FixSum (&acc)[GT]) {
-#pragma unroll 2
-    for (; g < Ge; g += gstep) {
-        const double* at = tab + g * ld + c;
-        const FixDigits a = fix_digits(to_fixed(WRITTEN ? __ldcg(at) : *at, k));
+// on; the next group's loads are in flight while one is added (8 to 16 warps an
+// SM hide little by themselves). WRITTEN: the table was written by this launch
+// (read past L1).
+__device__ __forceinline__ void walk_add(FixSum& s, unsigned n, const FixDigits& a) { fix_add(s, n, a); }
+__device__ __forceinline__ void walk_add(float& s, unsigned n, float a) { s = fmaf((float)n, a, s); }
+__device__ __forceinline__ FixDigits walk_value(double v, int k, const FixSum*) { return fix_digits(to_fixed(v, k)); }
+__device__ __forceinline__ float walk_value(float v, int, const float*) { return v; }
+
+template <typename CT, int GT, bool WRITTEN = false, typename T, typename A>
+__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const T* tab, int ld, int c, int k,
+                                           long long g, long long Ge, long long gstep, A (&acc)[GT]) {
+    constexpr int NP = (GT + AP_PART - 1) / AP_PART;
+    if (g >= Ge) return;
+    Piece<CT> next[NP];
+    T next_v = WRITTEN ? __ldcg(tab + g * ld + c) : tab[g * ld + c];
 #pragma unroll
-        for (int q = 0; q < GT; q += AP_PART) {
-            const Counts16 n = load_counts(N + g * pitch, w + q / AP_PART);
+    for (int q = 0; q < NP; ++q) next[q].load(N + g * pitch, w + q);
+#pragma unroll 1
+    while (true) {
+        const auto a = walk_value(next_v, k, static_cast<const A*>(nullptr));
+        Piece<CT> n[NP];
 #pragma unroll
-            for (int i = 0; i < AP_PART && q + i < GT; ++i) fix_add(acc[q + i], n.n[i], a);
+        for (int q = 0; q < NP; ++q) n[q] = next[q];
+        g += gstep;
+        const bool more = g < Ge;
+        if (more) {
+            next_v = WRITTEN ? __ldcg(tab + g * ld + c) : tab[g * ld + c];
+#pragma unroll
+            for (int q = 0; q < NP; ++q) next[q].load(N + g * pitch, w + q);
         }
-    }
-}
-template <typename CT, int GT>
-__device__ __forceinline__ void small_walk(const CT* __restrict__ N, int pitch, int w, const float* __restrict__ tab,
-                                           int ld, int c, int, long long g, long long Ge, long long gstep,
-                                           float (&acc)[GT]) {
-#pragma unroll 2
-    for (; g < Ge; g += gstep) {
-        const float a = tab[g * ld + c];
 #pragma unroll
-        for (int q = 0; q < GT; q += AP_PART) {
-            const Counts16 n = load_counts(N + g * pitch, w + q / AP_PART);
-#pragma unroll
-            for (int i = 0; i < AP_PART && q + i < GT; ++i) acc[q + i] = fmaf((float)n.n[i], a, acc[q + i]);
-        }
+        for (int i = 0; i < GT; ++i) walk_add(acc[i], n[i / AP_PART][i % AP_PART], a);
+        if (!more) break;
     }
 }
 template <int GT, typename T, typename A>
@@ -450,7 +458,7 @@ __device__ __forceinline__ void small_walk_any(const ApDense<T>& D, int w, int l
 // free); FP32 sums leave one FP64 partial per block, folded in block order.
 // The last block to finish turns the sums into the projections.
 // 100k x 20 and 12k x 20 counts, 12 columns: 81 us with FP64 sums of both
-// operands in shared memory, 41 us in this form; 940k x 13, 4 columns: 75 -> 44.
+// operands in shared memory, 41 us in this form; 940k x 13, 4 columns: 75 -> 26.
 template <typename T, int GT>
 __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > AP_PART ? 1 : 2) ap_small_kernel(ApSmall<T> p, ApSmallGrid gr) {
     if (p.ctl->stop) return;
@@ -1112,7 +1120,8 @@ int launch_ap_small(const ApSmall<T>& p, cudaStream_t s) {
     const long long per_block = (long long)(AP_THREADS / 32) * (32 / C) * AP_DEPTH;
     for (int e = 0; e < p.n_src; ++e) {
         const long long want = (p.src[e].Ge + per_block - 1) / per_block;
-        const int nb = (int)std::max(1LL, std::min<long long>(want, sizeof(T) == 8 ? AP_FIX_BLOCKS : AP_PART_BLOCKS));
+        const int limit = sizeof(T) == 4 ? AP_PART_BLOCKS : gr.parts == 1 && Gs > AP_PART ? AP_FIX_BLOCKS / 2 : AP_FIX_BLOCKS;
+        const int nb = (int)std::max(1LL, std::min<long long>(want, limit));
         for (int h = 0; h < gr.parts; ++h) gr.first[e * gr.parts + h + 1] = gr.first[e * gr.parts + h] + nb;
     }
     if (Gs <= 4) return launch_ap_small_gt<T, 4>(p, gr, smem, s);
