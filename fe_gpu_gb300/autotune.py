@@ -3,7 +3,7 @@
 The knobs select, for a problem shape, between equivalent forms of the hot
 kernels: the count-matrix pass on the tensor cores or the CUDA cores, the
 number of table columns one CG operator sweep carries per pass (4, 8 or all),
-the output size from which Gram products use the split-FP32 form, whether
+the output size from which Gram products use the tensor-core form, whether
 the CG loop runs as a CUDA graph, and whether operator sweeps of streams with
 short groups run one thread per group. None changes the result beyond rounding.
 

@@ -104,7 +104,7 @@ void configure_mem_pool();
 //   TUNE_CG_COLS_PER_PASS 0 all columns of a row in one pass of the operator
 //                         sweep, else at most 4 or 8 (more passes, fewer registers)
 //   TUNE_SPLIT_GRAM       output pairs per input column from which Gram
-//                         products use the split-FP32 form (>= 1)
+//                         products use the tensor-core form (>= 1)
 //   TUNE_CG_GRAPH         1 the CG loop runs as a CUDA graph, 0 host-driven
 //   TUNE_BATCH_ESTIMATOR  1 batched specifications are estimated class by
 //                         class in one batched pass, 0 one by one

@@ -58,6 +58,7 @@
 // memory and returns.
 #include "common.cuh"
 #include "sweep.cuh"
+#include "umma.cuh"
 
 #include <cuda_bf16.h>
 
@@ -73,7 +74,6 @@ constexpr int UCP = 16;        // columns per piece block (C <= 16)
 constexpr int UNP = 3;         // BF16 pieces per FP32 value
 constexpr int UN1 = UNP * UCP; // N of the e-side product
 constexpr int UM2 = 64;        // M of the small-side product (rows p * 16 + c; 48 used)
-constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;  // 2 s per wait
 
 // Tensor-memory columns: two E buffers (tile i in buffer i & 1) and the D2
 // accumulator; 128 columns when the small dimension has at most 32 groups.
@@ -86,100 +86,6 @@ struct TmemPlan {
 };
 
 __device__ int g_umma_error;  // nonzero: a wait of the tensor-core pass ran out of time
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned long long globaltimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// tcgen05 shared-memory matrix descriptor, no swizzle: start address, LBO and
-// SBO in 16-byte units, fixed version bits 0b001 at 46-48.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-           (1ull << 46);
-}
-
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, the
-// majorness of each operand (0 = K-major, 1 = MN-major), N >> 3 and M >> 4.
-__host__ __device__ constexpr uint32_t umma_idesc(int M, int N, int a_mn, int b_mn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, int acc) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// true once the phase of the given parity has completed, false after the time
-// limit. Each try suspends the thread in hardware (up to the hint, or until
-// the phase completes), so waiting warps take no issue slots from the warps
-// that work.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = smem_u32(bar);
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.b32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(parity), "r"(1000000u)
-        : "memory");
-    if (ok) return true;
-    const unsigned long long t0 = globaltimer();
-    while (true) {
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(a), "r"(parity), "r"(1000000u)
-            : "memory");
-        if (ok) return true;
-        if (globaltimer() - t0 > WAIT_LIMIT_NS) return false;
-    }
-}
-
-// bulk global -> shared copy completing on bar (16-byte aligned, size a multiple of 16)
-__device__ __forceinline__ void bulk_copy(void* sdst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(sdst)),
-                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-template <int N>
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[N], int base) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v[base + j] = __uint_as_float(r[j]);
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // v = h + m + l with BF16 pieces (exact for finite FP32 v)
 __device__ __forceinline__ void split3(float v, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
@@ -254,18 +160,6 @@ __host__ __device__ inline UmmaSmem umma_smem_plan(int KT, uint32_t raw_bytes, u
 // exact float of the byte b of a 32-bit word (2^23 + b as an FP32 bit pattern, minus 2^23)
 __device__ __forceinline__ float byte_f32(uint32_t w, uint32_t sel) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)) - 8388608.0f;
-}
-
-template <int N>
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[N], int base) {
-    uint32_t r0, r1, r2, r3;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(taddr));
-    v[base] = __uint_as_float(r0);
-    v[base + 1] = __uint_as_float(r1);
-    v[base + 2] = __uint_as_float(r2);
-    v[base + 3] = __uint_as_float(r3);
 }
 
 // Persistent pass: CTA b covers groups [b per, (b + 1) per) tile by tile.
@@ -427,7 +321,7 @@ __global__ void __launch_bounds__(BT, 4) dense_umma_kernel(UmmaArgs a) {
         const uint32_t ecol = (j & 1) ? TP::E1 : TP::E0;
 #pragma unroll
         for (int s = 0; s < KT / 16; ++s)
-            umma_bf16(tmem + ecol, umma_desc(sbase + cnt_off + s * 256, 128, CORE_ROW),
+            umma_f16(tmem + ecol, umma_desc(sbase + cnt_off + s * 256, 128, CORE_ROW),
                       umma_desc(sbase + L.b1 + s * 256, 128, CORE_ROW), id, s > 0);
         ++s_arm[4 + (j & 1)];
         umma_commit(&bars[4 + (j & 1)]);
@@ -582,7 +476,7 @@ __global__ void __launch_bounds__(BT, 4) dense_umma_kernel(UmmaArgs a) {
                 const uint32_t cnt_off = (i & 1) ? L.cnt1 : L.cnt0;
 #pragma unroll
                 for (int s = 0; s < UT / 16; ++s)
-                    umma_bf16(tmem + TP::D2, umma_desc(sbase + L.u + s * 2 * U_LBO, U_LBO, 128),
+                    umma_f16(tmem + TP::D2, umma_desc(sbase + L.u + s * 2 * U_LBO, U_LBO, 128),
                               umma_desc(sbase + cnt_off + s * 2 * CORE_ROW, CORE_ROW, 128), id,
                               (i > 0 || s > 0) ? 1 : 0);
                 ++s_arm[6];

@@ -23,19 +23,23 @@ struct MatView {
 int crossprod(const MatView& A, const MatView& B, long long n, bool gram, bool upper_only, double alpha, double beta,
               double* out, int ldo, cudaStream_t s, Scratch& scr);
 
-// Same result through the FP32 pipe: every FP64 value is split into an FP32
-// pair (hi + lo, 48 significant bits), products are formed error-free
-// (TwoProd by FMA plus the cross terms), summed with TwoSum into an FP32 pair
-// per output and folded into FP64 every tile of rows. Relative error per term
-// about 2^-47, against 2^-53 for FP64 products; GB300 issues FP32 at about 60x
-// its FP64 rate, so cross products whose FP64 form is bound by the FP64 pipe
-// (outputs at least "split_gram_pairs_per_col" times the input columns; the
-// knob's default is CROSSPROD_SPLIT_PAIRS_PER_COL)
-// run several times faster. The FP64 values are split while a tile is loaded;
-// a value beyond the split range sends the whole product to the FP64 path.
+// The Gram A^T A (row-major A) on the tensor cores: every FP64 value is split
+// into eight whole-number digits whose products are summed exactly
+// (gram_umma.cu), so the result carries FP64 rounding only. Taken where the FP64
+// form would be bound by the FP64 pipe (outputs at least
+// "split_gram_pairs_per_col" times the input columns; the knob's default is
+// CROSSPROD_SPLIT_PAIRS_PER_COL). A value that is not finite sends the whole
+// product to the FP64 path; so do more than CROSSPROD_SPLIT_MAX_COLS columns.
 constexpr long long CROSSPROD_SPLIT_PAIRS_PER_COL = 3;
-int crossprod_split(const MatView& A, const MatView& B, long long n, bool gram, bool upper_only, double alpha,
-                    double beta, double* out, int ldo, cudaStream_t s, Scratch& scr);
+constexpr int CROSSPROD_SPLIT_MAX_COLS = 1600;
+int crossprod_split(const MatView& A, long long n, bool upper_only, double alpha, double beta, double* out, int ldo,
+                    cudaStream_t s, Scratch& scr);
+// The tensor-core Gram (gram_umma.cu): launches the pass over the row-major X
+// (n x C, row stride rs) and gives its per-block partials (nb x C (C + 1) / 2,
+// FP64, allocated from scr); bad |= 1 when a value is not finite, |= 2 when a
+// wait ran out of time.
+int launch_gram_umma(const double* X, long long rs, int C, long long n, Scratch& scr, double** partials, int* nb,
+                     int* bad, cudaStream_t s);
 // crossprod_split when the output is large enough, else crossprod.
 int crossprod_auto(const MatView& A, const MatView& B, long long n, bool gram, bool upper_only, double alpha,
                    double beta, double* out, int ldo, cudaStream_t s, Scratch& scr);

@@ -903,7 +903,7 @@ int fegb_test_gram(const double* X, long long n, int a, int split, double* out) 
     FEGB_CUDA(cudaMemcpy(dX, X, sizeof(double) * n * a, cudaMemcpyHostToDevice), "test data copy");
     MatView A{dX, (long long)a, 1, a};
     if (split)
-        FEGB_TRY(crossprod_split(A, A, n, true, false, 1.0, 0.0, dout, a, kLegacy, scr));
+        FEGB_TRY(crossprod_split(A, n, false, 1.0, 0.0, dout, a, kLegacy, scr));
     else
         FEGB_TRY(crossprod(A, A, n, true, false, 1.0, 0.0, dout, a, kLegacy, scr));
     FEGB_CUDA(cudaMemcpy(out, dout, sizeof(double) * a * a, cudaMemcpyDeviceToHost), "test gram copy");

@@ -151,7 +151,7 @@ long long fegb_kernel_launches(void);
  *   "cg_cols_per_pass"          0: all columns of a table row in one pass of
  *                               the CG operator sweep; 4 or 8: at most that many
  *   "split_gram_pairs_per_col"  Gram products with at least this many output
- *                               pairs per input column use the split-FP32 form
+ *                               pairs per input column use the tensor-core form
  *   "cg_graph"                  1: the CG loop runs as a CUDA graph; 0: host loop
  *   "batch_estimator"           1: fegb_estimate_batch estimates each column
  *                               class in one batched pass; 0: spec by spec
@@ -200,9 +200,8 @@ int fegb_test_group_sums(const double* X, long long n, int C, const int* gid, in
 
 /* Self-test of the Gram products behind the normal equations and the
  * single-row cluster meats, on host arrays: X is n x a row-major; out (a x a,
- * column-major, both triangles) = X'X. split = 1: the split-FP32
- * (double-single) forms (rows kernel up to 10 columns, register-blocked
- * kernel above); 0: the FP64 form. */
+ * column-major, both triangles) = X'X. split = 1: the tensor-core
+ * form (FP64 values as eight digits, exact digit products); 0: the FP64 form. */
 int fegb_test_gram(const double* X, long long n, int a, int split, double* out);
 
 /* FE reconstruction of --save-fe (reconstruct_and_save_fixed_effects,
