@@ -61,7 +61,11 @@ inline void trace_phase(cudaStream_t s, Clock::time_point t0, const char* what) 
 }
 
 constexpr int MODE_SMALLG = 2;
-constexpr int CHUNK_R = 256;
+// Positions a chunk of the row sweeps has. One chunk is one thread's serial walk
+// a column (256 positions: 41 us, 64: 12, at 38k x 30), so rows whose chunks
+// do not fill the chip take short ones; with the chip full the longer ones leave
+// fewer edges to put together. 20M elements are 2,400 warps of 256-position chunks.
+inline int chunk_rows(long long n, int C) { return n * C < 20000000LL ? 64 : 256; }
 constexpr int MAX_CLUSTER_DIMS = 3;  // src/core/fe_pipeline.f90:20
 
 struct Dim {
@@ -115,6 +119,7 @@ struct Problem {
     double* alpha_all = nullptr;
     double* mu_all = nullptr;
     int smallg_nb = 0;
+    int chunk = 256;  // positions a chunk of the row sweeps (chunk_rows)
     // the CG operator's row sort by distinct id tuples of its swept dimensions
     // (positions grouped by tuple), kept for the cluster subset over the same
     // dimensions: tuple t holds sorted positions tuple_off[t] .. tuple_off[t+1]
@@ -588,7 +593,7 @@ int order_deferred_rows(Problem& P) {
         FEGB_TRY(dalloc(*P.scr, &D.off, (size_t)D.G + 1, "offsets"));
         FEGB_TRY(segment_offsets(reinterpret_cast<const uint32_t*>(D.gseq), P.n, D.G, D.off, P.s));
         FEGB_TRY(dalloc(*P.scr, &D.long_list, (size_t)D.G, "long groups"));
-        FEGB_TRY(find_long_groups(D.off, D.G, CHUNK_R, D.long_list, &D.n_long, P.s));
+        FEGB_TRY(find_long_groups(D.off, D.G, P.chunk, D.long_list, &D.n_long, P.s));
         for (int e = 0; e < P.n_fe; ++e) {
             if (e == d) continue;
             FEGB_TRY(dalloc(*P.scr, &D.gid_at_perm[e], (size_t)P.n, "gid at perm"));
@@ -656,6 +661,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
         }
     }
     P.n = n;
+    P.chunk = chunk_rows(n, P.C);
     const int C = P.C;
     // primary dimension: the one with most groups (first on ties)
     P.primary = -1;
@@ -769,7 +775,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
                 counts_from_offsets_kernel<<<(D.G + 255) / 256, 256, 0, s>>>(D.off, D.G, D.counts);
                 FEGB_LAUNCH_CHECK("counts");
                 FEGB_TRY(dalloc(scr, &D.long_list, (size_t)D.G, "long groups"));
-                FEGB_TRY(find_long_groups(D.off, D.G, CHUNK_R, D.long_list, &D.n_long, s));
+                FEGB_TRY(find_long_groups(D.off, D.G, P.chunk, D.long_list, &D.n_long, s));
                 if (sorted_all && (cg_sorted[d] || d == P.primary)) {  // the dimensions the CG operator sweeps
                     FEGB_TRY(dalloc(scr, &D.long_list_cg, (size_t)D.G, "long groups (cg)"));
                     FEGB_TRY(find_long_groups(D.off, D.G, CG_CHUNK, D.long_list_cg, &D.n_long_cg, s));
@@ -808,7 +814,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
             FEGB_LAUNCH_CHECK("gid at perm");
         }
     }
-    long long nchunks = std::max(1LL, seg_nchunks(n, CHUNK_R));
+    long long nchunks = std::max(1LL, seg_nchunks(n, P.chunk));
     FEGB_TRY(dalloc(scr, &P.sums, (size_t)gmax * C, "group sums"));
     FEGB_TRY(dalloc(scr, &P.head, (size_t)nchunks * C, "chunk heads"));
     FEGB_TRY(dalloc(scr, &P.tail, (size_t)nchunks * C, "chunk tails"));
@@ -965,12 +971,12 @@ int sweep_sums_impl(Problem& P, int d, T* data, const PendingSet<T>& ps, bool wr
     sp.gseq = D.gseq;
     sp.pend = ps;
     sp.writeback = (writeback && D.mode == MODE_CONTIG) ? 1 : 0;
-    sp.R = CHUNK_R;
+    sp.R = P.chunk;
     sp.sums = P.sums;
     sp.head = P.head;
     sp.tail = P.tail;
     FEGB_TRY(launch_seg_sweep<T>(sp, P.s));
-    return launch_long_sums(D.off, P.head, P.tail, CHUNK_R, P.C, D.long_list, D.n_long, P.sums, P.s);
+    return launch_long_sums(D.off, P.head, P.tail, P.chunk, P.C, D.long_list, D.n_long, P.sums, P.s);
 }
 
 FinalizeParams finalize_base(const Problem& P, int d) {
@@ -985,7 +991,7 @@ FinalizeParams finalize_base(const Problem& P, int d) {
         f.sums = P.sums;
         f.head = P.head;
         f.tail = P.tail;
-        f.R = CHUNK_R;
+        f.R = P.chunk;
     }
     f.counts = D.counts;
     f.inv_counts = P.inv_counts_all + P.goff[d];
@@ -2992,8 +2998,8 @@ int cluster_score_sums(Problem& P, const double* S, int ns, const int32_t* perm,
     sp.gseq = gseq;
     sp.pend.n = 0;
     sp.writeback = 0;
-    sp.R = CHUNK_R;
-    long long nchunks = std::max(1LL, seg_nchunks(sp.n, CHUNK_R));
+    sp.R = P.chunk;
+    long long nchunks = std::max(1LL, seg_nchunks(sp.n, P.chunk));
     double *sums = nullptr, *head = nullptr, *tail = nullptr;
     FEGB_TRY(scr.alloc(&sums, (size_t)std::max(1, n_cl) * ns, "score sums"));
     FEGB_TRY(scr.alloc(&head, (size_t)nchunks * ns, "score heads"));
@@ -3014,7 +3020,7 @@ int cluster_score_sums(Problem& P, const double* S, int ns, const int32_t* perm,
     if (!cached) {
         Scratch& where = persistent_off ? *P.scr : scr;
         FEGB_TRY(where.alloc(&long_list, (size_t)std::max(1, n_cl), "score long groups"));
-        FEGB_TRY(find_long_groups(off, n_cl, CHUNK_R, long_list, &n_long, P.s));
+        FEGB_TRY(find_long_groups(off, n_cl, P.chunk, long_list, &n_long, P.s));
         if (persistent_off) P.long_cache.push_back({off, n_cl, long_list, n_long});
     }
     // outputs: the finalize's other outputs (means, maxima), its sources set here
@@ -3025,7 +3031,7 @@ int cluster_score_sums(Problem& P, const double* S, int ns, const int32_t* perm,
     f.sums = sums;
     f.head = head;
     f.tail = tail;
-    f.R = CHUNK_R;
+    f.R = P.chunk;
     f.partials = nullptr;
     f.sum_out = Sc;
     CGTimer tm(P);
@@ -3033,7 +3039,7 @@ int cluster_score_sums(Problem& P, const double* S, int ns, const int32_t* perm,
         FEGB_TRY(tm.begin(timed_kind, (double)sp.n * (4.0 + (perm ? 4.0 : 0.0) + 8.0 * ns)));
     FEGB_TRY(launch_seg_sweep<double>(sp, P.s));
     FEGB_TRY(tm.end());
-    FEGB_TRY(launch_long_sums(off, head, tail, CHUNK_R, ns, long_list, n_long, sums, P.s));
+    FEGB_TRY(launch_long_sums(off, head, tail, P.chunk, ns, long_list, n_long, sums, P.s));
     return launch_finalize(f, P.s);
 }
 
@@ -3050,13 +3056,13 @@ int tuple_row_sums(Problem& P, const double* X, int C, double* out, Scratch& scr
     if (!c) {
         Problem::LongCache e{off, G, nullptr, 0};
         FEGB_TRY(P.scr->alloc(&e.list, (size_t)std::max(1, G), "tuple long groups"));
-        FEGB_TRY(find_long_groups(off, G, CHUNK_R, e.list, &e.n, P.s));
+        FEGB_TRY(find_long_groups(off, G, P.chunk, e.list, &e.n, P.s));
         P.long_cache.push_back(e);
         c = &P.long_cache.back();
     }
     if (!c->multi) {
         FEGB_TRY(P.scr->alloc(&c->multi, (size_t)std::max(1, G), "tuple multi-chunk groups"));
-        FEGB_TRY(find_multi_groups(off, G, CHUNK_R, c->multi, &c->n_multi, P.s));
+        FEGB_TRY(find_multi_groups(off, G, P.chunk, c->multi, &c->n_multi, P.s));
     }
     SegSweepParams<double> sp{};
     sp.X = const_cast<double*>(X);
@@ -3066,8 +3072,8 @@ int tuple_row_sums(Problem& P, const double* X, int C, double* out, Scratch& scr
     sp.n = P.n;
     sp.perm = P.tuple_perm;
     sp.gseq = P.tuple_gseq;
-    sp.R = CHUNK_R;
-    const long long nchunks = std::max(1LL, seg_nchunks(P.n, CHUNK_R));
+    sp.R = P.chunk;
+    const long long nchunks = std::max(1LL, seg_nchunks(P.n, P.chunk));
     FEGB_TRY(scr.alloc(&sp.head, (size_t)nchunks * C, "tuple heads"));
     FEGB_TRY(scr.alloc(&sp.tail, (size_t)nchunks * C, "tuple tails"));
     sp.sums = out;
@@ -3075,7 +3081,7 @@ int tuple_row_sums(Problem& P, const double* X, int C, double* out, Scratch& scr
     if (timed_kind >= 0) FEGB_TRY(tm.begin(timed_kind, (double)P.n * (8.0 + 8.0 * C)));
     FEGB_TRY(launch_seg_sweep<double>(sp, P.s));
     FEGB_TRY(tm.end());
-    return launch_group_sums<double>(off, sp.head, sp.tail, CHUNK_R, C, c->list, c->n, c->multi, c->n_multi, out,
+    return launch_group_sums<double>(off, sp.head, sp.tail, P.chunk, C, c->list, c->n, c->multi, c->n_multi, out,
                                      P.s);
 }
 

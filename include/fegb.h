@@ -94,7 +94,8 @@ typedef struct fegb_result {
      * data sweeps (rows read, and written back in storage order):
      *   [0] segment FP64, [1] segment FP32, [2] small-G FP64, [3] small-G FP32
      *   algorithmic bytes n (4 + 2 C s) per launch;
-     * CG operator sweeps (no row data; ids and gathered FE table rows):
+     * group-table sweeps (no row data; ids and gathered FE table rows): the CG operator, and the
+     * alternating projections on group tables
      *   [4] segment FP64, [5] segment FP32, [6] small-G FP64, [7] small-G FP32
      *   algorithmic bytes n (4 D + (D-1) C s) per launch, D = FE dimensions */
     int prof_launches[8];
