@@ -46,9 +46,12 @@ double be_seconds_since(BeClock::time_point t0) {
 constexpr int BE_THREADS = 256;
 // Rows (or clusters) per work item: the class cut into some BE_ITEMS items, so that
 // small classes fill the chip too (0.8M rows of 24 columns in 16384-row items
-// left two thirds of the SMs idle), within these limits.
+// left two thirds of the SMs idle), within these limits. The Gram's items always
+// have BE_ITEM_MAX rows, which its sums are ordered by; a small class shares out
+// their tiles instead (be_gram).
 constexpr int BE_ITEMS = 1216;
 constexpr int BE_ITEM_MIN = 1024, BE_ITEM_MAX = 16384;
+constexpr double BE_TILE_BYTES = 1.0e9;  // most for the sums of single tiles
 // rows per shared-memory tile of the Gram: about 4096 values (32 KB as FP64),
 // a multiple of 32 between 32 and 256
 __host__ __device__ inline int be_tile_rows(int Cw) {
@@ -68,6 +71,7 @@ inline int be_ppt(int Cw) {
 struct BeItem {
     int spec;
     long long r0, r1;
+    long long tile0;  // part of an item: index of its first tile
 };
 
 // Per-specification state on the device.
@@ -109,7 +113,8 @@ struct RowMajor {
 template <class Acc, bool SPLIT, int BE_PPT>
 __global__ void __launch_bounds__(BE_THREADS)
     be_gram_kernel(Acc X, const BeItem* __restrict__ items, int n_items, const int* __restrict__ width_of,
-                   int Cw, double* __restrict__ partials, int* __restrict__ queue, int* __restrict__ bad) {
+                   int Cw, double* __restrict__ partials, double* __restrict__ tile_sums, int* __restrict__ queue,
+                   int* __restrict__ bad) {
     extern __shared__ __align__(16) unsigned char be_smem[];
     __shared__ int s_item;
     __shared__ double s_fold[BE_THREADS];
@@ -177,7 +182,13 @@ __global__ void __launch_bounds__(BE_THREADS)
                         if (pv[q]) ds_fma(x[r * Cw + pi[q]], x[r * Cw + pj[q]], sh[q], sl[q]);
                 }
 #pragma unroll
-                for (int q = 0; q < BE_PPT; ++q) acc[q] += ((double)sh[q] + (double)sl[q]) + ((double)sh2[q] + (double)sl2[q]);
+                for (int q = 0; q < BE_PPT; ++q) {
+                    const double v = ((double)sh[q] + (double)sl[q]) + ((double)sh2[q] + (double)sl2[q]);
+                    if (tile_sums)
+                        tile_sums[((item.tile0 + (r0 - item.r0) / TR) * BE_PPT + q) * BE_THREADS + t] = v;
+                    else
+                        acc[q] += v;
+                }
             } else {
                 const double* x = reinterpret_cast<const double*>(be_smem);
                 for (int r = phase; r < rows; r += phases) {
@@ -188,7 +199,8 @@ __global__ void __launch_bounds__(BE_THREADS)
             }
         }
         double* out = partials + (long long)it * P;
-        if (one) {
+        if (SPLIT && tile_sums) {
+        } else if (one) {
             s_fold[t] = pv[0] ? acc[0] : 0.0;
             __syncthreads();
             if (t < P) {
@@ -215,7 +227,8 @@ __global__ void __launch_bounds__(BE_THREADS)
 template <class Acc>
 __global__ void __launch_bounds__(BE_THREADS)
     be_gram_blocked_kernel(Acc X, const BeItem* __restrict__ items, int n_items, const int* __restrict__ width_of,
-                           int Cw, double* __restrict__ partials, int* __restrict__ queue, int* __restrict__ bad) {
+                           int Cw, double* __restrict__ partials, double* __restrict__ tile_sums,
+                           int* __restrict__ queue, int* __restrict__ bad) {
     extern __shared__ __align__(16) unsigned char be_smem[];
     __shared__ int s_item;
     __shared__ double s_fold[BE_THREADS][17];  // a thread's 16 sums (odd stride: no bank conflicts)
@@ -273,9 +286,20 @@ __global__ void __launch_bounds__(BE_THREADS)
 #pragma unroll
                         for (int jj = 0; jj < 4; ++jj) ds_fma(xi[ii], xj[jj], sh[ii * 4 + jj], sl[ii * 4 + jj]);
                 }
+                double* ts = tile_sums ? tile_sums + (item.tile0 + (r0 - item.r0) / TR) * 16 * BE_THREADS + t : nullptr;
 #pragma unroll
-                for (int e = 0; e < 16; ++e) acc[e] += (double)sh[e] + (double)sl[e];
+                for (int e = 0; e < 16; ++e) {
+                    const double v = (double)sh[e] + (double)sl[e];
+                    if (ts)
+                        ts[e * BE_THREADS] = v;
+                    else
+                        acc[e] += v;
+                }
             }
+        }
+        if (tile_sums) {
+            __syncthreads();  // s_item is reused
+            continue;
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e) s_fold[t][e] = active ? acc[e] : 0.0;
@@ -296,6 +320,40 @@ __global__ void __launch_bounds__(BE_THREADS)
         __syncthreads();  // s_item and s_fold are reused
     }
     if (__any_sync(0xffffffffu, oor) && (t & 31) == 0) atomicOr(bad, 1);
+}
+
+// Sums of single tiles -> partials[item][p], as the kernels above add them: a
+// thread's tiles in order, then the row phases in order. blocked: sum e = blockIdx.y
+// of the threads' 4 x 4 blocks; else one pair per thread.
+__global__ void __launch_bounds__(BE_THREADS)
+    be_fold_tiles_kernel(const double* __restrict__ tile_sums, const long long* __restrict__ tile0, int Cw, int blocked,
+                         double* __restrict__ partials) {
+    __shared__ double s_fold[BE_THREADS];
+    const int t = threadIdx.x, e = blockIdx.y, slots = gridDim.y;
+    const int P = Cw * (Cw + 1) / 2;
+    const int nbk = (Cw + 3) / 4;
+    const int units = blocked ? nbk * (nbk + 1) / 2 : P;  // threads of a row phase
+    const int phases = BE_THREADS / units;
+    double acc = 0.0;
+    if (t < units * phases) {
+        const double* src = tile_sums + e * BE_THREADS + t;
+#pragma unroll 8
+        for (long long i = tile0[blockIdx.x]; i < tile0[blockIdx.x + 1]; ++i) acc += src[i * slots * BE_THREADS];
+    }
+    s_fold[t] = acc;
+    __syncthreads();
+    if (t >= units) return;
+    double v = 0.0;
+    for (int ph = 0; ph < phases; ++ph) v += s_fold[ph * units + t];
+    double* out = partials + (long long)blockIdx.x * P;
+    if (!blocked) {
+        out[t] = v;
+        return;
+    }
+    int jb = 0;
+    while ((jb + 1) * (jb + 2) / 2 <= t) ++jb;
+    const int i = 4 * (t - jb * (jb + 1) / 2) + e / 4, j = 4 * jb + e % 4;
+    if (i <= j && j < Cw) out[j * (j + 1) / 2 + i] = v;
 }
 
 // out[s][p] = sum over the items of specification s (in order) of partials[item][p]
@@ -381,7 +439,7 @@ __global__ void __launch_bounds__(DN_THREADS)
         for (int e = t; e < na * k; e += DN_THREADS) Qzx[e] = gram_at(G, S.za[e % na], 1 + e / na);
         for (int j = t; j < na; j += DN_THREADS) zy[j] = gram_at(G, S.za[j], 0);
         __syncthreads();
-        chol_solve_inv_block(na, Qzz, na, nullptr, zy, rhs, Qiz, &s_info, work, fits ? dn_stride(na) : na);
+        chol_solve_inv_block<true>(na, Qzz, na, nullptr, zy, rhs, Qiz, &s_info, work, fits ? dn_stride(na) : na);
         __syncthreads();
         if (s_info != 0) {
             if (t == 0) S.info = s_info;
@@ -428,7 +486,7 @@ __global__ void __launch_bounds__(DN_THREADS)
     __syncthreads();
     const int kk = s_kk;
     if (kk == 0) return;
-    chol_solve_inv_block(kk, Q, k, s_kept, b, bsel, Qinv, &s_info, work, fits ? dn_stride(kk) : kk);
+    chol_solve_inv_block<true>(kk, Q, k, s_kept, b, bsel, Qinv, &s_info, work, fits ? dn_stride(kk) : kk);
     __syncthreads();
     if (s_info != 0) {
         if (t == 0) S.info = s_info;
@@ -717,7 +775,11 @@ int be_sync_copy(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, 
 }
 
 // Gram products through the work queue: split-FP32 first, FP64 again when a
-// value is outside the split range; folded per specification into out.
+// value is outside the split range; folded per specification into out. The items
+// are the unit of the sums' order. A class with few of them shares out their
+// tiles, about BE_ITEMS parts in all: the double-single sums of every tile are kept
+// and added afterwards in the order in which a block with the whole item adds them
+// (60 specifications of 5k to 200k rows: Gram products 18.5 -> 2.9 ms).
 template <class Acc>
 int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& item0, const std::vector<int>& item1,
             const int* d_width, int ns, int Cw, double* out, cudaStream_t s, Scratch& scr) {
@@ -727,7 +789,24 @@ int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& it
         FEGB_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * (size_t)ns * P, s), "batch gram zero");
         return 0;
     }
-    BeItem* d_items = nullptr;
+    const bool blocked = Cw >= 16;
+    const int TR = be_tile_rows(Cw), slots = blocked ? 16 : 1;
+    std::vector<long long> tile0(n_items + 1, 0);
+    for (int i = 0; i < n_items; ++i) tile0[i + 1] = tile0[i] + (hitems[i].r1 - hitems[i].r0 + TR - 1) / TR;
+    const long long tiles = tile0[n_items];
+    const bool by_tiles = n_items < BE_ITEMS / 2 && (double)tiles * slots * BE_THREADS * sizeof(double) <= BE_TILE_BYTES;
+    std::vector<BeItem> parts;
+    if (by_tiles) {
+        const long long step = std::max(1LL, tiles / BE_ITEMS) * TR;
+        for (int i = 0; i < n_items; ++i)
+            for (long long r = hitems[i].r0; r < hitems[i].r1; r += step)
+                parts.push_back({hitems[i].spec, r, std::min(hitems[i].r1, r + step), tile0[i] + (r - hitems[i].r0) / TR});
+    }
+    const int n_parts = (int)parts.size();
+    Scratch sub(s);  // parts and tile sums, given back at the end
+    BeItem *d_items = nullptr, *d_parts = nullptr;
+    double* d_tiles = nullptr;
+    long long* d_tile0 = nullptr;
     int *d_i0 = nullptr, *d_i1 = nullptr, *d_q = nullptr, *d_bad = nullptr;
     double* part = nullptr;
     FEGB_TRY(scr.alloc(&d_items, hitems.size(), "batch items"));
@@ -742,18 +821,29 @@ int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& it
     FEGB_CUDA(cudaMemcpyAsync(d_i1, item1.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s), "batch item1 copy");
     FEGB_CUDA(cudaMemsetAsync(d_q, 0, sizeof(int) * 2, s), "batch queue reset");
     FEGB_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), s), "batch flag reset");
-    const int grid = std::min(n_items, num_sms() * 4);
+    if (by_tiles) {
+        FEGB_TRY(sub.alloc(&d_parts, parts.size(), "batch item parts"));
+        FEGB_TRY(sub.alloc(&d_tile0, tile0.size(), "batch item tiles"));
+        FEGB_TRY(sub.alloc(&d_tiles, (size_t)tiles * slots * BE_THREADS, "batch tile sums"));
+        FEGB_CUDA(cudaMemcpyAsync(d_parts, parts.data(), sizeof(BeItem) * parts.size(), cudaMemcpyHostToDevice, s),
+                  "batch parts copy");
+        FEGB_CUDA(cudaMemcpyAsync(d_tile0, tile0.data(), sizeof(long long) * tile0.size(), cudaMemcpyHostToDevice, s),
+                  "batch tiles copy");
+    }
+    const BeItem* d_split = by_tiles ? d_parts : d_items;  // what the double-single kernels work through
+    const int n_split = by_tiles ? n_parts : n_items;
+    const int grid = std::min(n_items, num_sms() * 4), split_grid = std::min(n_split, num_sms() * 4);
     const size_t smem = sizeof(double) * (size_t)be_tile_rows(Cw) * Cw;  // float2 and double are both 8 bytes
     auto launch = [&](bool split, int* q) -> int {
         const int ppt = be_ppt(Cw);
 #define BE_GRAM_CASE(NPT)                                                                                          \
     if (ppt == NPT) {                                                                                              \
         if (split)                                                                                                 \
-            be_gram_kernel<Acc, true, NPT><<<grid, BE_THREADS, smem, s>>>(X, d_items, n_items, d_width, Cw, part, q, \
-                                                                          d_bad);                                  \
+            be_gram_kernel<Acc, true, NPT><<<split_grid, BE_THREADS, smem, s>>>(X, d_split, n_split, d_width, Cw,    \
+                                                                                part, d_tiles, q, d_bad);           \
         else                                                                                                       \
             be_gram_kernel<Acc, false, NPT><<<grid, BE_THREADS, smem, s>>>(X, d_items, n_items, d_width, Cw, part,   \
-                                                                           q, d_bad);                              \
+                                                                           nullptr, q, d_bad);                     \
     }
         BE_GRAM_CASE(1)
         BE_GRAM_CASE(2)
@@ -763,7 +853,7 @@ int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& it
         FEGB_LAUNCH_CHECK("batch gram");
         return 0;
     };
-    if (Cw >= 16) {
+    if (blocked) {
         // the blocked double-single form (16 products per 8 shared-memory reads);
         // below 16 columns there are too few 4 x 4 blocks per row and the
         // phases' folds cost more than the reads saved (8 columns: 25 -> 30 ms)
@@ -773,11 +863,16 @@ int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& it
         static const cudaError_t attr = cudaFuncSetAttribute(be_gram_blocked_kernel<Acc>,
                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         if (attr != cudaSuccess) return set_cuda_error(attr, "batch gram (blocked) attr");
-        be_gram_blocked_kernel<Acc><<<grid, BE_THREADS, bsmem, s>>>(X, d_items, n_items, d_width, Cw, part, d_q,
-                                                                    d_bad);
+        be_gram_blocked_kernel<Acc><<<split_grid, BE_THREADS, bsmem, s>>>(X, d_split, n_split, d_width, Cw, part,
+                                                                          d_tiles, d_q, d_bad);
         FEGB_LAUNCH_CHECK("batch gram (blocked)");
     } else {
         FEGB_TRY(launch(true, d_q));
+    }
+    if (by_tiles) {
+        be_fold_tiles_kernel<<<dim3((unsigned)n_items, (unsigned)slots), BE_THREADS, 0, s>>>(d_tiles, d_tile0, Cw, blocked,
+                                                                                          part);
+        FEGB_LAUNCH_CHECK("batch tile fold");
     }
     int hbad = 0;
     FEGB_TRY(be_sync_copy(&hbad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s, "batch split flag copy"));
@@ -787,18 +882,21 @@ int be_gram(Acc X, const std::vector<BeItem>& hitems, const std::vector<int>& it
     return 0;
 }
 
+// Work items of the rows [begin[s], end[s]) of every specification; whole: of
+// BE_ITEM_MAX rows (the Gram's), else as many as fill the chip.
 void be_items(const std::vector<long long>& begin, const std::vector<long long>& end, std::vector<BeItem>& items,
-              std::vector<int>& item0, std::vector<int>& item1) {
+              std::vector<int>& item0, std::vector<int>& item1, bool whole = false) {
     const int ns = (int)begin.size();
     items.clear();
     item0.assign(ns, 0);
     item1.assign(ns, 0);
     long long total = 0;
     for (int s = 0; s < ns; ++s) total += std::max(0LL, end[s] - begin[s]);
-    const long long rows = std::min<long long>(BE_ITEM_MAX, std::max<long long>(BE_ITEM_MIN, (total / BE_ITEMS + 255) / 256 * 256));
+    const long long fill = (total / BE_ITEMS + 255) / 256 * 256;
+    const long long rows = whole ? BE_ITEM_MAX : std::min<long long>(BE_ITEM_MAX, std::max<long long>(BE_ITEM_MIN, fill));
     for (int s = 0; s < ns; ++s) {
         item0[s] = (int)items.size();
-        for (long long r = begin[s]; r < end[s]; r += rows) items.push_back({s, r, std::min(end[s], r + rows)});
+        for (long long r = begin[s]; r < end[s]; r += rows) items.push_back({s, r, std::min(end[s], r + rows), 0});
         item1[s] = (int)items.size();
     }
 }
@@ -928,7 +1026,12 @@ int estimate_class_batched(const fegb_config& cfg, const std::vector<BeSpecHost>
     FEGB_TRY(scr.alloc(&d_Qinv, (size_t)ns * Kb * Kb, "batch Qinv"));
     FEGB_TRY(scr.alloc(&d_Pi, (size_t)ns * Kb * Kb, "batch Pi"));
     ColMajorX X{yb, Wb, N};
-    FEGB_TRY(be_gram(X, items, item0, item1, d_width, ns, Cw, d_gram, s, scr));
+    {
+        std::vector<BeItem> gitems;
+        std::vector<int> gi0, gi1;
+        be_items(rb, re, gitems, gi0, gi1, true);
+        FEGB_TRY(be_gram(X, gitems, gi0, gi1, d_width, ns, Cw, d_gram, s, scr));
+    }
     FEGB_TRY(phase("gram"));
     static const cudaError_t solve_attr =
         cudaFuncSetAttribute(be_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
@@ -1072,7 +1175,7 @@ int estimate_class_batched(const fegb_config& cfg, const std::vector<BeSpecHost>
             }
             std::vector<BeItem> citems;
             std::vector<int> ci0, ci1;
-            be_items(cb, ce, citems, ci0, ci1);
+            be_items(cb, ce, citems, ci0, ci1, true);
             int* d_swidth = nullptr;
             FEGB_TRY(scr.alloc(&d_swidth, (size_t)ns, "score widths"));
             FEGB_CUDA(cudaMemcpyAsync(d_swidth, swidth.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s),

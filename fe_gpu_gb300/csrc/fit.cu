@@ -120,6 +120,14 @@ struct Problem {
     double* mu_all = nullptr;
     int smallg_nb = 0;
     int chunk = 256;  // positions a chunk of the row sweeps (chunk_rows)
+    // Specifications stacked in one problem (a batch). One of them may be close to
+    // unidentified (2SLS with two endogenous regressors of nearly the same first
+    // stage: condition numbers of 1e4 to 1e11), and then another rounding of the
+    // within-transform moves its coefficients in the 7th to 9th digit. The CG form
+    // of a stack therefore adds in one order whatever its size: 256-position chunks,
+    // 4,096-row blocks, sixteen vector steps, row streams sorted by group and the
+    // refinement on the rows.
+    bool stacked = false;
     // the CG operator's row sort by distinct id tuples of its swept dimensions
     // (positions grouped by tuple), kept for the cluster subset over the same
     // dimensions: tuple t holds sorted positions tuple_off[t] .. tuple_off[t+1]
@@ -661,7 +669,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
         }
     }
     P.n = n;
-    P.chunk = chunk_rows(n, P.C);
+    P.chunk = P.stacked ? 256 : chunk_rows(n, P.C);
     const int C = P.C;
     // primary dimension: the one with most groups (first on ties)
     P.primary = -1;
@@ -737,7 +745,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     }
     // rows that come in the primary's order, and one other swept dimension: its
     // runs may serve instead of its row order
-    if (sorted_all && in_primary_order && n >= 4096) {
+    if (sorted_all && in_primary_order && n >= 4096 && !P.stacked) {
         const std::vector<char> dense = cg_dense_plan(G, C, n);
         int other = -1, swept = 0;
         for (int d = 0; d < n_fe; ++d)
@@ -818,7 +826,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     FEGB_TRY(dalloc(scr, &P.sums, (size_t)gmax * C, "group sums"));
     FEGB_TRY(dalloc(scr, &P.head, (size_t)nchunks * C, "chunk heads"));
     FEGB_TRY(dalloc(scr, &P.tail, (size_t)nchunks * C, "chunk tails"));
-    P.smallg_nb = smallg_nblocks(std::max(1LL, n));
+    P.smallg_nb = smallg_nblocks(std::max(1LL, n), P.stacked ? SMALLG_STACKED_ROWS : SMALLG_MIN_ROWS);
     if (gmax_small > 0) FEGB_TRY(dalloc(scr, &P.partials, (size_t)P.smallg_nb * gmax_small * C, "small-G partials"));
     FEGB_TRY(dalloc(scr, &P.relax, (size_t)std::max(1, n_fe), "relaxation"));
     FEGB_TRY(dalloc(scr, &P.prev_change, (size_t)std::max(1, n_fe), "prev change"));
@@ -1682,11 +1690,12 @@ int cg_alloc(Problem& P, CGBuffers<T>& B) {
     FEGB_TRY(dalloc(scr, &B.rz_new, (size_t)C, "cg rz new"));
     FEGB_TRY(dalloc(scr, &B.pq, (size_t)C, "cg pq"));
     FEGB_TRY(dalloc(scr, &B.zmax, 1, "cg zmax"));
-    B.rz_blocks = cg_partial_blocks(B.Gv, C);
+    B.rz_blocks = cg_partial_blocks(B.Gv, C, P.stacked);
     B.pq_block_off.assign(P.n_fe + 1, 0);
     for (int d = 0; d < P.n_fe; ++d)
         B.pq_block_off[d + 1] =
-            B.pq_block_off[d] + (B.schur && d == B.prim ? 0 : cg_partial_blocks(std::max(1, P.dims[d].G), C));
+            B.pq_block_off[d] +
+            (B.schur && d == B.prim ? 0 : cg_partial_blocks(std::max(1, P.dims[d].G), C, P.stacked));
     B.pq_blocks = B.pq_block_off[P.n_fe];
     FEGB_TRY(dalloc(scr, &B.rz_part, (size_t)B.rz_blocks * C, "cg rz partials"));
     FEGB_TRY(dalloc(scr, &B.zmax_part, (size_t)B.rz_blocks, "cg zmax partials"));
@@ -1945,7 +1954,7 @@ int cg_apply_rest(Problem& P, CGBuffers<T>& B, bool prim_small_done = false) {
         }
         FEGB_TRY(launch_cg_q<T>(src, C, B.p + B.off[d] * L, L, B.q + B.off[d] * C,
                                 B.pq_part + (size_t)B.pq_block_off[d] * C, P.s,
-                                B.any_dense ? B.extra + B.off[d] * C : nullptr));
+                                B.any_dense ? B.extra + B.off[d] * C : nullptr, P.stacked));
         P.projections += 1;
     }
     for (int sd = 0; sd < P.n_fe; ++sd) {
@@ -1956,7 +1965,7 @@ int cg_apply_rest(Problem& P, CGBuffers<T>& B, bool prim_small_done = false) {
         src.sums = B.dense_sums + B.dsum_off[sd];  // complete sums of -p, compact rows
         src.counts = P.dims[sd].counts;
         FEGB_TRY(launch_cg_q<T>(src, C, B.p + B.off[sd] * L, L, B.q + B.off[sd] * C,
-                                B.pq_part + (size_t)B.pq_block_off[sd] * C, P.s));
+                                B.pq_part + (size_t)B.pq_block_off[sd] * C, P.s, nullptr, P.stacked));
         P.projections += 1;
     }
     return 0;
@@ -1983,7 +1992,7 @@ int cg_start(Problem& P, CGBuffers<T>& B) {
     const int L = B.ld;
     if (!B.schur)
         return launch_cg_init<T>(P.Gt, C, P.counts_all, P.mu_all, B.r, B.z, B.p, L, B.x, B.rz_part, B.zmax_part,
-                                 B.zmax, P.s);
+                                 B.zmax, P.s, P.stacked);
     const int pd = B.prim;
     FEGB_CUDA(cudaMemsetAsync(B.p, 0, sizeof(T) * (size_t)B.Gv * L, P.s), "cg p zero");
     FEGB_TRY(launch_table_from_f64<T>(P.mu_all + P.goff[pd] * C, P.dims[pd].G, C, -1.0, B.p + B.off[pd] * L, L,
@@ -1995,7 +2004,7 @@ int cg_start(Problem& P, CGBuffers<T>& B) {
                                       sizeof(double) * (size_t)P.dims[d].G * C, cudaMemcpyDeviceToDevice, P.s),
                       "cg means copy");
     return launch_cg_init_rhs<T>(B.Gv, C, B.counts_v, B.mu_v, B.q, B.inv, B.r, B.z, B.p, L, B.x, B.rz_part,
-                                 B.zmax_part, B.zmax, P.s);
+                                 B.zmax_part, B.zmax, P.s, P.stacked);
 }
 
 // End of an inner solve: the FE increments of x become the FP64 table applied
@@ -2145,7 +2154,7 @@ int cg_build_graph(Problem& P, CGBuffers<T>& B, CGGraph<T>& G) {
     int st = cg_apply<T>(P, B);
     if (!st)
         st = launch_cg_update<T>(B.Gv, C, B.inv, B.rz, B.pq, B.p, B.ld, B.q, B.x, B.r, B.z, B.rz_part, B.zmax_part,
-                                 B.zmax, cs);
+                                 B.zmax, cs, P.stacked);
     if (!st) st = launch_fold_partials(B.rz_part, B.rz_blocks, C, B.rz_new, cs);
     if (!st) {
         cg_loop_check_kernel<<<1, 1, 0, cs>>>(B.zmax, B.rz_new, C, G.ctl, h);
@@ -2200,7 +2209,7 @@ int cg_solve_host(Problem& P, CGBuffers<T>& B, double inner_tol, int max_it, int
     for (; it < max_it; ++it) {
         FEGB_TRY(cg_apply<T>(P, B));
         FEGB_TRY(launch_cg_update<T>(B.Gv, C, B.inv, B.rz, B.pq, B.p, B.ld, B.q, B.x, B.r, B.z, B.rz_part,
-                                     B.zmax_part, B.zmax, P.s));
+                                     B.zmax_part, B.zmax, P.s, P.stacked));
         FEGB_TRY(launch_fold_partials(B.rz_part, B.rz_blocks, C, B.rz_new, P.s));
         FEGB_CUDA(cudaMemcpyAsync(rz_host.data(), B.rz_new, sizeof(double) * C, cudaMemcpyDeviceToHost, P.s),
                   "cg r.z copy");
@@ -2723,7 +2732,7 @@ int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* conver
         }
     }
     Refinement R;
-    if (ap_on_groups(P.C, P.n_fe, P.n)) {
+    if (ap_on_groups(P.C, P.n_fe, P.n) && !P.stacked) {
         FEGB_TRY(R.A.adopt(P, B));
         R.possible = true;
     }
@@ -3767,7 +3776,8 @@ int reconstruct_fe_impl(const fegb_config& cfg, long long n, int k, int n_fe, co
 
 // In-place within-transform of device columns (column-major, ld n).
 int within_impl(const fegb_config& cfg, long long n, int k, int l, int n_fe, double* d_y, double* d_W, double* d_Z,
-                const int32_t* const* ids, const int* group_sizes, cudaStream_t s, PreDemeaned* out) {
+                const int32_t* const* ids, const int* group_sizes, cudaStream_t s, PreDemeaned* out,
+                bool stacked = false) {
     configure_mem_pool();
     auto t0 = Clock::now();
     Scratch scr(s);
@@ -3775,6 +3785,7 @@ int within_impl(const fegb_config& cfg, long long n, int k, int l, int n_fe, dou
     P.s = s;
     P.scr = &scr;
     P.profile = cfg.profile != 0;
+    P.stacked = stacked;
     long long n_single = 0;
     FEGB_TRY(build_problem(P, n, k, l, n_fe, d_y, d_W, d_Z, ids, group_sizes, false,
                            ap_needs_rows(cfg, 1 + k + l, n_fe, n), &n_single,
@@ -4013,7 +4024,7 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
         for (int d = 0; d < fe_b; ++d) ids_b[d] = idsb + (size_t)d * N;
         PreDemeaned pre;
         auto tc0 = Clock::now();
-        FEGB_TRY(within_impl(cfg, N, kb, 0, fe_b, yb, Wb, nullptr, ids_b.data(), Gb.data(), s, &pre));
+        FEGB_TRY(within_impl(cfg, N, kb, 0, fe_b, yb, Wb, nullptr, ids_b.data(), Gb.data(), s, &pre, true));
         FEGB_CUDA(cudaStreamSynchronize(s), "batch demean sync");
         const double t_within = seconds_since(tc0);
         tc0 = Clock::now();
@@ -4167,7 +4178,7 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
     struct BatchClass {
         int cb;
         std::vector<int> idx;
-        double bytes;  // device memory while it runs: the stack, the data block, scores, ids and orders
+        double bytes;  // device memory while it runs: the stack, the data block, scores, tile sums, ids and orders
     };
     std::vector<BatchClass> classes;
     for (size_t pos = 0; pos < order.size();) {
@@ -4177,7 +4188,7 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
             c.idx.push_back(order[pos].second);
             rows += (double)specs[order[pos].second].n;
         }
-        c.bytes = rows * (8.0 * 5 * c.cb + 4.0 * 40);
+        c.bytes = rows * (8.0 * 6 * c.cb + 4.0 * 40);
         classes.push_back(std::move(c));
     }
     std::stable_sort(classes.begin(), classes.end(),

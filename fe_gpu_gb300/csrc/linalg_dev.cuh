@@ -75,7 +75,12 @@ __device__ inline int block_chol_factor(int k, double* U, int ld) {
 // One block of DN_THREADS threads: Q_sel = Q[idx, idx] (or the leading k x k
 // block), upper Cholesky factor, solve for b_sel and the inverse. info: 0 ok,
 // j > 0 when the leading minor j is not positive definite. work: 2 k ld doubles
-// (global or shared), ld >= k.
+// (global or shared), ld >= k. BY_COLUMN: a thread per column of the inverse and
+// one for the back substitution, every sum over ascending indexes (stacked
+// specifications, some of them so ill-conditioned that another order of these sums
+// moves a standard error by 1e-7; up to 64 columns, where the longer chains cost
+// some microseconds).
+template <bool BY_COLUMN = false>
 __device__ inline void chol_solve_inv_block(int k, const double* __restrict__ Q, int ldq, const int* __restrict__ idx,
                                      const double* __restrict__ b, double* __restrict__ beta,
                                      double* __restrict__ Qinv, int* __restrict__ info, double* work, int ld) {
@@ -96,7 +101,19 @@ __device__ inline void chol_solve_inv_block(int k, const double* __restrict__ Q,
     }
     // rows of U^{-1} from the last: X[i][j] gathers sum_p U[i][p] X[p][j] over the
     // finished rows p > i, then row i is -that / U[i][i]
-    for (int p = k - 1; p >= 0; --p) {
+    if (BY_COLUMN) {
+        for (int j = t; j < k; j += DN_THREADS) {
+            X[(size_t)j * ld + j] = 1.0 / U[(size_t)j * ld + j];
+            for (int i = j - 1; i >= 0; --i) {
+                const double* ui = U + (size_t)i * ld;
+                double s = 0.0;
+                for (int p = i + 1; p <= j; ++p) s = fma(ui[p], X[(size_t)p * ld + j], s);
+                X[(size_t)i * ld + j] = -s / ui[i];
+            }
+        }
+        __syncthreads();
+    }
+    for (int p = BY_COLUMN ? -1 : k - 1; p >= 0; --p) {
         double* xp = X + (size_t)p * ld;
         const double u = U[(size_t)p * ld + p];
         for (int j = p + t; j < k; j += DN_THREADS) xp[j] = j == p ? 1.0 / u : -xp[j] / u;
@@ -132,7 +149,15 @@ __device__ inline void chol_solve_inv_block(int k, const double* __restrict__ Q,
             for (int c = i + 1 + lane; c < k; c += 32) v[c] = fma(-ui[c], y, v[c]);
             __syncwarp();
         }
-        for (int i = k - 1; i >= 0; --i) {
+        if (BY_COLUMN && lane == 0)
+            for (int i = k - 1; i >= 0; --i) {
+                const double* ui = U + (size_t)i * ld;
+                double y = v[i];
+                for (int p = i + 1; p < k; ++p) y = fma(-ui[p], v[p], y);
+                v[i] = y / ui[i];
+            }
+        __syncwarp();
+        for (int i = BY_COLUMN ? -1 : k - 1; i >= 0; --i) {
             const double y = v[i] / U[(size_t)i * ld + i];
             __syncwarp();
             if (lane == 0) v[i] = y;

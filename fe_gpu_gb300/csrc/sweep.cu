@@ -836,9 +836,8 @@ bool smallg_eligible(int G, int C) {
 
 // Four blocks an SM, of at least 256 rows (a block's warps walk 32 rows each; with
 // 4,096 rows a block 38k x 30 elements took 69 us on 10 blocks, 8 on 149).
-int smallg_nblocks(long long n) {
+int smallg_nblocks(long long n, long long min_rows) {
     long long nb = (long long)num_sms() * 4;
-    long long min_rows = 256;
     if (n / nb < min_rows) nb = (n + min_rows - 1) / min_rows;
     if (nb < 1) nb = 1;
     return (int)nb;
@@ -892,17 +891,17 @@ int launch_convert_f64_f32(const double* src, float* dst, long long n, cudaStrea
 }
 
 
-int cg_vec_steps(long long G, int C) {
+int cg_vec_steps(long long G, int C, bool fixed) {
     constexpr long long FILL = 304;  // blocks that fill the chip (a constant: the same sums on any GPU)
     const long long rps = std::max(1, 256 / C);
     int steps = 16;
-    while (steps > 1 && G < FILL * rps * steps) steps /= 4;
+    while (!fixed && steps > 1 && G < FILL * rps * steps) steps /= 4;
     return steps;
 }
 
-int cg_partial_blocks(long long G, int C) {
+int cg_partial_blocks(long long G, int C, bool fixed) {
     if (C <= 256) {
-        const long long rows = (long long)(256 / C) * cg_vec_steps(G, C);
+        const long long rows = (long long)(256 / C) * cg_vec_steps(G, C, fixed);
         return (int)((G + rows - 1) / rows);
     }
     return (int)((G * C + FIN_THREADS - 1) / FIN_THREADS);
@@ -910,12 +909,12 @@ int cg_partial_blocks(long long G, int C) {
 
 template <typename T>
 int launch_cg_q(const FinalizeParams& src, int C, const T* p, int pld, T* q, double* pq_partials, cudaStream_t s,
-                const T* extra) {
+                const T* extra, bool fixed) {
     long long total = (long long)src.G * C;
     if (total <= 0) return 0;
-    const int nb = cg_partial_blocks(src.G, C);
+    const int nb = cg_partial_blocks(src.G, C, fixed);
     if (C <= 256)
-        cg_q_rows_kernel<T><<<nb, 256, 0, s>>>(src, cg_vec_steps(src.G, C), C, p, pld, q, pq_partials, extra);
+        cg_q_rows_kernel<T><<<nb, 256, 0, s>>>(src, cg_vec_steps(src.G, C, fixed), C, p, pld, q, pq_partials, extra);
     else
         cg_q_kernel<T><<<nb, FIN_THREADS, 0, s>>>(src, C, p, pld, q, pq_partials, extra);
     FEGB_LAUNCH_CHECK("cg q");
@@ -1009,13 +1008,13 @@ int launch_inv_counts(const int32_t* counts, long long G, double* inv_counts, cu
 template <typename T>
 int launch_cg_update(long long Gt, int C, const T* inv_counts, const double* rz, const double* pq, const T* p,
                      int pld, const T* q, T* x, T* r, T* z, double* rz_partials, double* zmax_partials,
-                     unsigned long long* zmax, cudaStream_t s) {
+                     unsigned long long* zmax, cudaStream_t s, bool fixed) {
     long long total = Gt * C;
     if (total <= 0) return 0;
-    const int nb = cg_partial_blocks(Gt, C);
+    const int nb = cg_partial_blocks(Gt, C, fixed);
     if (C <= 256)
-        cg_update_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, inv_counts, rz, pq, p, pld, q, x, r, z, rz_partials,
-                                                    zmax_partials);
+        cg_update_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C, fixed), C, inv_counts, rz, pq, p, pld, q, x, r,
+                                                    z, rz_partials, zmax_partials);
     else
         cg_update_kernel<T><<<nb, FIN_THREADS, 0, s>>>(Gt, C, inv_counts, rz, pq, p, pld, q, x, r, z, rz_partials,
                                                        zmax_partials);
@@ -1041,12 +1040,13 @@ int launch_cg_direction(long long Gt, int C, double* rz_old, const double* rz_ne
 
 template <typename T>
 int launch_cg_init(long long Gt, int C, const int32_t* counts, const double* mu, T* r, T* z, T* p, int pld, T* x,
-                   double* rz_partials, double* zmax_partials, unsigned long long* zmax, cudaStream_t s) {
+                   double* rz_partials, double* zmax_partials, unsigned long long* zmax, cudaStream_t s, bool fixed) {
     long long total = Gt * C;
     if (total <= 0) return 0;
-    const int nb = cg_partial_blocks(Gt, C);
+    const int nb = cg_partial_blocks(Gt, C, fixed);
     if (C <= 256)
-        cg_init_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, counts, mu, r, z, p, pld, x, rz_partials, zmax_partials);
+        cg_init_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C, fixed), C, counts, mu, r, z, p, pld, x,
+                                                  rz_partials, zmax_partials);
     else
         cg_init_kernel<T><<<nb, FIN_THREADS, 0, s>>>(Gt, C, counts, mu, r, z, p, pld, x, rz_partials,
                                                      zmax_partials);
@@ -1059,12 +1059,12 @@ int launch_cg_init(long long Gt, int C, const int32_t* counts, const double* mu,
 template <typename T>
 int launch_cg_init_rhs(long long Gt, int C, const int32_t* counts, const double* mu, const T* qb, const T* inv, T* r,
                        T* z, T* p, int pld, T* x, double* rz_partials, double* zmax_partials, unsigned long long* zmax,
-                       cudaStream_t s) {
+                       cudaStream_t s, bool fixed) {
     if (Gt * C <= 0) return 0;
     if (C > 256) return set_error("cg: %d columns exceed the right-hand-side initialisation", C);
-    const int nb = cg_partial_blocks(Gt, C);
-    cg_init_rhs_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C), C, counts, mu, qb, inv, r, z, p, pld, x, rz_partials,
-                                                  zmax_partials);
+    const int nb = cg_partial_blocks(Gt, C, fixed);
+    cg_init_rhs_rows_kernel<T><<<nb, 256, 0, s>>>(Gt, cg_vec_steps(Gt, C, fixed), C, counts, mu, qb, inv, r, z, p, pld, x,
+                                                  rz_partials, zmax_partials);
     FEGB_LAUNCH_CHECK("cg init (rhs)");
     fold_max_kernel<<<1, FIN_THREADS, 0, s>>>(zmax_partials, nb, zmax);
     FEGB_LAUNCH_CHECK("cg max fold");
@@ -1072,15 +1072,15 @@ int launch_cg_init_rhs(long long Gt, int C, const int32_t* counts, const double*
 }
 template int launch_cg_init_rhs<float>(long long, int, const int32_t*, const double*, const float*, const float*,
                                        float*, float*, float*, int, float*, double*, double*, unsigned long long*,
-                                       cudaStream_t);
+                                       cudaStream_t, bool);
 template int launch_cg_init_rhs<double>(long long, int, const int32_t*, const double*, const double*, const double*,
                                         double*, double*, double*, int, double*, double*, double*,
-                                        unsigned long long*, cudaStream_t);
+                                        unsigned long long*, cudaStream_t, bool);
 
 template int launch_cg_q<double>(const FinalizeParams&, int, const double*, int, double*, double*, cudaStream_t,
-                                 const double*);
+                                 const double*, bool);
 template int launch_cg_q<float>(const FinalizeParams&, int, const float*, int, float*, double*, cudaStream_t,
-                                const float*);
+                                const float*, bool);
 
 // ---- dense count matrices of small-G dimensions ----
 
@@ -1724,10 +1724,10 @@ int launch_fold_dense(const double* partials, int nparts, int Gs, int C, double*
 
 template int launch_cg_update<double>(long long, int, const double*, const double*, const double*, const double*, int,
                                       const double*, double*, double*, double*, double*, double*,
-                                      unsigned long long*, cudaStream_t);
+                                      unsigned long long*, cudaStream_t, bool);
 template int launch_cg_update<float>(long long, int, const float*, const double*, const double*, const float*, int,
                                      const float*, float*, float*, float*, double*, double*, unsigned long long*,
-                                     cudaStream_t);
+                                     cudaStream_t, bool);
 
 template <typename T>
 int launch_to_f64(const T* src, int ld, double* dst, int C, long long G, cudaStream_t s) {
@@ -1754,9 +1754,9 @@ template int launch_cg_direction<double>(long long, int, double*, const double*,
 template int launch_cg_direction<float>(long long, int, double*, const double*, const float*, float*, int,
                                         cudaStream_t, const int*);
 template int launch_cg_init<double>(long long, int, const int32_t*, const double*, double*, double*, double*, int,
-                                    double*, double*, double*, unsigned long long*, cudaStream_t);
+                                    double*, double*, double*, unsigned long long*, cudaStream_t, bool);
 template int launch_cg_init<float>(long long, int, const int32_t*, const double*, float*, float*, float*, int, float*,
-                                   double*, double*, unsigned long long*, cudaStream_t);
+                                   double*, double*, unsigned long long*, cudaStream_t, bool);
 
 
 // ----------------------- row-per-lane CG operator sweep -----------------------

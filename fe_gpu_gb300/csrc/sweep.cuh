@@ -145,8 +145,9 @@ int launch_finalize(const FinalizeParams& p, cudaStream_t s);
 
 // Number of chunks for a segment traversal.
 inline long long seg_nchunks(long long n, int R) { return (n + R - 1) / R; }
-// Number of blocks used by the small-G kernel for n rows.
-int smallg_nblocks(long long n);
+// Number of blocks used by the small-G kernel for n rows, of at least min_rows each.
+constexpr long long SMALLG_MIN_ROWS = 256, SMALLG_STACKED_ROWS = 4096;
+int smallg_nblocks(long long n, long long min_rows = SMALLG_MIN_ROWS);
 // Whether the small-G path can hold G x C per thread slot in shared memory.
 bool smallg_eligible(int G, int C);
 
@@ -233,7 +234,7 @@ inline int cg_row_stride(int C, int elem_bytes) {
 // from the sweep, e.g. from dense small-G count matrices).
 template <typename T>
 int launch_cg_q(const FinalizeParams& src, int C, const T* p, int pld, T* q, double* pq_partials, cudaStream_t s,
-                const T* extra = nullptr);
+                const T* extra = nullptr, bool fixed = false);
 
 // ---- dense count matrices of small-G dimensions ----
 // For a dimension s with few groups and any other dimension e, the operator
@@ -328,9 +329,10 @@ int launch_fold_dense(const double* partials, int nparts, int Gs, int C, double*
 // (C <= 256), else one block per 256 elements. Sixteen steps a block for large
 // tables; fewer where that would leave most of the chip idle and each block a
 // chain of sixteen dependent loads (2,000 groups, 5 columns: update 14 -> 6
-// us a launch, q 7.5 -> 4.3).
-int cg_vec_steps(long long G, int C);
-int cg_partial_blocks(long long G, int C);
+// us a launch, q 7.5 -> 4.3). fixed: sixteen whatever the table (stacked
+// specifications, whose sums keep one order of additions).
+int cg_vec_steps(long long G, int C, bool fixed = false);
+int cg_partial_blocks(long long G, int C, bool fixed = false);
 
 // out[c] = sum_b partials[b * C + c] for b < nb (fixed order)
 int launch_fold_partials(const double* partials, int nb, int C, double* out, cudaStream_t s);
@@ -341,7 +343,7 @@ int launch_fold_partials(const double* partials, int nb, int C, double* out, cud
 template <typename T>
 int launch_cg_update(long long Gt, int C, const T* inv_counts, const double* rz, const double* pq, const T* p,
                      int pld, const T* q, T* x, T* r, T* z, double* rz_partials, double* zmax_partials,
-                     unsigned long long* zmax, cudaStream_t s);
+                     unsigned long long* zmax, cudaStream_t s, bool fixed = false);
 // dst[g * C + c] = (double) src[g * ld + c] for c < C
 template <typename T>
 int launch_to_f64(const T* src, int ld, double* dst, int C, long long G, cudaStream_t s);
@@ -361,7 +363,7 @@ int launch_cg_direction(long long Gt, int C, double* rz_old, const double* rz_ne
 template <typename T>
 int launch_cg_init_rhs(long long Gt, int C, const int32_t* counts, const double* mu, const T* qb, const T* inv, T* r,
                        T* z, T* p, int pld, T* x, double* rz_partials, double* zmax_partials, unsigned long long* zmax,
-                       cudaStream_t s);
+                       cudaStream_t s, bool fixed = false);
 // r = counts * mu, z = p = mu (cast to T); partials of r.z and max |z|
 // inv_counts[g] = 1 / counts[g] (0 for empty groups)
 int launch_inv_counts(const int32_t* counts, long long G, double* inv_counts, cudaStream_t s);
@@ -369,6 +371,7 @@ int launch_inv_counts(const int32_t* counts, long long G, double* inv_counts, cu
 // mu is G x C; p is written at the padded stride pld (its padding is left untouched).
 template <typename T>
 int launch_cg_init(long long Gt, int C, const int32_t* counts, const double* mu, T* r, T* z, T* p, int pld, T* x,
-                   double* rz_partials, double* zmax_partials, unsigned long long* zmax, cudaStream_t s);
+                   double* rz_partials, double* zmax_partials, unsigned long long* zmax, cudaStream_t s,
+                   bool fixed = false);
 
 }  // namespace fegb

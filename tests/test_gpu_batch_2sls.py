@@ -1,0 +1,73 @@
+"""Batches with 2SLS specifications close to unidentified: two endogenous
+regressors share one first stage, so the second stage's condition number reaches
+1e4 to 1e11 and a change of rounding anywhere before it (the order of the
+within-transform's or the Gram's additions) shows from the 7th digit on. The
+stacked form keeps one order of additions; its results are held to recorded ones
+(golden/batch_2sls.json, one GB300 run) at 1e-9 of each vector's norm."""
+import json
+import os
+
+import numpy as np
+import pytest
+
+from fe_gpu_gb300.estimator import DeviceBuffer, fe_batch_spec, fe_gpu_estimate_batch, fe_runtime_config
+
+pytestmark = pytest.mark.gpu
+
+GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "batch_2sls.json")
+SETS = [(0, 10), (0, 13), (1, 0)]
+
+
+def specifications(ordered, base):
+    """28 specifications of 2k to 60k rows, three quarters of them 2SLS; ordered: rows sorted by the first dimension, in
+    runs of equal ids."""
+    specs = []
+    for s in range(28):
+        r = np.random.RandomState(1000 * ordered + 100 * base + s)
+        n = int(np.exp(r.uniform(np.log(2_000), np.log(60_000))))
+        sizes = [max(2, int(c * n ** 0.7)) for c in r.uniform(0.2, 1.0, 2 + s % 2)]
+        k, endog = (2, 3, 6, 9, 14, 19, 22)[s % 7], 2 if s % 4 else 0
+        l = 2 + s % 2 if endog else 0
+        ids = [r.randint(0, m, n) for m in sizes]
+        if ordered:
+            at = np.sort(r.randint(0, sizes[0], n))
+            ids = [at, (at * 7 + np.arange(n) // 5 % 3) % sizes[1]] + ids[2:]
+        W, Z, u = r.normal(size=(k, n)), r.normal(size=(l, n)), r.normal(size=n)
+        for j in range(endog):
+            W[j] += 0.4 * u + np.linspace(0.4, 0.8, l) @ Z
+        y = u + np.linspace(-1.0, 1.0, k) @ W
+        for i, m in zip(ids, sizes):
+            y += (0.3 * r.normal(size=m))[i]
+        specs.append(dict(y=y, W=W, Z=Z, ids=[(i + 1).astype(np.int32) for i in ids], endog=list(range(1, endog + 1)),
+                          clusters=list(range(1, 1 + s % (len(sizes) + 1)))))
+    return specs
+
+
+def fits(specs, **cfg):
+    keep, rows = [], []
+    for s in specs:
+        b = [DeviceBuffer.from_array(np.ascontiguousarray(v)) for v in [s["y"], s["W"]] + s["ids"]]
+        z = DeviceBuffer.from_array(s["Z"]) if len(s["Z"]) else None
+        keep.append((b, z))
+        rows.append(fe_batch_spec(n=len(s["y"]), k=len(s["W"]), l=len(s["Z"]), d_y=b[0].ptr, d_W=b[1].ptr,
+                                  d_Z=z.ptr if z else None, d_fe_ids=[v.ptr for v in b[2:]],
+                                  cluster_fe_dims=s["clusters"], iv_regressors=s["endog"]))
+    return fe_gpu_estimate_batch(fe_runtime_config(fe_tolerance=1e-8, fe_max_iterations=20_000, precision="mixed",
+                                                   demean_cg=True, **cfg), rows)
+
+
+def off(a, b):
+    return np.linalg.norm(np.asarray(a) - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("ordered,base", SETS)
+def test_ill_conditioned_specifications_keep_their_results(built, ordered, base):
+    with open(GOLDEN) as f:
+        want = json.load(f)[SETS.index((ordered, base))]
+    got = fits(specifications(ordered, base))
+    assert len(got) == len(want)
+    for r, w in zip(got, want):
+        assert r.converged
+        for name in ("beta", "se"):
+            assert off(getattr(r, name), np.array([float.fromhex(v) for v in w[name]])) < 1e-9
+        assert abs(r.rss / float.fromhex(w["rss"]) - 1.0) < 1e-9
