@@ -924,6 +924,12 @@ __global__ void __launch_bounds__(AP_THREADS, 2) ap_star_kernel(const __grid_con
         for (int i = 0; i < ns; ++i)
             for (int e = threadIdx.x; e < p.s[i].G * C; e += AP_THREADS)
                 p.s[i].tab[(e / C) * p.s[i].ld + e % C] = tab[i][e];
+        for (int i = 0; i < ns; ++i)
+            for (int cc = threadIdx.x; cc < C; cc += AP_THREADS) {
+                unsigned long long m = 0;
+                for (int t = 0; t < p.s[i].G; ++t) m = umax64(m, abs_bits(tab[i][t * C + cc]));
+                p.s[i].amax[cc] = m;
+            }
         if (threadIdx.x == 0) {
             p.ctl->iterations = iter;
             p.ctl->max_update = bits_dbl(it_max);

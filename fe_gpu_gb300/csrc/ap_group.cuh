@@ -139,7 +139,7 @@ size_t ap_small_scratch(int Gs, int C, int n_src);
 struct ApStar {
     ApTables<double> w;          // the large dimension (amax: running column maxima, zeroed)
     int n_small;
-    ApTables<double> s[SWEEP_MAXP];        // small dimensions in sweep order
+    ApTables<double> s[SWEEP_MAXP];        // small dimensions in sweep order (amax: of the last tables)
     ApDense<double> sw[SWEEP_MAXP];        // counts of small i against the large dimension (Ge = w.G)
     ApDense<double> ss[SWEEP_MAXP][SWEEP_MAXP];  // counts of small i against small j (Ge = groups of j)
     unsigned long long* sums;    // AP_STAR_RING x ap_star_sums() words, zeroed

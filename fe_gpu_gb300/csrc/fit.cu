@@ -2272,7 +2272,23 @@ bool ap_on_groups(int C, int n_fe, long long n) { return C <= 32 && n_fe > 0 && 
 // 2^-53 of the largest mean, some 64 of them over the sums. While that is not far
 // below the tolerance (columns with a large level) the work stays on the rows,
 // whose level the first pass over them takes out.
+// The same holds for the increments: the means that are left are differences of
+// sums over them, uncertain by as much of the largest. Increments far above the
+// means (a few groups that hardly anything links to the rest) could leave means
+// above the tolerance on the rows where the tables say otherwise, so beyond this
+// bound the rows are looked at again.
 bool level_fits(double level, double tol) { return 64.0 * 0x1p-53 * level <= 1e-3 * tol; }
+
+// The largest finite of n maxima that are given as bits (a column with a value that
+// is not finite has no convergence to speak of, and is passed over elsewhere too).
+double largest_finite(const std::vector<unsigned long long>& bits) {
+    double m = 0.0;
+    for (unsigned long long b : bits) {
+        const double v = bits_to_double(b);
+        if (std::isfinite(v)) m = std::max(m, v);
+    }
+    return m;
+}
 
 // The group tables of an AP run in storage type T, with what they gather from.
 template <typename T>
@@ -2575,8 +2591,17 @@ struct ApGroups {
         return (double)a.w.G * P.C <= AP_STAR_ELEMENTS && ap_star_smem(a) <= AP_STAR_SMEM;
     }
 
-    int run_star(Problem& P, ApStar& a, int* iterations, double* max_update) {
+    // column maxima of the tables -> host, after the next synchronisation
+    int fetch_maxima(Problem& P, std::vector<unsigned long long>& h) {
+        h.resize((size_t)P.n_fe * P.C);
+        FEGB_CUDA(cudaMemcpyAsync(h.data(), amax, sizeof(h[0]) * h.size(), cudaMemcpyDeviceToHost, P.s),
+                  "table maxima copy");
+        return 0;
+    }
+
+    int run_star(Problem& P, ApStar& a, int* iterations, double* max_update, double* largest) {
         Scratch tmp(P.s);
+        std::vector<unsigned long long> maxima;
         const size_t words = ap_star_sums(a) * AP_STAR_RING + AP_STAR_RING + 1;
         unsigned long long* w = nullptr;
         FEGB_TRY(tmp.alloc(&w, words, "projection exchange"));
@@ -2589,18 +2614,21 @@ struct ApGroups {
         ApCtl last{};
         int bad = 0;
         FEGB_CUDA(cudaMemcpyAsync(&last, ctl, sizeof(last), cudaMemcpyDeviceToHost, P.s), "projection state copy");
+        FEGB_TRY(fetch_maxima(P, maxima));
         FEGB_TRY(d2h_sync(&bad, a.error, sizeof(bad), P.s, "projection error copy"));
         if (bad) return set_error("alternating projections: a barrier of the one-launch form ran out of time");
         *iterations = last.iterations;
         *max_update = last.max_update;
+        *largest = largest_finite(maxima);
         P.projections += 4 * P.n_fe * last.iterations;
         return 0;
     }
 
     // Iterations from the means mu_all (of the current rows) until the largest
     // update stays below tol; the relaxation state continues from P.relax,
-    // P.prev_change and the prev tables. Leaves the updates in alpha_all.
-    int run(Problem& P, double tol, int max_iter, int* iterations, double* max_update) {
+    // P.prev_change and the prev tables. Leaves the updates in alpha_all, the largest
+    // that a table held in *largest.
+    int run(Problem& P, double tol, int max_iter, int* iterations, double* max_update, double* largest) {
         const int C = P.C;
         FEGB_CUDA(cudaMemsetAsync(B.p, 0, sizeof(T) * (size_t)std::max(1LL, P.Gt) * B.ld, P.s), "group tables zero");
         FEGB_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (size_t)P.n_fe * C, P.s), "table maxima zero");
@@ -2617,7 +2645,7 @@ struct ApGroups {
         if constexpr (sizeof(T) == 8) {
             ApStar star;
             if (!P.profile && star_of(P, max_iter, &star)) {
-                FEGB_TRY(run_star(P, star, iterations, max_update));
+                FEGB_TRY(run_star(P, star, iterations, max_update, largest));
                 return launch_to_f64<double>(reinterpret_cast<const double*>(B.p), B.ld, P.alpha_all, C, P.Gt, P.s);
             }
         }
@@ -2637,7 +2665,10 @@ struct ApGroups {
                 last = poll.host[old];
             }
         }
+        std::vector<unsigned long long> maxima;
+        FEGB_TRY(fetch_maxima(P, maxima));
         FEGB_TRY(d2h_sync(&last, ctl, sizeof(last), P.s, "projection state copy"));
+        *largest = largest_finite(maxima);
         // projections of the iterations that ran
         if (queued > 0) P.projections = proj0 + (int)((long long)(P.projections - proj0) / queued * last.iterations);
         *iterations = last.iterations;
@@ -2660,8 +2691,9 @@ struct ApGroups {
     }
 
     // Takes the increments alpha_all out of the residual: mu_all becomes the
-    // means of what is left; their largest -> *mu_max.
-    int refine_step(Problem& P, double* mu_max) {
+    // means of what is left; their largest -> *mu_max, the largest increment ->
+    // *largest.
+    int refine_step(Problem& P, double* mu_max, double* largest) {
         const int C = P.C;
         FEGB_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (size_t)P.n_fe * C, P.s), "table maxima zero");
         FEGB_CUDA(cudaMemsetAsync(slots, 0, sizeof(ApSlot) * (size_t)P.n_fe * AP_SLOTS, P.s), "refinement slots");
@@ -2674,10 +2706,13 @@ struct ApGroups {
         for (int d = 0; d < P.n_fe; ++d) FEGB_TRY(visit(P, d, 0, 1));
         P.projections = proj;
         std::vector<ApSlot> h((size_t)P.n_fe * AP_SLOTS);
+        std::vector<unsigned long long> maxima;
+        FEGB_TRY(fetch_maxima(P, maxima));
         FEGB_TRY(d2h_sync(h.data(), slots, sizeof(ApSlot) * h.size(), P.s, "refinement maxima copy"));
         double m = 0.0;
         for (int d = 0; d < P.n_fe; ++d) m = std::max(m, bits_to_double(h[(size_t)d * AP_SLOTS].change));
         *mu_max = m;
+        *largest = largest_finite(maxima);
         return 0;
     }
 
@@ -2693,14 +2728,23 @@ struct ApGroups {
 
 // The FP64 refinement around an inner solve: group means of the residual, on the
 // rows at first and, once their level allows it (level_fits), on FP64 group
-// tables; there the rows are read once and written once, whatever the rounds.
+// tables; there the rows are read once and written once, whatever the rounds. A
+// round whose increments are too large for the tables' means goes back to the rows.
 struct Refinement {
     ApGroups<double> A;
     bool possible = false, on_tables = false;
+    bool taken = false;  // the tables hold increments that the rows do not
 
     // means of the residual after the increments alpha_all of the previous round (if any)
     int means(Problem& P, bool increments, double tol, double* mu) {
-        if (on_tables) return A.refine_step(P, mu);
+        if (on_tables) {
+            double largest = 0.0;
+            FEGB_TRY(A.refine_step(P, mu, &largest));
+            taken = true;
+            if (level_fits(largest, tol)) return 0;
+            FEGB_TRY(finish(P));
+            increments = false;
+        }
         FEGB_TRY(fp64_mean_pass(P, increments, mu));
         if (possible && level_fits(*mu, tol)) {
             on_tables = true;
@@ -2708,7 +2752,11 @@ struct Refinement {
         }
         return 0;
     }
-    int finish(Problem& P, bool increments) { return on_tables && increments ? A.refine_finish(P) : 0; }
+    int finish(Problem& P) {
+        if (on_tables && taken) FEGB_TRY(A.refine_finish(P));
+        on_tables = taken = false;
+        return 0;
+    }
 };
 
 // FP64 refinement loop around a CG inner solve in storage type T.
@@ -2763,7 +2811,7 @@ int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* conver
         total += it;
         apply_alpha = true;
     }
-    FEGB_TRY(R.finish(P, apply_alpha));
+    FEGB_TRY(R.finish(P));
     if (sizeof(T) == 4 && B.any_dense) {
         // the tensor-core count-matrix passes record a wait that ran out of time
         int umma_err = 0;
@@ -2791,18 +2839,31 @@ int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* con
     if (ap_on_groups(P.C, P.n_fe, P.n)) {
         ApGroups<double> A;
         FEGB_TRY(A.build(P));
-        while (iter < max_iter && iter <= AP_ROW_ITERATIONS) {
+        int on_rows = 0;
+        bool again = false;  // the tables converged on increments too large for them
+        while (iter < max_iter || again) {
             double level = 0.0;
             FEGB_TRY(fp64_mean_pass(P, false, &level));
+            if (again && level < tol) {
+                hit = 1;
+                break;
+            }
+            if (iter == max_iter) break;
             if (level_fits(level, tol)) {
                 int it = 0;
-                FEGB_TRY(A.run(P, tol, max_iter - iter, &it, &mu));
+                double largest = 0.0;
+                FEGB_TRY(A.run(P, tol, max_iter - iter, &it, &mu, &largest));
                 FEGB_TRY(apply_alpha_rows(P));
-                *iterations = iter + it;
+                iter += it;
+                again = mu < tol && !level_fits(largest, tol);
+                if (again) continue;
+                *iterations = iter;
                 *converged = mu < tol;
                 *max_update = mu;
                 return 0;
             }
+            again = false;
+            if (on_rows++ == AP_ROW_ITERATIONS) break;
             FEGB_TRY(order_deferred_rows(P));
             FEGB_TRY(ap_iteration<double>(P, P.X, pl, o, &mu));
             ++iter;
@@ -2888,15 +2949,15 @@ int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* con
         FEGB_TRY(reset_ap_state(P, true));
         const double inner_tol = std::max(0.25 * tol, 1e-5 * mu);
         int it = 0;
-        double upd = 0.0;
+        double upd = 0.0, largest = 0.0;
         if (groups)
-            FEGB_TRY(A.run(P, inner_tol, max_iter - total_iter, &it, &upd));
+            FEGB_TRY(A.run(P, inner_tol, max_iter - total_iter, &it, &upd, &largest));
         else
             FEGB_TRY(ap_solve_rows(P, inner_tol, max_iter - total_iter, &it));
         total_iter += it;
         apply_alpha = true;
     }
-    FEGB_TRY(R.finish(P, apply_alpha));
+    FEGB_TRY(R.finish(P));
     *iterations = total_iter;
     *converged = hit;
     *max_update = mu;
