@@ -456,12 +456,17 @@ std::vector<char> cg_dense_plan(const std::vector<int>& G, int C, long long n) {
     return dense;
 }
 
-// flags[i] = 1 where the pair (ga, gb) changes along an ordered list of rows
-__global__ void pair_flags_kernel(const int32_t* __restrict__ ga, const int32_t* __restrict__ gb, long long n,
+// Row counts of runs and tuples are FP32 weights, exact up to this many rows
+constexpr int WEIGHT_ROWS = 1 << 24;
+
+// flags[i] = 1 where the pair (ga, gb) changes along an ordered list of rows, and
+// every `cut` positions (0: nowhere else)
+__global__ void pair_flags_kernel(const int32_t* __restrict__ ga, const int32_t* __restrict__ gb, long long n, int cut,
                                   uint32_t* __restrict__ flags) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long st = (long long)gridDim.x * blockDim.x;
-    for (; i < n; i += st) flags[i] = (i == 0 || ga[i] != ga[i - 1] || gb[i] != gb[i - 1]) ? 1u : 0u;
+    for (; i < n; i += st)
+        flags[i] = (i == 0 || ga[i] != ga[i - 1] || gb[i] != gb[i - 1] || (cut && i % cut == 0)) ? 1u : 0u;
 }
 
 // rank[i] = the run of position i; off[run] = its first position
@@ -501,7 +506,8 @@ __global__ void run_counts_kernel(const int32_t* __restrict__ gid, const int32_t
 // Runs of the primary and dimension e over the storage order (Problem::runs),
 // taken as the tuples of the operator when they are at most three quarters of the
 // rows and at most a quarter more than the distinct pairs (rows of a primary
-// group in no order of e would give many runs for one pair). What remains is
+// group in no order of e would give many runs for one pair). A run ends at the
+// latest after WEIGHT_ROWS rows. What remains is
 // sorted run by run: the rows themselves are neither sorted by e nor gathered in
 // that order (150M rows, 12M runs: 10 digit passes of 4 ms over the rows become
 // three of 0.4 ms over the runs; preparation 27.6 -> 11.9 ms).
@@ -515,7 +521,7 @@ int build_runs(Problem& P, int e) {
     FEGB_TRY(tmp.alloc(&flags, (size_t)n, "run flags"));
     FEGB_TRY(tmp.alloc(&excl, (size_t)n, "run scan"));
     FEGB_TRY(tmp.alloc(&total, 1, "run count"));
-    pair_flags_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(gw, ge, n, flags);
+    pair_flags_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(gw, ge, n, WEIGHT_ROWS, flags);
     FEGB_LAUNCH_CHECK("run flags");
     FEGB_TRY(scan_exclusive_u32(flags, excl, n, total, s, tmp));
     uint32_t hm = 0;
@@ -547,7 +553,8 @@ int build_runs(Problem& P, int e) {
     int32_t *pgs = nullptr, *pof = nullptr;
     FEGB_TRY(dalloc(scr, &pgs, (size_t)m, "pair ranks"));
     FEGB_TRY(dalloc(scr, &pof, (size_t)m + 1, "pair offsets"));
-    pair_flags_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(reinterpret_cast<const int32_t*>(sorted), wj, m, flags);
+    pair_flags_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(reinterpret_cast<const int32_t*>(sorted), wj, m, 0,
+                                                                 flags);
     FEGB_LAUNCH_CHECK("pair flags");
     FEGB_TRY(scan_exclusive_u32(flags, excl, m, total, s, tmp));
     run_ranks_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(flags, excl, m, pof, pgs);
@@ -1385,7 +1392,8 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
             FEGB_TRY(tmp.alloc(&flags, (size_t)n, "pair run flags"));
             FEGB_TRY(tmp.alloc(&excl, (size_t)n, "pair run scan"));
             FEGB_TRY(tmp.alloc(&total, 1, "pair run count"));
-            pair_flags_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(E->gseq, E->gid_at_perm[P.primary], n, flags);
+            pair_flags_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(E->gseq, E->gid_at_perm[P.primary], n, 0,
+                                                                         flags);
             FEGB_LAUNCH_CHECK("pair run flags");
             FEGB_TRY(scan_exclusive_u32(flags, excl, n, total, s, tmp));
             run_ranks_kernel<<<grid_stride_blocks(n, 256), 256, 0, s>>>(flags, excl, n, toff, tseq);
@@ -1411,6 +1419,11 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
             P.tuple_n = n;
         }
         if (m <= 0 || (double)m > 0.75 * (double)n) return 0;
+        if (n > WEIGHT_ROWS) {  // a weight that FP32 does not hold: the rows themselves
+            int longest = 0;
+            FEGB_TRY(max_group_length(toff, m, &longest, s));
+            if (longest > WEIGHT_ROWS) return 0;
+        }
         std::vector<int32_t*> tg(sw.size());
         for (size_t j = 0; j < sw.size(); ++j) FEGB_TRY(dalloc(scr, &tg[j], (size_t)m, "tuple ids"));
         float* w = nullptr;
