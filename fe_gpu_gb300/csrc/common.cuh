@@ -88,6 +88,11 @@ class Scratch {
         for (void* p : ptrs_) cudaFreeAsync(p, stream_);
         ptrs_.clear();
     }
+    // takes over what `other` (of the same stream) holds
+    void adopt(Scratch& other) {
+        ptrs_.insert(ptrs_.end(), other.ptrs_.begin(), other.ptrs_.end());
+        other.ptrs_.clear();
+    }
     cudaStream_t stream() const { return stream_; }
 
   private:

@@ -503,6 +503,25 @@ __global__ void run_counts_kernel(const int32_t* __restrict__ gid, const int32_t
     for (; i < m; i += st) atomicAdd(counts + gid[i], off[i + 1] - off[i]);  // integer: order-free
 }
 
+// *count += runs whose pair occurs among the RUN_LOOKBACK runs before them
+constexpr int RUN_LOOKBACK = 16;
+__global__ void __launch_bounds__(256) run_returns_kernel(const int32_t* __restrict__ tw, const int32_t* __restrict__ te,
+                                                          long long m, uint32_t* __restrict__ count) {
+    long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    unsigned mine = 0;
+    for (; k < m; k += st) {
+        const int w = tw[k], e = te[k];
+        for (long long j = k - 1; j >= 0 && k - j <= RUN_LOOKBACK && tw[j] == w; --j)
+            if (te[j] == e) {
+                ++mine;
+                break;
+            }
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, mine);
+}
+
 // Runs of the primary and dimension e over the storage order (Problem::runs),
 // taken as the tuples of the operator when they are at most three quarters of the
 // rows and at most a quarter more than the distinct pairs (rows of a primary
@@ -512,11 +531,10 @@ __global__ void run_counts_kernel(const int32_t* __restrict__ gid, const int32_t
 // that order (150M rows, 12M runs: 10 digit passes of 4 ms over the rows become
 // three of 0.4 ms over the runs; preparation 27.6 -> 11.9 ms).
 int build_runs(Problem& P, int e) {
-    Scratch& scr = *P.scr;
     cudaStream_t s = P.s;
     const long long n = P.n;
     const int32_t *gw = P.dims[P.primary].gid, *ge = P.dims[e].gid;
-    Scratch tmp(s);
+    Scratch tmp(s), scr(s);  // scr: what stays when the runs are taken
     uint32_t *flags = nullptr, *excl = nullptr, *total = nullptr;
     FEGB_TRY(tmp.alloc(&flags, (size_t)n, "run flags"));
     FEGB_TRY(tmp.alloc(&excl, (size_t)n, "run scan"));
@@ -542,6 +560,13 @@ int build_runs(Problem& P, int e) {
     FEGB_TRY(dalloc(scr, &w, (size_t)m, "run lengths"));
     run_build_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(off, m, gw, ge, tw, te, w);
     FEGB_LAUNCH_CHECK("run ids");
+    // runs that return to a pair within RUN_LOOKBACK runs: with many of them the
+    // pairs are too few whatever the sort would say
+    FEGB_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), s), "run returns");
+    run_returns_kernel<<<grid_stride_blocks(m, 256), 256, 0, s>>>(tw, te, m, total);
+    FEGB_LAUNCH_CHECK("run returns");
+    FEGB_TRY(d2h_sync(&hm, total, sizeof(hm), s, "run returns copy"));
+    if ((double)m > 1.25 * (double)(m - (int)hm)) return 0;
     FEGB_TRY(dalloc(scr, &sorted, (size_t)m, "run order ids"));
     FEGB_TRY(dalloc(scr, &order, (size_t)m, "run order"));
     FEGB_TRY(radix_sort_u32(reinterpret_cast<const uint32_t*>(te), nullptr, sorted, order, m,
@@ -564,6 +589,7 @@ int build_runs(Problem& P, int e) {
     if ((double)m > 1.25 * (double)mp) return 0;
     const int32_t m32 = m;
     FEGB_TRY(h2d_sync(pof + mp, &m32, sizeof(m32), s, "pair end"));
+    P.scr->adopt(scr);
     P.runs = true;
     P.run_dim = e;
     P.run_sorted = reinterpret_cast<const int32_t*>(sorted);
