@@ -128,6 +128,7 @@ struct Problem {
     // 4,096-row blocks, sixteen vector steps, row streams sorted by group and the
     // refinement on the rows.
     bool stacked = false;
+    bool padded_counts = false;  // the count matrices are the group tables' (projections), not the CG operator's
     // the CG operator's row sort by distinct id tuples of its swept dimensions
     // (positions grouped by tuple), kept for the cluster subset over the same
     // dimensions: tuple t holds sorted positions tuple_off[t] .. tuple_off[t+1]
@@ -440,18 +441,22 @@ double bits_to_double(unsigned long long b) {
 // ---------------------------- preparation ---------------------------------
 
 // Builds the storage-order problem from device inputs in the reference layout.
+constexpr double COUNT_BYTES = 8e9;  // most for the count matrices, and for padded copies of them
+
 // Dimensions the CG operator handles through dense count matrices: at most
 // DENSE_SMALL_MAX_G groups, C <= 32, and all matrices together within 8 GB at
 // uint32 counts. Such a dimension needs no row sort of its own.
-std::vector<char> cg_dense_plan(const std::vector<int>& G, int C, long long n) {
+// padded: with the rows of ap_count_pitch counts that the group tables read (up to
+// sixteen times as wide).
+std::vector<char> cg_dense_plan(const std::vector<int>& G, int C, long long n, bool padded) {
     std::vector<char> dense(G.size(), 0);
     if (C > 32 || n <= 0) return dense;
     double bytes = 0.0;  // worst case: uint32 counts
     for (size_t d = 0; d < G.size(); ++d)
         if (G[d] > 0 && G[d] <= DENSE_SMALL_MAX_G)
             for (size_t e = 0; e < G.size(); ++e)
-                if (e != d) bytes += 4.0 * std::max(1, G[e]) * G[d];
-    if (bytes > 8e9) return dense;
+                if (e != d) bytes += 4.0 * std::max(1, G[e]) * (padded ? ap_count_pitch(G[d]) : G[d]);
+    if (bytes > COUNT_BYTES) return dense;
     for (size_t d = 0; d < G.size(); ++d) dense[d] = G[d] > 0 && G[d] <= DENSE_SMALL_MAX_G;
     return dense;
 }
@@ -760,7 +765,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     // the CG operator sweeps every dimension it does not handle densely
     std::vector<char> cg_sorted(n_fe, 0);
     if (sorted_all) {
-        const std::vector<char> dense = cg_dense_plan(G, C, n);
+        const std::vector<char> dense = cg_dense_plan(G, C, n, P.padded_counts);
         for (int d = 0; d < n_fe; ++d) cg_sorted[d] = d != P.primary && !dense[d];
     }
     for (int d = 0; d < n_fe; ++d) {
@@ -779,7 +784,7 @@ int build_problem(Problem& P, long long n_in, int k, int l, int n_fe, const doub
     // rows that come in the primary's order, and one other swept dimension: its
     // runs may serve instead of its row order
     if (sorted_all && in_primary_order && n >= 4096 && !P.stacked) {
-        const std::vector<char> dense = cg_dense_plan(G, C, n);
+        const std::vector<char> dense = cg_dense_plan(G, C, n, P.padded_counts);
         int other = -1, swept = 0;
         for (int d = 0; d < n_fe; ++d)
             if (!dense[d] && G[d] > 0) {
@@ -1749,7 +1754,7 @@ int cg_alloc(Problem& P, CGBuffers<T>& B) {
     B.dsum_off.assign(P.n_fe, 0);
     std::vector<int> Gd(P.n_fe);
     for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
-    const std::vector<char> plan = cg_dense_plan(Gd, C, P.n);
+    const std::vector<char> plan = cg_dense_plan(Gd, C, P.n, P.padded_counts);
     if (std::find(plan.begin(), plan.end(), 1) != plan.end()) {
         {
             long long parts = 0, sums = 0;
@@ -2362,7 +2367,7 @@ struct ApGroups {
         B.N32.assign(P.n_fe, std::vector<uint32_t*>(P.n_fe, nullptr));
         std::vector<int> Gd(P.n_fe);
         for (int d = 0; d < P.n_fe; ++d) Gd[d] = P.dims[d].G;
-        const std::vector<char> plan = cg_dense_plan(Gd, C, P.n);
+        const std::vector<char> plan = cg_dense_plan(Gd, C, P.n, P.padded_counts);
         unsigned* mx = nullptr;
         FEGB_TRY(dalloc(scr, &mx, 1, "count max"));
         for (int d = 0; d < P.n_fe; ++d) {
@@ -2375,6 +2380,19 @@ struct ApGroups {
         FEGB_TRY(operator_streams(P, B));
         FEGB_TRY(alloc(P));
         return poll.open();
+    }
+
+    // Whether padded copies of a CG operator's count rows stay within bounds.
+    template <typename S>
+    static bool adoptable(const Problem& P, const CGBuffers<S>& O) {
+        double bytes = 0.0;
+        for (int d = 0; d < P.n_fe; ++d)
+            for (int e = 0; e < P.n_fe; ++e) {
+                const int pitch = ap_count_pitch(P.dims[d].G);
+                if (pitch != P.dims[d].G && (O.N8[d][e] || O.N32[d][e]))
+                    bytes += (O.N8[d][e] ? 1.0 : 4.0) * P.dims[e].G * pitch;
+            }
+        return bytes <= COUNT_BYTES;
     }
 
     // The couplings of a CG operator (count rows without padding).
@@ -2819,7 +2837,7 @@ int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* conver
         }
     }
     Refinement R;
-    if (ap_on_groups(P.C, P.n_fe, P.n) && !P.stacked) {
+    if (ap_on_groups(P.C, P.n_fe, P.n) && !P.stacked && R.A.adoptable(P, B)) {
         FEGB_TRY(R.A.adopt(P, B));
         R.possible = true;
     }
@@ -3745,6 +3763,7 @@ int estimate_device_impl(const fegb_config* cfg_in, long long n, int k, int l, i
     P.scr = &scr;
     P.profile = cfg.profile != 0;
     P.data_ready = data_ready;
+    P.padded_counts = cfg.demean_method == FEGB_DEMEAN_AP;
     FitTimes tm;
     auto t0 = Clock::now();
     long long n_single = 0;
@@ -3886,6 +3905,7 @@ int within_impl(const fegb_config& cfg, long long n, int k, int l, int n_fe, dou
     P.scr = &scr;
     P.profile = cfg.profile != 0;
     P.stacked = stacked;
+    P.padded_counts = cfg.demean_method == FEGB_DEMEAN_AP;
     long long n_single = 0;
     FEGB_TRY(build_problem(P, n, k, l, n_fe, d_y, d_W, d_Z, ids, group_sizes, false,
                            ap_needs_rows(cfg, 1 + k + l, n_fe, n), &n_single,
@@ -4369,6 +4389,15 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
 using namespace fegb;
 
 extern "C" {
+
+int fegb_test_dense_plan(const int* group_counts, int n_fe, int C, long long n, int padded, int* dense) {
+    using namespace fegb;
+    if (!group_counts || !dense || n_fe < 1) return set_error("fegb_test_dense_plan: invalid sizes");
+    const std::vector<char> plan = cg_dense_plan({group_counts, group_counts + n_fe}, C, n, padded != 0);
+    for (int d = 0; d < n_fe; ++d) dense[d] = plan[d];
+    return set_ok();
+}
+
 
 void fegb_config_init(fegb_config* cfg) {
     if (!cfg) return;

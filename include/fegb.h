@@ -205,6 +205,11 @@ int fegb_test_group_sums(const double* X, long long n, int C, const int* gid, in
  * form (FP64 values as eight digits, exact digit products); 0: the FP64 form. */
 int fegb_test_gram(const double* X, long long n, int a, int split, double* out);
 
+/* Self-test of the rule behind the count matrices: dense[d] = 1 when dimension d
+ * of a problem of n rows, C columns and these group counts is held as count
+ * matrices (padded = 1: those of the group tables), else 0. No GPU needed. */
+int fegb_test_dense_plan(const int* group_counts, int n_fe, int C, long long n, int padded, int* dense);
+
 /* FE reconstruction of --save-fe (reconstruct_and_save_fixed_effects,
  * src/core/fe_pipeline.f90:1619-1733): forward Gauss-Seidel sweeps of the
  * residual y - W beta (beta: host, k values), dimension by dimension, each
