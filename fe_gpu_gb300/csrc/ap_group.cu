@@ -1,5 +1,6 @@
 // Alternating projections on group tables (see ap_group.cuh).
 #include "ap_group.cuh"
+#include "umma.cuh"
 
 #include <algorithm>
 
@@ -622,27 +623,31 @@ __global__ void __launch_bounds__(AP_THREADS, sizeof(T) == 8 && GT > AP_PART ? 1
 // ------------------------ one large dimension, small others ------------------------
 
 // Barrier of all blocks of a cooperative launch, the n-th one. Bounded: after
-// about a second of waiting the error word is set and every block leaves.
-__device__ __forceinline__ bool star_barrier(const ApStar& p, unsigned n, int* s_bad) {
+// p.wait_ns of waiting the error word is set and every block leaves.
+__device__ __forceinline__ bool star_barrier(const ApStar& p, unsigned long long n, int* s_bad) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        const unsigned target = n * gridDim.x;
-        atomicAdd(p.arrived, 1u);
-        volatile unsigned* a = p.arrived;
+        const unsigned long long target = n * gridDim.x;
+        atomicAdd(p.arrived, 1ULL);
+        volatile unsigned long long* a = p.arrived;
         volatile int* e = p.error;
         int bad = 0;
-        for (long long spin = 0; *a < target; ++spin) {
-            if ((spin & 1023) == 1023 && *e) {
+        unsigned long long t0 = 0;  // from the 64th poll on (a limit of zero: the first)
+        for (unsigned spin = 0; *a < target; ++spin) {
+            if (spin < 64 && p.wait_ns) continue;
+            if (*e) {
                 bad = 1;
                 break;
             }
-            if (spin > (1LL << 23)) {
+            const unsigned long long now = globaltimer();
+            if (t0 == 0) t0 = now;
+            if (now - t0 >= p.wait_ns) {
                 *e = 1;
                 bad = 1;
                 break;
             }
-            if (spin > 64) __nanosleep(64);
+            __nanosleep(64);
         }
         __threadfence();
         *s_bad = bad;
@@ -726,7 +731,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) ap_star_kernel(const __grid_con
     while (top < slots) top <<= 1;
     top >>= 1;
     unsigned long long it_max = 0;  // largest update of the iteration
-    unsigned barrier = 0;
+    unsigned long long barrier = 0;
     int turn = 0;     // projections of w so far (ring of change)
     int visit = 0;    // visits of w so far (ring of sums)
     int iter = 0;

@@ -144,7 +144,8 @@ struct ApStar {
     ApDense<double> ss[SWEEP_MAXP][SWEEP_MAXP];  // counts of small i against small j (Ge = groups of j)
     unsigned long long* sums;    // AP_STAR_RING x ap_star_sums() words, zeroed
     unsigned long long* change;  // AP_STAR_RING words, zeroed: largest update of a projection of w
-    unsigned* arrived;           // zeroed: the barrier's count
+    unsigned long long* arrived;  // zeroed: the barrier's count
+    unsigned long long wait_ns;  // limit of a wait at the barrier
     int* error;                  // zeroed: a barrier ran out of time
     ApCtl* ctl;                  // tol in; iterations, max_update, stop out
     const double* relax;         // starting relaxation and last change of the small dimensions, then of w

@@ -2334,6 +2334,11 @@ double largest_finite(const std::vector<unsigned long long>& bits) {
     return m;
 }
 
+// Limit of a wait at the barrier of the one-launch projections (2 s; another for
+// the calling thread's fits by fegb_test_projection_wait).
+constexpr unsigned long long STAR_WAIT_NS = 2000000000ull;
+thread_local unsigned long long star_wait_ns = STAR_WAIT_NS;
+
 // The group tables of an AP run in storage type T, with what they gather from.
 template <typename T>
 struct ApGroups {
@@ -2659,14 +2664,15 @@ struct ApGroups {
     int run_star(Problem& P, ApStar& a, int* iterations, double* max_update, double* largest) {
         Scratch tmp(P.s);
         std::vector<unsigned long long> maxima;
-        const size_t words = ap_star_sums(a) * AP_STAR_RING + AP_STAR_RING + 1;
+        const size_t words = ap_star_sums(a) * AP_STAR_RING + AP_STAR_RING + 2;
         unsigned long long* w = nullptr;
         FEGB_TRY(tmp.alloc(&w, words, "projection exchange"));
         FEGB_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long) * words, P.s), "projection exchange zero");
         a.change = w;
-        a.arrived = reinterpret_cast<unsigned*>(w + AP_STAR_RING);
+        a.arrived = w + AP_STAR_RING;
         a.error = reinterpret_cast<int*>(a.arrived + 1);
-        a.sums = w + AP_STAR_RING + 1;
+        a.sums = w + AP_STAR_RING + 2;
+        a.wait_ns = star_wait_ns;
         FEGB_TRY(launch_ap_star(a, P.s));
         ApCtl last{};
         int bad = 0;
@@ -4389,6 +4395,11 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
 using namespace fegb;
 
 extern "C" {
+
+int fegb_test_projection_wait(long long ns) {
+    fegb::star_wait_ns = ns < 0 ? fegb::STAR_WAIT_NS : (unsigned long long)ns;
+    return fegb::set_ok();
+}
 
 int fegb_test_dense_plan(const int* group_counts, int n_fe, int C, long long n, int padded, int* dense) {
     using namespace fegb;

@@ -210,6 +210,11 @@ int fegb_test_gram(const double* X, long long n, int a, int split, double* out);
  * matrices (padded = 1: those of the group tables), else 0. No GPU needed. */
 int fegb_test_dense_plan(const int* group_counts, int n_fe, int C, long long n, int padded, int* dense);
 
+/* Self-test of the bounded wait of the one-launch projections: the limit in
+ * nanoseconds for the fits of the calling thread (0: a wait gives up at once and
+ * the fit returns an error; negative: the default). */
+int fegb_test_projection_wait(long long ns);
+
 /* FE reconstruction of --save-fe (reconstruct_and_save_fixed_effects,
  * src/core/fe_pipeline.f90:1619-1733): forward Gauss-Seidel sweeps of the
  * residual y - W beta (beta: host, k values), dimension by dimension, each
