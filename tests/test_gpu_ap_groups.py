@@ -104,3 +104,19 @@ def test_clean_columns_converge_beside_a_non_finite_one(built, n, sizes, k, bad)
         out.append(host.W)
     # updates below 1e-10 at a rate of at most 0.9 an iteration (these panels converge in a few dozen) leave 1e-9 each
     np.testing.assert_allclose(out[1], out[0], atol=2e-9, rtol=0)
+
+
+@pytest.mark.parametrize("n,sizes,k", [c for c in CASES if len(c[1]) > 1 and c[0] < 1_000_000])
+@pytest.mark.parametrize("order", ["random", "sorted"])
+def test_mixed_form_reaches_the_fp64_limit(built, n, sizes, k, order):
+    y, W, fe = panel(n, sizes, k, seed=n + k, order=order)
+    out = []
+    for precision, tol in (("mixed", 1e-9), ("fp64", 1e-11)):
+        host = fe_host_arrays(y=y.copy(), W=W.copy(order="F"), Z=np.zeros((n, 0), order="F"), fe_ids=fe)
+        cfg = fe_runtime_config(fe_tolerance=tol, fe_max_iterations=2000, precision=precision)
+        conv, _, _ = fe_gpu_within_transform(cfg, host)
+        assert conv
+        out.append(np.column_stack([host.y, host.W]))
+    # means below 1e-9 in every dimension; the projection on these panels' dimensions (a few dozen iterations)
+    # is at most 20 times the largest mean of each of up to four
+    np.testing.assert_allclose(out[0], out[1], atol=8e-8, rtol=0)
