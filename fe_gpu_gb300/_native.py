@@ -211,6 +211,7 @@ SIGNATURES = {
     "fegb_test_dense_pair": (_I, [_P, _LL, _I, _P, _P, _I, _I, _P, _P, _I, _I, _P, _P, _P]),
     "fegb_test_group_sums": (_I, [_P, _LL, _I, _P, _I, _I, _P]),
     "fegb_test_gram": (_I, [_P, _LL, _I, _I, _P]),
+    "fegb_test_fail_alloc": (_I, [C.c_char_p, _I]),
     "fegb_test_projection_wait": (_I, [_LL]),
     "fegb_test_dense_plan": (_I, [_IP, _I, _I, _LL, _I, _IP]),
     "fegb_reconstruct_fe": (_I, [C.POINTER(FegbConfig), _LL, _I, _I, _P, _P, _DP, C.POINTER(C.c_void_p), _IP, _DP,

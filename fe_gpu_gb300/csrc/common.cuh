@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -62,6 +63,18 @@ inline unsigned grid_stride_blocks(long long n, int threads) {
 // ---------------------------------------------------------------------------
 // Stream-ordered scratch: a list of cudaMallocAsync blocks freed together.
 // ---------------------------------------------------------------------------
+// Self-test of what happens when memory runs out: the next `left` allocations with
+// this label fail. Set for the calling thread (fegb_test_fail_alloc); the threads
+// of a batch share their caller's.
+struct AllocFailure {
+    const char* what;
+    std::atomic<int> left;
+};
+extern thread_local AllocFailure* alloc_failure;
+inline bool alloc_fails(const char* what) {
+    return alloc_failure && std::strcmp(alloc_failure->what, what) == 0 && alloc_failure->left.fetch_sub(1) > 0;
+}
+
 class Scratch {
   public:
     explicit Scratch(cudaStream_t s) : stream_(s) {}
@@ -75,7 +88,7 @@ class Scratch {
         size_t bytes = count * sizeof(T);
         if (bytes == 0) bytes = 16;
         bytes = (bytes + 255) & ~size_t(255);
-        cudaError_t e = cudaMallocAsync(&p, bytes, stream_);
+        cudaError_t e = alloc_fails(what) ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, stream_);
         if (e != cudaSuccess) {
             *out = nullptr;
             return set_cuda_error(e, what);

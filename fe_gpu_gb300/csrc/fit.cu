@@ -2334,6 +2334,45 @@ double largest_finite(const std::vector<unsigned long long>& bits) {
     return m;
 }
 
+// Runs build() with a scratch of its own. Its memory stays with the fit, or goes
+// back when there is too little of it: then *built is false and the fit goes on
+// without the tables, as it could before there were any.
+template <typename F>
+int build_if_room(Problem& P, bool* built, F build) {
+    Scratch own(P.s);
+    Scratch* const fit = P.scr;
+    P.scr = &own;
+    const int rc = build();
+    P.scr = fit;
+    *built = rc == 0;
+    if (rc == 0)
+        fit->adopt(own);
+    else if (rc == (int)cudaErrorMemoryAllocation) {
+        own.release();
+        cudaGetLastError();
+        return set_ok();
+    }
+    return rc;
+}
+
+// Row sweeps after a build that ran out of memory: no tuples, the row orders.
+int back_to_rows(Problem& P) {
+    P.tuple_dims.clear();
+    P.tuple_gid.clear();
+    P.tuple_perm = P.tuple_off = P.tuple_gseq = nullptr;
+    P.tuple_m = 0;
+    P.tuple_n = 0;
+    P.row_tuple = nullptr;
+    P.tuple_sw.clear();
+    P.tuple_ids.clear();
+    P.tuple_dim_order.clear();
+    P.tuple_dim_gseq.clear();
+    P.tuple_dim_off.clear();
+    P.inc_tab = nullptr;
+    P.runs = false;
+    return order_deferred_rows(P);
+}
+
 // Limit of a wait at the barrier of the one-launch projections (2 s; another for
 // the calling thread's fits by fegb_test_projection_wait).
 constexpr unsigned long long STAR_WAIT_NS = 2000000000ull;
@@ -2428,6 +2467,7 @@ struct ApGroups {
         B.N8 = O.N8;
         B.N32 = O.N32;
         B.stream = O.stream;
+        FEGB_TRY(dalloc(*P.scr, &total, (size_t)std::max(1LL, P.Gt) * P.C, "increments taken out"));
         return alloc(P);
     }
 
@@ -2746,7 +2786,6 @@ struct ApGroups {
     // mu_all holds the means of the rows; nothing taken out yet.
     int refine_start(Problem& P) {
         refine = true;
-        if (!total) FEGB_TRY(dalloc(*P.scr, &total, (size_t)std::max(1LL, P.Gt) * P.C, "increments taken out"));
         FEGB_CUDA(cudaMemsetAsync(total, 0, sizeof(double) * (size_t)std::max(1LL, P.Gt) * P.C, P.s),
                   "increments zero");
         FEGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ApCtl), P.s), "refinement state");
@@ -2843,10 +2882,8 @@ int demean_cg(Problem& P, double tol, int max_iter, int* iterations, int* conver
         }
     }
     Refinement R;
-    if (ap_on_groups(P.C, P.n_fe, P.n) && !P.stacked && R.A.adoptable(P, B)) {
-        FEGB_TRY(R.A.adopt(P, B));
-        R.possible = true;
-    }
+    if (ap_on_groups(P.C, P.n_fe, P.n) && !P.stacked && R.A.adoptable(P, B))
+        FEGB_TRY(build_if_room(P, &R.possible, [&] { return R.A.adopt(P, B); }));
     const int max_outer = 12;
     double mu = 0.0, mu_prev = DBL_MAX;
     int total = 0, hit = 0;
@@ -2901,10 +2938,12 @@ int demean_plain(Problem& P, double tol, int max_iter, int* iterations, int* con
     int iter = 0;
     if (ap_on_groups(P.C, P.n_fe, P.n)) {
         ApGroups<double> A;
-        FEGB_TRY(A.build(P));
+        bool tables = false;
+        FEGB_TRY(build_if_room(P, &tables, [&] { return A.build(P); }));
+        if (!tables) FEGB_TRY(back_to_rows(P));
         int on_rows = 0;
         bool again = false;  // the tables converged on increments too large for them
-        while (iter < max_iter || again) {
+        while (tables && (iter < max_iter || again)) {
             double level = 0.0;
             FEGB_TRY(fp64_mean_pass(P, false, &level));
             if (again && level < tol) {
@@ -2991,13 +3030,21 @@ int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* con
     int total_iter = 0;
     bool apply_alpha = false;
     int hit = 0;
-    const bool groups = ap_on_groups(P.C, P.n_fe, P.n);
+    bool groups = ap_on_groups(P.C, P.n_fe, P.n);
     ApGroups<float> A;
     Refinement R;
     if (groups) {
-        FEGB_TRY(A.build(P));
-        FEGB_TRY(R.A.share(P, A.B));
-        R.possible = true;
+        FEGB_TRY(build_if_room(P, &groups, [&] {
+            FEGB_TRY(A.build(P));
+            return R.A.share(P, A.B);
+        }));
+        R.possible = groups;
+        if (!groups) {
+            FEGB_TRY(back_to_rows(P));
+            FEGB_TRY(dalloc(*P.scr, &P.Xc, (size_t)P.n * P.C, "correction block"));
+            for (Dim& D : P.dims)
+                FEGB_TRY(dalloc(*P.scr, &D.pend32, (size_t)std::max(1, D.G) * P.C, "pending means fp32"));
+        }
     }
     for (int round = 0; round < max_outer; ++round) {
         FEGB_TRY(R.means(P, apply_alpha, tol, &mu));
@@ -4343,7 +4390,10 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
     size_t next = 0;
     int running = 0;
     std::string message;
+    std::vector<size_t> again;  // classes that ran out of memory beside others: alone, afterwards
+    AllocFailure* const failure = alloc_failure;
     auto worker = [&]() {
+        alloc_failure = failure;
         cudaStream_t ws = nullptr;
         int err = 0;
         if (cudaSetDevice(dev) != cudaSuccess || cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking) != cudaSuccess ||
@@ -4356,7 +4406,7 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
                 room.wait(lk);
                 continue;
             }
-            ++next;
+            const size_t at = next++;
             ++running;
             in_use += c.bytes;
             lk.unlock();
@@ -4365,6 +4415,11 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
             lk.lock();
             --running;
             in_use -= c.bytes;
+            if (err == (int)cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                again.push_back(at);
+                err = 0;
+            }
             room.notify_all();
         }
         if (err && !st) {
@@ -4377,10 +4432,19 @@ int estimate_batch_impl(const fegb_config& cfg, int n_specs, const fegb_spec* sp
     };
     if (!st) {
         std::vector<std::thread> pool;
-        for (int t = 0; t < n_threads; ++t) pool.emplace_back(worker);
+        try {
+            for (int t = 1; t < n_threads; ++t) pool.emplace_back(worker);
+        } catch (const std::exception&) {  // no more threads: those there are, and this one
+        }
+        worker();
         for (auto& th : pool) th.join();
     }
     cudaEventDestroy(ready);
+    for (size_t at : again)
+        if (!st) {
+            st = run_class(classes[at].cb, classes[at].idx, s);
+            if (st) message = last_error();
+        }
     if (st) {
         if (!message.empty()) set_error("%s", message.c_str());
         return st;

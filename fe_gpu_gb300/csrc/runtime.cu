@@ -46,6 +46,8 @@ int set_cuda_error(cudaError_t err, const char* context) {
 
 const char* last_error() { return g_last_error; }
 
+thread_local AllocFailure* alloc_failure = nullptr;
+
 namespace {
 std::atomic<long long> g_launches{0};
 }
@@ -417,6 +419,17 @@ int fegb_get_tuning(const char* key, int* value) {
 int fegb_reset_tuning(void) {
     using namespace fegb;
     for (int i = 0; i < TUNE_COUNT; ++i) g_tune[i].store(kTune[i].def, std::memory_order_relaxed);
+    return set_ok();
+}
+
+int fegb_test_fail_alloc(const char* what, int times) {
+    static thread_local char label[64];
+    static thread_local fegb::AllocFailure plan{label, {0}};
+    fegb::alloc_failure = nullptr;
+    if (!what || times <= 0) return set_ok();
+    std::snprintf(label, sizeof(label), "%s", what);
+    plan.left = times;
+    fegb::alloc_failure = &plan;
     return set_ok();
 }
 

@@ -215,6 +215,11 @@ int fegb_test_dense_plan(const int* group_counts, int n_fe, int C, long long n, 
  * the fit returns an error; negative: the default). */
 int fegb_test_projection_wait(long long ns);
 
+/* Self-test of what happens when device memory runs out: the next `times` scratch
+ * allocations with this label in the fits of the calling thread fail (times 0:
+ * none). No memory is used up. */
+int fegb_test_fail_alloc(const char* what, int times);
+
 /* FE reconstruction of --save-fe (reconstruct_and_save_fixed_effects,
  * src/core/fe_pipeline.f90:1619-1733): forward Gauss-Seidel sweeps of the
  * residual y - W beta (beta: host, k values), dimension by dimension, each
