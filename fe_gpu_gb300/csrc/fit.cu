@@ -461,6 +461,8 @@ std::vector<char> cg_dense_plan(const std::vector<int>& G, int C, long long n, b
     return dense;
 }
 
+constexpr size_t TUPLE_DIMS = 4;  // cluster_ids_by_key
+
 // Row counts of runs and tuples are FP32 weights, exact up to this many rows
 constexpr int WEIGHT_ROWS = 1 << 24;
 
@@ -1390,6 +1392,8 @@ int cg_streams(Problem& P, CGBuffers<T>& B) {
         st.n_multi = D.n_multi_cg;
     }
     if (sw.size() < 2 || n < 4096) return 0;
+    // the projections take any number of dimensions: beyond what a tuple's key holds, their rows
+    if (P.padded_counts && sw.size() > TUPLE_DIMS) return 0;
     std::vector<const int32_t*> ptrs;
     std::vector<unsigned long long> strides;
     unsigned long long stride = 1;
