@@ -3064,10 +3064,13 @@ int demean_mixed(Problem& P, double tol, int max_iter, int* iterations, int* con
         const double inner_tol = std::max(0.25 * tol, 1e-5 * mu);
         int it = 0;
         double upd = 0.0, largest = 0.0;
+        // an inner solve may use half of the iterations that are left (the first half
+        // rounded up), so that a fit at its limit ends on refined means
+        const int most = (max_iter - total_iter + 1) / 2;
         if (groups)
-            FEGB_TRY(A.run(P, inner_tol, max_iter - total_iter, &it, &upd, &largest));
+            FEGB_TRY(A.run(P, inner_tol, most, &it, &upd, &largest));
         else
-            FEGB_TRY(ap_solve_rows(P, inner_tol, max_iter - total_iter, &it));
+            FEGB_TRY(ap_solve_rows(P, inner_tol, most, &it));
         total_iter += it;
         apply_alpha = true;
     }
