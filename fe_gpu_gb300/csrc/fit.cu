@@ -64,7 +64,9 @@ constexpr int MODE_SMALLG = 2;
 // Positions a chunk of the row sweeps has. One chunk is one thread's serial walk
 // a column (256 positions: 41 us, 64: 12, at 38k x 30), so rows whose chunks
 // do not fill the chip take short ones; with the chip full the longer ones leave
-// fewer edges to put together. 20M elements are 2,400 warps of 256-position chunks.
+// fewer edges to put together. Whole fits with 64 and 256 positions: 1.8M elements
+// 3.56 and 3.78 ms, 20M 5.3 and 5.5, 22M (30 columns) 6.56 and 6.53, 79M 9.9 and
+// 10.1, 162M 16.8 and 16.7: the line could lie anywhere from 20M to 100M.
 inline int chunk_rows(long long n, int C) { return n * C < 20000000LL ? 64 : 256; }
 constexpr int MAX_CLUSTER_DIMS = 3;  // src/core/fe_pipeline.f90:20
 

@@ -926,7 +926,7 @@ int fegb_test_gram(const double* X, long long n, int a, int split, double* out) 
 int fegb_test_group_sums(const double* X, long long n, int C, const int32_t* gid, int G, int small_g,
                          double* out_sums) {
     using namespace fegb;
-    constexpr int kChunk = 256;  // positions per segment-sweep chunk, as the fits use
+    constexpr int kChunk = 256;  // positions per segment-sweep chunk, the longer of the fits' two
     if (n <= 0 || C <= 0 || G <= 0 || !X || !gid || !out_sums) return set_error("fegb_test_group_sums: invalid sizes");
     if (small_g && !smallg_eligible(G, C)) return set_error("fegb_test_group_sums: G=%d C=%d not small-G", G, C);
     Scratch scr(kLegacy);
